@@ -289,9 +289,7 @@ int mlf_ilu0_solve(mlf_ctx* h, const double* y, double* x, int nrhs) {
     int st;
     if ((st = ensure_io(c, n))) return st;
     if ((st = h2d_cols(c, c->dx_io, y, nrhs, c->N))) return st;
-    for (int r = 0; r < nrhs; ++r)
-        if ((st = device_ilu_solve(c, c->dx_io + (size_t)r * c->N, c->dy_io + (size_t)r * c->N, c->stream)))
-            return st;
+    if ((st = device_ilu_solve(c, c->dx_io, c->dy_io, nrhs, c->stream))) return st;
     if ((st = d2h_cols(c, x, c->dy_io, nrhs, c->N))) return st;
     CK(cudaStreamSynchronize(c->stream));
     return MLF_OK;
@@ -397,9 +395,7 @@ int mlf_precond_apply(mlf_ctx* h, int precond_kind, const double* y, double* x, 
     if (precond_kind == 2) {
         if ((st = device_nearinv_apply(c, c->dx_io, c->dy_io, nrhs, c->stream))) return st;
     } else {
-        for (int r = 0; r < nrhs; ++r)
-            if ((st = device_ilu_solve(c, c->dx_io + (size_t)r * c->N, c->dy_io + (size_t)r * c->N, c->stream)))
-                return st;
+        if ((st = device_ilu_solve(c, c->dx_io, c->dy_io, nrhs, c->stream))) return st;
     }
     if ((st = d2h_cols(c, x, c->dy_io, nrhs, c->N))) return st;
     CK(cudaStreamSynchronize(c->stream));

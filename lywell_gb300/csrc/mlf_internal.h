@@ -179,6 +179,8 @@ struct Ctx {
     std::vector<int> jlu, ju;
     float2* dalu = nullptr;
     int *djlu = nullptr, *dju = nullptr;
+    double2* dalu64 = nullptr;        // alu in FP64, instead of dalu and the level lists, where the
+                                      // sweeps run in one CTA a column (narrow levels)
     // neighbourhood-inverse preconditioner (near CSR pattern)
     double2* dMinv = nullptr;         // CSR values, or compact own-box blocks when nearinv_own
     long long* dboff = nullptr;       // own-box block offsets
@@ -240,7 +242,7 @@ int device_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaSt
 int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s,
                        double2* const* Cf, double2* const* Bf, double2* const* Af, cudaEvent_t* ev);
 int device_ilu_upload(Ctx* c);
-int device_ilu_solve(Ctx* c, const double2* y, double2* x, cudaStream_t s);
+int device_ilu_solve(Ctx* c, const double2* y, double2* x, int nrhs, cudaStream_t s);
 int device_cgs(Ctx* c, const double2* b, const double2* x0, double tol, int maxit, int nrhs,
                double2* x, int* iters, double* relres, int precond, int* status);
 int device_nearinv_setup(Ctx* c, int* bad_box, int own_only);

@@ -789,13 +789,7 @@ static int col_norms32(Ctx* c, int nrhs, const float2* w, double2* partial, doub
 // FP64 M^-1 applied to the correction once per cycle
 static int apply_precond64(Ctx* c, int precond, int nrhs, const double2* in, double2* out, cudaStream_t s) {
     if (precond == 2) return device_nearinv_apply(c, in, out, nrhs, s);
-    if (precond == 1) {
-        for (int col = 0; col < nrhs; ++col) {
-            const int st = device_ilu_solve(c, in + (size_t)col * c->N, out + (size_t)col * c->N, s);
-            if (st) return st;
-        }
-        return MLF_OK;
-    }
+    if (precond == 1) return device_ilu_solve(c, in, out, nrhs, s);
     CK(cudaMemcpyAsync(out, in, (size_t)c->N * nrhs * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     return MLF_OK;
 }

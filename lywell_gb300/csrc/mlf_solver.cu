@@ -2,9 +2,10 @@
 // iteration with device-resident scalars, the plane-wave excitation and the
 // RCS far-field sum.
 //
-//   lusol0C       modIterativo.f90:504-560   -> k_sweep_fwd / k_sweep_bwd, one
-//                 warp per row, rows of one dependency level per launch; the
-//                 launches of one application are captured in a CUDA graph.
+//   lusol0C       modIterativo.f90:504-560   -> k_ilu_cta, both sweeps of a
+//                 column in one CTA with x in shared memory, where dependency
+//                 levels are narrow; else k_sweep_fwd / k_sweep_bwd, one warp
+//                 per row, rows of one dependency level per launch.
 //   CGSold        modIterativo.f90:331-493   -> device_cgs: per-column scalars
 //                 (rho, alpha, beta) live on the device; dot products are
 //                 block partial sums reduced in a fixed order (run-to-run
@@ -94,40 +95,170 @@ __global__ void k_sweep_bwd(const int* __restrict__ rows, int nrows, const int* 
     }
 }
 
+// Both sweeps of one column in one CTA, x in shared memory, for factors whose
+// dependency levels are narrow (ILUT's hold about two rows).  Warp w takes the
+// rows w, w + 32, ... in dependency order, so about 32 rows are in flight;
+// their entries are loaded ahead and a row's lanes wait on a flag per row.
+// The serial chain from row to row bounds it -- poll, DFMA, reduction, store,
+// about 1.1 us a level -- against the 5 to 7 us that a launch per level takes;
+// values are kept in FP64 (a conversion costs a slot of the SM's FP64 pipe)
+// and the reduction carries Re in lanes 0-15 and Im in lanes 16-31.  The sums
+// are those of k_sweep_fwd / k_sweep_bwd in the same order, bit for bit: CGS
+// magnifies a last-place change here beyond its own stopping test.
+// Measured, one column (before -> now): ILUT of 1080 unknowns 6.1 -> 1.45 ms,
+// ILU0 of 1920 2.1 -> 0.66 ms, of 13230 8.3 -> 5.2 ms; 16 warps are 4 to 38 %
+// slower, 8 warps 6 to 79 %.
+// A wait that runs out (2^22 polls; nothing in a valid factor makes it) ends
+// the sweeps and x is NaN.
+constexpr int ILU_WARPS = 32;
+constexpr int ILU_SPIN = 1 << 22;
+
+template <bool FWD>
+__device__ void ilu_cta_sweep(int N, const int* __restrict__ jlu, const int* __restrict__ ju,
+                              const double2* __restrict__ alu, volatile double* xs, volatile unsigned char* rdy,
+                              volatile int* fail) {
+    constexpr unsigned char EP = FWD ? 1 : 2;
+    constexpr int NU = 4;   // entries per lane loaded ahead
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool re = lane < 16;
+    for (int t = warp; t < N; t += ILU_WARPS) {
+        if (__any_sync(0xffffffffu, *fail)) break;
+        const int i = FWD ? t : N - 1 - t;
+        const int k0 = FWD ? jlu[i + 1] : ju[i + 1], k1 = FWD ? ju[i + 1] : jlu[i + 2];
+        const double2 d = FWD ? make_double2(0, 0) : alu[i + 1];
+        double ar = 0, ai = 0;
+        for (int kb = k0; kb < k1; kb += 32 * NU) {
+            int c[NU];
+            double2 v[NU];
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                const int k = kb + 32 * u + lane;
+                c[u] = k < k1 ? jlu[k] - 1 : -1;
+                v[u] = k < k1 ? alu[k] : make_double2(0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                if (kb + 32 * u >= k1) break;   // warp-uniform
+                const bool has = c[u] >= 0;
+                const int cu = has ? c[u] : 0;
+                for (int n = 1; !__all_sync(0xffffffffu, !has || rdy[cu] == EP); ++n)
+                    if ((n & 1023) == 0 && __any_sync(0xffffffffu, n > ILU_SPIN || *fail)) {   // one decision a warp
+                        *fail = 1;
+                        break;
+                    }
+                __threadfence_block();
+                if (has) {
+                    const double xr = xs[2 * cu], xi = xs[2 * cu + 1];
+                    ar = fma(v[u].x, xr, ar); ar = fma(-v[u].y, xi, ar);
+                    ai = fma(v[u].x, xi, ai); ai = fma(v[u].y, xr, ai);
+                }
+                __syncwarp();
+            }
+        }
+        double s = (re ? ar : ai) + __shfl_xor_sync(0xffffffffu, re ? ai : ar, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const double ti = __shfl_sync(0xffffffffu, s, 16);
+        if (lane == 0) {
+            double2 x = make_double2(xs[2 * i] - s, xs[2 * i + 1] - ti);
+            if (!FWD)   // the fused forms k_sweep_bwd's product compiles to
+                x = make_double2(fma(d.x, x.x, -(d.y * x.y)), fma(d.x, x.y, d.y * x.x));
+            xs[2 * i] = x.x;
+            xs[2 * i + 1] = x.y;
+            __threadfence_block();
+            rdy[i] = EP;
+        }
+        __syncwarp();
+    }
+}
+
+// blockIdx.x = column; dynamic shared memory: x (N double2), a flag byte per row
+__global__ void __launch_bounds__(32 * ILU_WARPS)
+k_ilu_cta(int N, const int* __restrict__ jlu, const int* __restrict__ ju, const double2* __restrict__ alu,
+          const double2* __restrict__ y, double2* __restrict__ x) {
+    extern __shared__ __align__(16) unsigned char ilu_smem[];
+    __shared__ int fail;
+    double2* xs = reinterpret_cast<double2*>(ilu_smem);
+    unsigned char* rdy = ilu_smem + (size_t)N * sizeof(double2);
+    const double2* yc = y + (size_t)blockIdx.x * N;
+    double2* xc = x + (size_t)blockIdx.x * N;
+    if (threadIdx.x == 0) fail = 0;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        xs[i] = yc[i];
+        rdy[i] = 0;
+    }
+    __syncthreads();
+    volatile double* xv = reinterpret_cast<volatile double*>(xs);
+    ilu_cta_sweep<true>(N, jlu, ju, alu, xv, rdy, &fail);
+    __syncthreads();
+    ilu_cta_sweep<false>(N, jlu, ju, alu, xv, rdy, &fail);
+    __syncthreads();
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) xc[i] = fail ? make_double2(nan, nan) : xs[i];
+}
+
+// Whether k_ilu_cta takes the factors: x must fit in one CTA's shared memory
+// (13 900 unknowns), and levels must be narrow: one SM takes up to 0.2 us a row
+// (measured 0.15 to 0.20 with ILU0's 180 to 600 levels), a launch per level
+// 6 us (measured 4.7 to 7).
+static bool ilu_in_cta(const Ctx* c, int optin) {
+    constexpr double ROW_US = 0.2, LEVEL_US = 6.0;
+    if ((size_t)c->N * (sizeof(double2) + 1) + 1024 > (size_t)optin) return false;
+    const double levels = (double)(c->lvl_ptr_f.size() + c->lvl_ptr_b.size() - 2);
+    return 2 * ROW_US * c->N < LEVEL_US * levels;
+}
+
 int device_ilu_upload(Ctx* c) {
     auto F = [](void* p) { if (p) cudaFree(p); };
-    F(c->dalu); F(c->djlu); F(c->dju); F(c->dlvl_rows_f); F(c->dlvl_rows_b);
-    CK(cudaMalloc(&c->dalu, c->alu.size() * sizeof(float2)));
-    CK(cudaMemcpy(c->dalu, c->alu.data(), c->alu.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->djlu, c->jlu.size() * sizeof(int)));
-    CK(cudaMemcpy(c->djlu, c->jlu.data(), c->jlu.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->dju, c->ju.size() * sizeof(int)));
-    CK(cudaMemcpy(c->dju, c->ju.data(), c->ju.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->dlvl_rows_f, c->lvl_rows_f.size() * sizeof(int)));
-    CK(cudaMemcpy(c->dlvl_rows_f, c->lvl_rows_f.data(), c->lvl_rows_f.size() * sizeof(int),
-                  cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&c->dlvl_rows_b, c->lvl_rows_b.size() * sizeof(int)));
-    CK(cudaMemcpy(c->dlvl_rows_b, c->lvl_rows_b.data(), c->lvl_rows_b.size() * sizeof(int),
-                  cudaMemcpyHostToDevice));
+    F(c->dalu); F(c->djlu); F(c->dju); F(c->dlvl_rows_f); F(c->dlvl_rows_b); F(c->dalu64);
+    c->dalu = nullptr;
+    c->dalu64 = nullptr;
+    c->djlu = c->dju = c->dlvl_rows_f = c->dlvl_rows_b = nullptr;
+    auto up = [&](auto** dst, const auto& v) {
+        CK(cudaMalloc(dst, v.size() * sizeof(v[0])));
+        CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+        return MLF_OK;
+    };
+    int optin = 0, st;
+    if ((st = up(&c->djlu, c->jlu)) || (st = up(&c->dju, c->ju))) return st;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
+    if (ilu_in_cta(c, optin)) {
+        std::vector<double2> a64(c->alu.size());
+        for (size_t k = 0; k < a64.size(); ++k) a64[k] = make_double2((double)c->alu[k].x, (double)c->alu[k].y);
+        if ((st = up(&c->dalu64, a64))) return st;
+        // a limit of the kernel, shared by every context: the device's maximum
+        CK(cudaFuncSetAttribute(k_ilu_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+        return MLF_OK;
+    }
+    if ((st = up(&c->dalu, c->alu)) || (st = up(&c->dlvl_rows_f, c->lvl_rows_f)) ||
+        (st = up(&c->dlvl_rows_b, c->lvl_rows_b)))
+        return st;
     return MLF_OK;
 }
 
-// x = (LU)^-1 y for one column; y and x must not alias.
-int device_ilu_solve(Ctx* c, const double2* y, double2* x, cudaStream_t s) {
+// x = (LU)^-1 y for nrhs columns (leading dimension N); y and x must not alias.
+int device_ilu_solve(Ctx* c, const double2* y, double2* x, int nrhs, cudaStream_t s) {
     if (!c->ilu_ok) {
         c->err = "ILU0 factors not available (mlf_ilu0 has not succeeded)";
         return MLF_E_STATE;
     }
-    const int nlf = (int)c->lvl_ptr_f.size() - 1, nlb = (int)c->lvl_ptr_b.size() - 1;
-    for (int l = 0; l < nlf; ++l) {
-        const int r0 = c->lvl_ptr_f[l], nr = c->lvl_ptr_f[l + 1] - r0;
-        k_sweep_fwd<<<(nr * 32 + 255) / 256, 256, 0, s>>>(c->dlvl_rows_f + r0, nr, c->djlu, c->dju, c->dalu,
-                                                          y, x);
+    if (c->dalu64) {
+        k_ilu_cta<<<nrhs, 32 * ILU_WARPS, (size_t)c->N * (sizeof(double2) + 1), s>>>(c->N, c->djlu, c->dju, c->dalu64,
+                                                                                     y, x);
+        return cuda_ok(c, cudaGetLastError(), "ilu sweeps") ? MLF_OK : MLF_E_CUDA;
     }
-    for (int l = 0; l < nlb; ++l) {
-        const int r0 = c->lvl_ptr_b[l], nr = c->lvl_ptr_b[l + 1] - r0;
-        k_sweep_bwd<<<(nr * 32 + 255) / 256, 256, 0, s>>>(c->dlvl_rows_b + r0, nr, c->djlu, c->dju, c->dalu,
-                                                          x);
+    const int nlf = (int)c->lvl_ptr_f.size() - 1, nlb = (int)c->lvl_ptr_b.size() - 1;
+    for (int r = 0; r < nrhs; ++r, y += c->N, x += c->N) {
+        for (int l = 0; l < nlf; ++l) {
+            const int r0 = c->lvl_ptr_f[l], nr = c->lvl_ptr_f[l + 1] - r0;
+            k_sweep_fwd<<<(nr * 32 + 255) / 256, 256, 0, s>>>(c->dlvl_rows_f + r0, nr, c->djlu, c->dju, c->dalu,
+                                                              y, x);
+        }
+        for (int l = 0; l < nlb; ++l) {
+            const int r0 = c->lvl_ptr_b[l], nr = c->lvl_ptr_b[l + 1] - r0;
+            k_sweep_bwd<<<(nr * 32 + 255) / 256, 256, 0, s>>>(c->dlvl_rows_b + r0, nr, c->djlu, c->dju, c->dalu,
+                                                              x);
+        }
     }
     return cuda_ok(c, cudaGetLastError(), "ilu sweeps") ? MLF_OK : MLF_E_CUDA;
 }
@@ -334,11 +465,7 @@ static int precond_apply(Ctx* c, int precond, int nrhs, const double2* y, double
         return MLF_OK;
     }
     if (precond == 2) return device_nearinv_apply(c, y, x, nrhs, s);
-    for (int r = 0; r < nrhs; ++r) {
-        const int st = device_ilu_solve(c, y + (size_t)r * c->N, x + (size_t)r * c->N, s);
-        if (st) return st;
-    }
-    return MLF_OK;
+    return device_ilu_solve(c, y, x, nrhs, s);
 }
 
 // b, x0, x: device arrays N x nrhs (ld = N).  x0 may equal nullptr.
