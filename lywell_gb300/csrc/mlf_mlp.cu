@@ -32,40 +32,79 @@ namespace mlp {
 constexpr int IN = 16, H = 128, OUT = 2, TT = 64;
 constexpr int OW1 = 0, OB1 = OW1 + IN * H, OW2 = OB1 + H, OB2 = OW2 + H * H, OW3 = OB2 + H, OB3 = OW3 + H * OUT,
               NPARAM = OB3 + OUT;
+constexpr size_t GBYTES = NPARAM * sizeof(float) + sizeof(double);
+static_assert(NPARAM % 2 == 0 && OW2 % 8 == 0 && OB2 % 8 == 0 && OW3 % 8 == 0, "aligned parts of the parameter vector");
 
 struct Net {
     int dev = 0;
     cudaStream_t stream = nullptr;
     float* P = nullptr;            // FP32 master
     __nv_bfloat16* Pb = nullptr;   // BF16 copy
-    float *G = nullptr, *M1 = nullptr, *M2 = nullptr;
+    float *G = nullptr, *M1 = nullptr, *M2 = nullptr;   // G: gradient, then the loss sum (a double)
     float* norm = nullptr;         // mu[16], sd[16]
-    double* dloss = nullptr;
     int* derr = nullptr;           // set when a tensor-core forward CTA gave up a wait
     int adam_t = 0;
     std::string err;
 };
 
-// shared-memory image of one tile
+// Shared-memory image of one training tile.  Rows are padded so that the
+// 16-byte accesses below meet no bank twice: W2 by 4 floats (read down a column
+// block by 16 lanes in the backward pass), H1 and H2 by 8 BF16.
+constexpr int W2P = H + 4, HP = H + 8;
 struct Smem {
-    float W1[IN * H], b1[H], W2[H * H], b2[H], W3[H * OUT], b3[OUT];
+    float W1[IN * H], b1[H], W2[H * W2P], b2[H], W3[H * OUT], b3[OUT + 2];
     float X[TT * IN];
-    __nv_bfloat16 H1[TT * H], H2[TT * H];
+    __nv_bfloat16 H1[TT * HP], H2[TT * HP];
     float out[TT * OUT];
     float dH2[TT * H], dH1[TT * H];
 };
 
 __device__ __forceinline__ float bf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-__device__ void load_weights(Smem& s, const __nv_bfloat16* __restrict__ Pb) {
-    for (int q = threadIdx.x; q < IN * H; q += blockDim.x) s.W1[q] = __bfloat162float(Pb[OW1 + q]);
-    for (int q = threadIdx.x; q < H * H; q += blockDim.x) s.W2[q] = __bfloat162float(Pb[OW2 + q]);
-    for (int q = threadIdx.x; q < H * OUT; q += blockDim.x) s.W3[q] = __bfloat162float(Pb[OW3 + q]);
-    for (int q = threadIdx.x; q < H; q += blockDim.x) {
-        s.b1[q] = __bfloat162float(Pb[OB1 + q]);
-        s.b2[q] = __bfloat162float(Pb[OB2 + q]);
+__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+// two BF16 values in one word, a at the lower address
+__device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+
+// count (a multiple of 8) BF16 values to floats, row-major rows of H with the given stride
+__device__ __forceinline__ void load_bf16_rows(float* dst, int stride, const __nv_bfloat16* __restrict__ src, int count) {
+    for (int q = threadIdx.x; q < count / 8; q += blockDim.x) {
+        const uint4 v = reinterpret_cast<const uint4*>(src)[q];
+        float4* d = reinterpret_cast<float4*>(dst + (8 * q / H) * stride + 8 * q % H);
+        d[0] = make_float4(bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y));
+        d[1] = make_float4(bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w));
     }
+}
+
+__device__ void load_weights(Smem& s, const __nv_bfloat16* __restrict__ Pb) {
+    load_bf16_rows(s.W1, H, Pb + OW1, IN * H);
+    load_bf16_rows(s.W2, W2P, Pb + OW2, H * H);
+    load_bf16_rows(s.W3, H, Pb + OW3, H * OUT);
+    load_bf16_rows(s.b1, H, Pb + OB1, H);
+    load_bf16_rows(s.b2, H, Pb + OB2, H);
     if (threadIdx.x < OUT) s.b3[threadIdx.x] = __bfloat162float(Pb[OB3 + threadIdx.x]);
+}
+
+// The 256 threads of a training tile: token group tg = tid / 16 (4 tokens) and
+// neuron group ng = tid % 16, the eight neurons 4 ng .. 4 ng + 3 and
+// 64 + 4 ng .. 64 + 4 ng + 3: a quarter warp's 16-byte reads of a row are
+// contiguous.
+__device__ __forceinline__ void load8(float (&v)[8], const float* row, int ng) {
+    const float4 a = *reinterpret_cast<const float4*>(row + 4 * ng);
+    const float4 b = *reinterpret_cast<const float4*>(row + 64 + 4 * ng);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void store_relu8(__nv_bfloat16* row, const float (&v)[8], int ng) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<uint2*>(row + 64 * h + 4 * ng) =
+            make_uint2(pack_bf2(fmaxf(v[4 * h], 0.f), fmaxf(v[4 * h + 1], 0.f)),
+                       pack_bf2(fmaxf(v[4 * h + 2], 0.f), fmaxf(v[4 * h + 3], 0.f)));
 }
 
 // forward of one tile of nt <= TT tokens starting at token t0 (rows past nt are zero)
@@ -76,58 +115,71 @@ __device__ void forward_tile(Smem& s, const float* __restrict__ X, const float* 
         s.X[q] = t < nt ? (X[(t0 + t) * IN + i] - norm[i]) / norm[IN + i] : 0.f;
     }
     __syncthreads();
-    // 256 threads: token group tg = tid / 16 (4 tokens), neuron group ng = tid % 16 (8 neurons)
     const int tg = threadIdx.x >> 4, ng = threadIdx.x & 15;
     {
-        float acc[4][8];
+        float acc[4][8], b[8];
+        load8(b, s.b1, ng);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) acc[a][u] = s.b1[ng * 8 + u];
-        for (int i = 0; i < IN; ++i) {
-            float w[8];
+            for (int u = 0; u < 8; ++u) acc[a][u] = b[u];
+        for (int i = 0; i < IN; i += 4) {
+            float4 x[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) w[u] = s.W1[i * H + ng * 8 + u];
+            for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const float4*>(&s.X[(tg * 4 + a) * IN + i]);
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float x = s.X[(tg * 4 + a) * IN + i];
+            for (int q = 0; q < 4; ++q) {
+                float w[8];
+                load8(w, s.W1 + (i + q) * H, ng);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(x, w[u], acc[a][u]);
+                for (int a = 0; a < 4; ++a) {
+                    const float xv = q == 0 ? x[a].x : q == 1 ? x[a].y : q == 2 ? x[a].z : x[a].w;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(xv, w[u], acc[a][u]);
+                }
             }
         }
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s.H1[(tg * 4 + a) * H + ng * 8 + u] = __float2bfloat16_rn(fmaxf(acc[a][u], 0.f));
+        for (int a = 0; a < 4; ++a) store_relu8(s.H1 + (tg * 4 + a) * HP, acc[a], ng);
     }
     __syncthreads();
     {
-        float acc[4][8];
+        float acc[4][8], b[8];
+        load8(b, s.b2, ng);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) acc[a][u] = s.b2[ng * 8 + u];
-        for (int k = 0; k < H; ++k) {
-            float w[8];
+            for (int u = 0; u < 8; ++u) acc[a][u] = b[u];
+        for (int k = 0; k < H; k += 4) {
+            uint2 h[4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) w[u] = s.W2[k * H + ng * 8 + u];
+            for (int a = 0; a < 4; ++a) h[a] = *reinterpret_cast<const uint2*>(&s.H1[(tg * 4 + a) * HP + k]);
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float h = __bfloat162float(s.H1[(tg * 4 + a) * H + k]);
+            for (int q = 0; q < 4; ++q) {
+                float w[8];
+                load8(w, s.W2 + (k + q) * W2P, ng);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(h, w[u], acc[a][u]);
+                for (int a = 0; a < 4; ++a) {
+                    const float hv = q == 0 ? bf_lo(h[a].x) : q == 1 ? bf_hi(h[a].x) : q == 2 ? bf_lo(h[a].y) : bf_hi(h[a].y);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(hv, w[u], acc[a][u]);
+                }
             }
         }
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s.H2[(tg * 4 + a) * H + ng * 8 + u] = __float2bfloat16_rn(fmaxf(acc[a][u], 0.f));
+        for (int a = 0; a < 4; ++a) store_relu8(s.H2 + (tg * 4 + a) * HP, acc[a], ng);
     }
     __syncthreads();
     if (threadIdx.x < TT * OUT) {
         const int t = threadIdx.x / OUT, o = threadIdx.x - t * OUT;
         float acc = s.b3[o];
-        for (int k = 0; k < H; ++k) acc = fmaf(__bfloat162float(s.H2[t * H + k]), s.W3[k * OUT + o], acc);
+        for (int k = 0; k < H; k += 4) {
+            const uint2 h = *reinterpret_cast<const uint2*>(&s.H2[t * HP + k]);
+            acc = fmaf(bf_lo(h.x), s.W3[k * OUT + o], acc);
+            acc = fmaf(bf_hi(h.x), s.W3[(k + 1) * OUT + o], acc);
+            acc = fmaf(bf_lo(h.y), s.W3[(k + 2) * OUT + o], acc);
+            acc = fmaf(bf_hi(h.y), s.W3[(k + 3) * OUT + o], acc);
+        }
         s.out[threadIdx.x] = acc;
     }
     __syncthreads();
@@ -156,11 +208,6 @@ struct TcMlpSmem {
     uint32_t tmem;
     int fail;
 };
-
-__device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
-    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);   // a at the lower address
-    return *reinterpret_cast<const uint32_t*>(&p);
-}
 
 __global__ void __launch_bounds__(TQ, 2) k_mlp_forward_tc(long long ntok, const float* __restrict__ X,
                                                          const float* __restrict__ norm,
@@ -274,7 +321,12 @@ __global__ void __launch_bounds__(TQ, 2) k_mlp_forward_tc(long long ntok, const 
 
 // Forward + loss + backward over tokens idx[0..ntok) (idx NULL: 0..ntok-1);
 // gradients of the mean loss (scale = 1 / (ntok_total * OUT)) added into G,
-// the loss sum into *loss.
+// the loss sum into *loss.  A tile's three 64 x 128 x 128 products are FP32
+// FMAs on values in shared memory (4 x 8 or 8 x 8 sums a thread); 16-byte
+// shared-memory reads without bank conflicts and 16-byte reductions into G
+// keep the FMA pipe the bound (about 13 us a tile).  8192 tokens, one tile on
+// each of 128 SMs, mlf_mlp_grad with its copy to the host: 172 us with scalar
+// reads (conflicts of 4 to 16 ways) and scalar atomics, 65 us now.
 __global__ void __launch_bounds__(256) k_mlp_grad(long long ntok, const long long* __restrict__ idx,
                                                   const float* __restrict__ X, const float* __restrict__ T,
                                                   const float* __restrict__ norm,
@@ -327,7 +379,7 @@ __global__ void __launch_bounds__(256) k_mlp_grad(long long ntok, const long lon
         {
             const int k = threadIdx.x >> 1, o = threadIdx.x & 1;   // 256 = 128 x 2
             float g = 0.f;
-            for (int t = 0; t < TT; ++t) g = fmaf(__bfloat162float(s.H2[t * H + k]), s.out[t * OUT + o], g);
+            for (int t = 0; t < TT; ++t) g = fmaf(__bfloat162float(s.H2[t * HP + k]), s.out[t * OUT + o], g);
             atomicAdd(&G[OW3 + k * OUT + o], g);
             if (threadIdx.x < OUT) {
                 float gb = 0.f;
@@ -336,64 +388,77 @@ __global__ void __launch_bounds__(256) k_mlp_grad(long long ntok, const long lon
             }
         }
         // dH2 = relu'(H2) * dOut W3^T
-        for (int q = threadIdx.x; q < TT * H; q += blockDim.x) {
-            const int t = q / H, k = q - t * H;
-            const float h = __bfloat162float(s.H2[q]);
-            s.dH2[q] = h > 0.f ? s.out[t * OUT] * s.W3[k * OUT] + s.out[t * OUT + 1] * s.W3[k * OUT + 1] : 0.f;
+        for (int q = threadIdx.x; q < TT * H / 4; q += blockDim.x) {
+            const int t = q / (H / 4), k = 4 * (q - t * (H / 4));
+            const uint2 h = *reinterpret_cast<const uint2*>(&s.H2[t * HP + k]);
+            const float4 wa = *reinterpret_cast<const float4*>(&s.W3[k * OUT]);
+            const float4 wb = *reinterpret_cast<const float4*>(&s.W3[(k + 2) * OUT]);
+            const float o0 = s.out[t * OUT], o1 = s.out[t * OUT + 1];
+            *reinterpret_cast<float4*>(&s.dH2[t * H + k]) =
+                make_float4(bf_lo(h.x) > 0.f ? o0 * wa.x + o1 * wa.y : 0.f, bf_hi(h.x) > 0.f ? o0 * wa.z + o1 * wa.w : 0.f,
+                            bf_lo(h.y) > 0.f ? o0 * wb.x + o1 * wb.y : 0.f, bf_hi(h.y) > 0.f ? o0 * wb.z + o1 * wb.w : 0.f);
         }
         __syncthreads();
-        // dW2[k][n] = sum_t H1[t][k] dH2[t][n]: thread (kg = tid / 16: 8 k's, ng: 8 n's)
+        // dW2[k][n] = sum_t H1[t][k] dH2[t][n]: thread (tg: 8 k's, ng: 8 n's)
         {
             float acc[8][8];
 #pragma unroll
             for (int a = 0; a < 8; ++a)
 #pragma unroll
                 for (int u = 0; u < 8; ++u) acc[a][u] = 0.f;
+#pragma unroll 2
             for (int t = 0; t < TT; ++t) {
                 float d[8];
+                load8(d, s.dH2 + t * H, ng);
+                const uint4 hw = *reinterpret_cast<const uint4*>(&s.H1[t * HP + tg * 8]);
+                const float h[8] = {bf_lo(hw.x), bf_hi(hw.x), bf_lo(hw.y), bf_hi(hw.y),
+                                    bf_lo(hw.z), bf_hi(hw.z), bf_lo(hw.w), bf_hi(hw.w)};
 #pragma unroll
-                for (int u = 0; u < 8; ++u) d[u] = s.dH2[t * H + ng * 8 + u];
+                for (int a = 0; a < 8; ++a)
 #pragma unroll
-                for (int a = 0; a < 8; ++a) {
-                    const float h = __bfloat162float(s.H1[t * H + tg * 8 + a]);
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(h, d[u], acc[a][u]);
-                }
+                    for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(h[a], d[u], acc[a][u]);
             }
 #pragma unroll
             for (int a = 0; a < 8; ++a)
 #pragma unroll
-                for (int u = 0; u < 8; ++u) atomicAdd(&G[OW2 + (tg * 8 + a) * H + ng * 8 + u], acc[a][u]);
+                for (int q = 0; q < 2; ++q)
+                    atomicAdd(reinterpret_cast<float4*>(&G[OW2 + (tg * 8 + a) * H + 64 * q + 4 * ng]),
+                              make_float4(acc[a][4 * q], acc[a][4 * q + 1], acc[a][4 * q + 2], acc[a][4 * q + 3]));
         }
         if (threadIdx.x < H) {
             float gb = 0.f;
             for (int t = 0; t < TT; ++t) gb += s.dH2[t * H + threadIdx.x];
             atomicAdd(&G[OB2 + threadIdx.x], gb);
         }
-        // dH1 = relu'(H1) * dH2 W2^T
+        // dH1 = relu'(H1) * dH2 W2^T: thread (tg: 4 tokens, the 8 k's ng + 16 u)
         {
             float acc[4][8];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int u = 0; u < 8; ++u) acc[a][u] = 0.f;
-            for (int n = 0; n < H; ++n) {
-                float w[8];
+            for (int n = 0; n < H; n += 4) {
+                float4 d[4];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) w[u] = s.W2[(ng * 8 + u) * H + n];
+                for (int a = 0; a < 4; ++a) d[a] = *reinterpret_cast<const float4*>(&s.dH2[(tg * 4 + a) * H + n]);
 #pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    const float d = s.dH2[(tg * 4 + a) * H + n];
+                for (int u = 0; u < 8; ++u) {
+                    const float4 w = *reinterpret_cast<const float4*>(&s.W2[(ng + 16 * u) * W2P + n]);
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) acc[a][u] = fmaf(d, w[u], acc[a][u]);
+                    for (int a = 0; a < 4; ++a) {
+                        acc[a][u] = fmaf(d[a].x, w.x, acc[a][u]);
+                        acc[a][u] = fmaf(d[a].y, w.y, acc[a][u]);
+                        acc[a][u] = fmaf(d[a].z, w.z, acc[a][u]);
+                        acc[a][u] = fmaf(d[a].w, w.w, acc[a][u]);
+                    }
                 }
             }
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const int q = (tg * 4 + a) * H + ng * 8 + u;
-                    s.dH1[q] = __bfloat162float(s.H1[q]) > 0.f ? acc[a][u] : 0.f;
+                    const int t = tg * 4 + a, k = ng + 16 * u;
+                    s.dH1[t * H + k] = __bfloat162float(s.H1[t * HP + k]) > 0.f ? acc[a][u] : 0.f;
                 }
         }
         __syncthreads();
@@ -405,11 +470,15 @@ __global__ void __launch_bounds__(256) k_mlp_grad(long long ntok, const long lon
             for (int u = 0; u < 8; ++u) acc[u] = 0.f;
             for (int t = 0; t < TT; ++t) {
                 const float x = s.X[t * IN + i];
+                float d[8];
+                load8(d, s.dH1 + t * H, ng);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc[u] = fmaf(x, s.dH1[t * H + ng * 8 + u], acc[u]);
+                for (int u = 0; u < 8; ++u) acc[u] = fmaf(x, d[u], acc[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) atomicAdd(&G[OW1 + i * H + ng * 8 + u], acc[u]);
+            for (int q = 0; q < 2; ++q)
+                atomicAdd(reinterpret_cast<float4*>(&G[OW1 + i * H + 64 * q + 4 * ng]),
+                          make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]));
         }
         if (threadIdx.x < H) {
             float gb = 0.f;
@@ -489,11 +558,10 @@ int mlf_mlp_create(mlf_mlp** out, int device, unsigned long long seed) {
     if (!ok(n, cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking), "stream")) return fail(MLF_E_CUDA);
     if (!ok(n, cudaMalloc(&n->P, NPARAM * sizeof(float)), "alloc") ||
         !ok(n, cudaMalloc(&n->Pb, NPARAM * sizeof(__nv_bfloat16)), "alloc") ||
-        !ok(n, cudaMalloc(&n->G, NPARAM * sizeof(float)), "alloc") ||
+        !ok(n, cudaMalloc(&n->G, GBYTES), "alloc") ||
         !ok(n, cudaMalloc(&n->M1, NPARAM * sizeof(float)), "alloc") ||
         !ok(n, cudaMalloc(&n->M2, NPARAM * sizeof(float)), "alloc") ||
         !ok(n, cudaMalloc(&n->norm, 2 * IN * sizeof(float)), "alloc") ||
-        !ok(n, cudaMalloc(&n->dloss, sizeof(double)), "alloc") ||
         !ok(n, cudaMalloc(&n->derr, sizeof(int)), "alloc") || !ok(n, cudaMemset(n->derr, 0, sizeof(int)), "memset"))
         return fail(MLF_E_CUDA);
     if (!ok(n, cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -530,7 +598,7 @@ void mlf_mlp_free(mlf_mlp* h) {
     Net* n = &h->n;
     cudaSetDevice(n->dev);
     for (void* p : {(void*)n->P, (void*)n->Pb, (void*)n->G, (void*)n->M1, (void*)n->M2, (void*)n->norm,
-                    (void*)n->dloss, (void*)n->derr})
+                    (void*)n->derr})
         if (p) cudaFree(p);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete h;
@@ -598,16 +666,18 @@ int mlf_mlp_grad(mlf_mlp* h, const float* X, const float* T, long long ntok, flo
     if (!h || !X || !T || ntok <= 0) return MLF_E_ARG;
     Net* n = &h->n;
     NCK(cudaSetDevice(n->dev));
-    NCK(cudaMemsetAsync(n->G, 0, NPARAM * sizeof(float), n->stream));
-    NCK(cudaMemsetAsync(n->dloss, 0, sizeof(double), n->stream));
+    NCK(cudaMemsetAsync(n->G, 0, GBYTES, n->stream));
     const float scale = (float)(1.0 / ((double)ntok * OUT));
     k_mlp_grad<<<grid_for(ntok), 256, sizeof(Smem), n->stream>>>(ntok, nullptr, X, T, n->norm, n->Pb, scale, n->G,
-                                                                 n->dloss, nullptr, nullptr);
+                                                                 reinterpret_cast<double*>(n->G + NPARAM), nullptr,
+                                                                 nullptr);
     NCK(cudaGetLastError());
-    if (grad) NCK(cudaMemcpyAsync(grad, n->G, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
-    double l = 0;
-    NCK(cudaMemcpyAsync(&l, n->dloss, sizeof(double), cudaMemcpyDeviceToHost, n->stream));
+    std::vector<float> g(GBYTES / sizeof(float));
+    NCK(cudaMemcpyAsync(g.data(), n->G, GBYTES, cudaMemcpyDeviceToHost, n->stream));
     NCK(cudaStreamSynchronize(n->stream));
+    if (grad) std::memcpy(grad, g.data(), NPARAM * sizeof(float));
+    double l = 0;
+    std::memcpy(&l, g.data() + NPARAM, sizeof(double));
     if (loss) *loss = l / ((double)ntok * OUT);
     return MLF_OK;
 }

@@ -168,3 +168,17 @@ def test_learned_preconditioner_gain(gpu_lib):
     assert exact["status"] == "converged"
     assert out["iters"] < exact["iters"]
     m.close()
+
+
+@pytest.mark.parametrize("ntok", [1, 63, 64, 65, 80001])
+def test_gradient_at_tile_edges(net, ntok):
+    """Partial and single tiles of 64 tokens, and more tiles than CTAs.  A BF16
+    tie that falls the other way moves one of 128 hidden units by 2^-8, at
+    most 2^-8 of one token's gradient: 5e-3."""
+    import torch
+    P, norm, X, T = _problem(5, n=ntok)
+    net.set_params(P, norm)
+    loss, G = net.grad(torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda())
+    lref, gref = mlp.grad(P, norm, X, T)
+    assert abs(loss - lref) < 5e-3 * lref
+    assert np.linalg.norm(G - gref) < 5e-3 * np.linalg.norm(gref)
