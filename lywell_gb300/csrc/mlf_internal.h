@@ -201,6 +201,12 @@ struct Ctx {
     double* dscal = nullptr;          // device scalars
     size_t scal_cap = 0;
     int* dflags = nullptr;
+    // RCS sum: dipole data of the edges (built once), observation radius, and
+    // the workspace of directions, partial sums and results (grown on demand)
+    double *drcs_edge = nullptr, *drcs_ws = nullptr;
+    size_t rcs_cap = 0;
+    double rcs_R = 0;
+    bool rcs_near = false;            // the radius is under 500 body lengths
     size_t io_cap = 0;
     double2 *dx_io = nullptr, *dy_io = nullptr;
     // profiling

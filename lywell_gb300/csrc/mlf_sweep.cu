@@ -173,7 +173,7 @@ extern "C" int mlf_monostatic(mlf_ctx* h, int nang, const double* phis, int hh, 
             if ((st = device_solve_mixed(c, b, x0, tol, maxit, nb, x, it.data(), rr.data(), precond_kind,
                                          stc.data(), 0.9 * tol, &outer)))
                 break;
-            // the block's backscatter in one launch (a CTA per column)
+            // the block's backscatter in one launch
             std::vector<double> thq(nb, PI / 2.), phq(nb), sq(nb);
             for (int q = 0; q < nb; ++q) {
                 const int a = q * nrun + k;
