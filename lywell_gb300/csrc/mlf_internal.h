@@ -103,7 +103,7 @@ struct Mixed32 {
         float *wth = nullptr, *wph = nullptr, *thT_w = nullptr, *phT_w = nullptr;
         // translation by groups of G = 2 (grp[0]) or 4 (grp[1]) consecutive boxes:
         // merged far lists, sources ascending, tid = the source's translation
-        // index for each box of the group (-1: not far)
+        // index for each box of the group (-1: not far); those of 4 on first use
         struct Grp {
             int *ptr = nullptr, *src = nullptr, *tid = nullptr;
         } grp[2];
@@ -117,8 +117,8 @@ struct Ctx {
     int mv_prec = 0;                  // operator precision used by device_matvec: 0 FP64, 1 FP32
     int gmres_m = 0;                  // restart length of the mixed-precision GMRES cycles (0: automatic)
     int gs_passes = 1;                // classical Gram-Schmidt passes per Arnoldi step (1 or 2)
-    int tr_group = 0;                 // FP32 translation: boxes per thread (1, 2, 4; 0: 2 for one column, else 4)
-    int tr_cols = 0;                  // ... and columns per thread for grouped boxes (1, 2, 4; 0: 2 with 4 boxes, else 4)
+    int tr_group = 0;                 // FP32 translation: boxes per thread (1, 2, 4; 0: 2)
+    int tr_cols = 0;                  // ... and columns per thread (1, 2, 4; 0: 2)
     int basis_bits = 32;              // Krylov basis storage of the mixed solve: 32 (FP32) or 16 (FP16)
     int stag_window = 0;              // stagnation window in iterations (0: off): a column whose residual
                                       // sets no new minimum within this many iterations stops as stagnated

@@ -80,105 +80,112 @@ __global__ void k32_aggregate(int K, int nrhs, int N, const int* __restrict__ bo
     }
 }
 
-// B(:, col, box) = wq * sum over the far boxes of T_tid * C(:, col, src)
-// (llenar_campoCyB, modMLFMA.f90:1838-1852) for both polarisations and columns
-// [c0, c0 + NR): each thread owns one sample k, so each translation value is
-// read once per 2 NR products.
-template <int NR>
-__global__ void k32_translate(int K, int nrhs, int nchunk, const int* __restrict__ far_ptr,
-                              const int* __restrict__ far_src, const int* __restrict__ far_tid,
-                              const float2* __restrict__ T, const float* __restrict__ wq,
-                              const float2* __restrict__ C, float2* __restrict__ B) {
-    const int chunk = blockIdx.x % nchunk;
-    const int b = blockIdx.x / nchunk;
-    const int c0 = blockIdx.y * NR;
-    const int k = chunk * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    const size_t K2 = 2 * (size_t)K;
-    float2 a0[NR], a1[NR];
-#pragma unroll
-    for (int u = 0; u < NR; ++u) a0[u] = a1[u] = make_float2(0.f, 0.f);
-    const int f1 = far_ptr[b + 1];
-    for (int f = far_ptr[b]; f < f1; ++f) {
-        const float2 t = T[(size_t)far_tid[f] * K + k];
-        const float2* cs = C + ((size_t)far_src[f] * nrhs + c0) * K2 + k;
-#pragma unroll
-        for (int u = 0; u < NR; ++u) {
-            if (c0 + u < nrhs) {
-                fmac(a0[u], cs[u * K2], t);
-                fmac(a1[u], cs[u * K2 + K], t);
-            }
-        }
-    }
-    const float wk = wq[k];
-    float2* bo = B + ((size_t)b * nrhs + c0) * K2 + k;
-#pragma unroll
-    for (int u = 0; u < NR; ++u) {
-        if (c0 + u < nrhs) {
-            bo[u * K2] = make_float2(a0[u].x * wk, a0[u].y * wk);
-            bo[u * K2 + K] = make_float2(a1[u].x * wk, a1[u].y * wk);
-        }
-    }
+// Two FP32 values in one 64-bit register pair: Blackwell's packed FMA does two
+// per instruction slot.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 up2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-// The same sums for a group of G consecutive boxes (G i .. G i + G - 1, in
-// depth-first order and mostly siblings) over the merged list of their far
-// boxes: each source value read from L2 serves every box of the group that
-// has it, so the stage's L2 traffic, which bounds it, drops.  One thread per
-// sample k, both polarisations, NR columns and the G boxes in registers.
+// 16 bytes if on, else r as it was (not read then): the load is predicated, so
+// that it can be issued ahead of the branch that uses it
+__device__ __forceinline__ void ldg128_if(bool on, float4& r, const float4* p) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(r.x), "+f"(r.y), "+f"(r.z), "+f"(r.w)
+        : "l"(p), "r"((unsigned)on));
+}
+
+// B(:, col, box) = wq * sum over the far boxes of T_tid * C(:, col, src)
+// (llenar_campoCyB, modMLFMA.f90:1838-1852), for a group of G consecutive boxes
+// (G i .. G i + G - 1, in depth-first order and mostly siblings) over the
+// merged list of their far boxes: each source value read serves every box of
+// the group that has it.  A thread owns two consecutive samples (K = 2 L^2 is
+// even), both polarisations, NR columns and the G boxes, in registers: 16-byte
+// loads, and the index, address and branch work of a source is spent once for
+// 4 NR values.  The sums C Re T and C Im T are kept apart, (Re, Im) of C in one
+// packed FMA each, and joined at the end: no value is swapped or negated.
+// One warp per CTA: what bounds the stage is the reads through L1 and L2 (44 GB
+// of them on the sphere below), and groups in one CTA (2 to 8 warps, for L1
+// hits) were up to 15 % slower, as were 4 boxes (3.5 ms), two and three sources
+// in flight (3.0, 3.5 ms).  69120-RWG sphere, 16 columns: 2.97 -> 2.58 ms;
+// 122880-RWG sphere, one column: 0.449 -> 0.389 ms; 30720-RWG spheroid, 64
+// columns: 0.180 -> 0.141 ms (before: one sample a thread, unpacked, 4 boxes).
 template <int NR, int G>
-__global__ void k32_translate_grp(int K, int nb, int nrhs, int nchunk, const int* __restrict__ gptr,
-                                  const int* __restrict__ gsrc, const int* __restrict__ gtid,
-                                  const float2* __restrict__ T, const float* __restrict__ wq,
-                                  const float2* __restrict__ C, float2* __restrict__ B) {
-    const int chunk = blockIdx.x % nchunk;
+__global__ void __launch_bounds__(32)
+k32_translate_grp(int KP, int nb, int nrhs, int nchunk, const int* __restrict__ gptr,
+                  const int* __restrict__ gsrc, const int* __restrict__ gtid, const float4* __restrict__ T,
+                  const float2* __restrict__ wq, const float4* __restrict__ C, float4* __restrict__ B) {
     const int gr = blockIdx.x / nchunk;
     const int c0 = blockIdx.y * NR;
-    const int k = chunk * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    const size_t K2 = 2 * (size_t)K;
-    float2 acc[G][2][NR];
+    const int k = blockIdx.x % nchunk * 32 + threadIdx.x;   // pair of samples
+    if (k >= KP) return;
+    f32x2 a[G][2 * NR][2], b[G][2 * NR][2];   // sums of C Re T and C Im T, per box, slot and sample
 #pragma unroll
     for (int h = 0; h < G; ++h)
 #pragma unroll
-        for (int u = 0; u < NR; ++u) acc[h][0][u] = acc[h][1][u] = make_float2(0.f, 0.f);
+        for (int u = 0; u < 2 * NR; ++u) a[h][u][0] = a[h][u][1] = b[h][u][0] = b[h][u][1] = 0;
+    const float4* Cu[2 * NR];   // columns past the last read the last one's values
+#pragma unroll
+    for (int u = 0; u < 2 * NR; ++u) Cu[u] = C + (size_t)(2 * min(c0 + u / 2, nrhs - 1) + u % 2) * KP + k;
+    const size_t cstride = 2 * (size_t)nrhs * KP;
+    const float4* Tk = T + k;
     const int e1 = gptr[gr + 1];
     for (int e = gptr[gr]; e < e1; ++e) {
-        int t[G];   // the same for the whole CTA: uniform branches
+        int t[G];   // the same for the whole warp: uniform branches
+        const size_t so = (size_t)gsrc[e] * cstride;
         if (G == 4) {
             const int4 q = reinterpret_cast<const int4*>(gtid)[e];
-            t[0] = q.x; t[1] = q.y; t[2 % G] = q.z; t[3 % G] = q.w;
-        } else {
+            t[0] = q.x; t[1 % G] = q.y; t[2 % G] = q.z; t[3 % G] = q.w;
+        } else if (G == 2) {
             const int2 q = reinterpret_cast<const int2*>(gtid)[e];
             t[0] = q.x; t[1 % G] = q.y;
+        } else {
+            t[0] = gtid[e];
         }
-        const float2* cs = C + ((size_t)gsrc[e] * nrhs + c0) * K2 + k;
-        float2 tv[G];
+        float4 v[2 * NR], w[G];
 #pragma unroll
-        for (int h = 0; h < G; ++h) tv[h] = t[h] >= 0 ? T[(size_t)t[h] * K + k] : make_float2(0.f, 0.f);
+        for (int u = 0; u < 2 * NR; ++u) v[u] = Cu[u][so];
 #pragma unroll
-        for (int u = 0; u < NR; ++u) {
-            if (c0 + u < nrhs) {
-                const float2 p = cs[u * K2], q = cs[u * K2 + K];
+        for (int h = 0; h < G; ++h) ldg128_if(t[h] >= 0, w[h], Tk + (size_t)t[h] * KP);
 #pragma unroll
-                for (int h = 0; h < G; ++h)
-                    if (t[h] >= 0) { fmac(acc[h][0][u], p, tv[h]); fmac(acc[h][1][u], q, tv[h]); }
+        for (int h = 0; h < G; ++h)
+            if (t[h] >= 0) {
+                const f32x2 x0 = pk2(w[h].x, w[h].x), y0 = pk2(w[h].y, w[h].y);
+                const f32x2 x1 = pk2(w[h].z, w[h].z), y1 = pk2(w[h].w, w[h].w);
+#pragma unroll
+                for (int u = 0; u < 2 * NR; ++u) {
+                    const f32x2 p0 = pk2(v[u].x, v[u].y), p1 = pk2(v[u].z, v[u].w);
+                    a[h][u][0] = fma2(p0, x0, a[h][u][0]);
+                    b[h][u][0] = fma2(p0, y0, b[h][u][0]);
+                    a[h][u][1] = fma2(p1, x1, a[h][u][1]);
+                    b[h][u][1] = fma2(p1, y1, b[h][u][1]);
+                }
             }
-        }
     }
-    const float wk = wq[k];
+    const float2 wk = wq[k];
 #pragma unroll
     for (int h = 0; h < G; ++h) {
-        const int b = G * gr + h;
-        if (b >= nb) break;
-        float2* bo = B + ((size_t)b * nrhs + c0) * K2 + k;
+        const int box = G * gr + h;
+        if (box >= nb) break;
 #pragma unroll
-        for (int u = 0; u < NR; ++u) {
-            if (c0 + u < nrhs) {
-                bo[u * K2] = make_float2(acc[h][0][u].x * wk, acc[h][0][u].y * wk);
-                bo[u * K2 + K] = make_float2(acc[h][1][u].x * wk, acc[h][1][u].y * wk);
+        for (int u = 0; u < 2 * NR; ++u)
+            if (c0 + u / 2 < nrhs) {
+                const float2 a0 = up2(a[h][u][0]), b0 = up2(b[h][u][0]), a1 = up2(a[h][u][1]), b1 = up2(b[h][u][1]);
+                B[((size_t)box * nrhs + c0) * 2 * KP + (size_t)u * KP + k] =
+                    make_float4((a0.x - b0.y) * wk.x, (a0.y + b0.x) * wk.x, (a1.x - b1.y) * wk.y, (a1.y + b1.x) * wk.y);
             }
-        }
     }
 }
 
@@ -259,13 +266,27 @@ static int group_lists(Ctx* c, const Level& L, int G, Mixed32::Lv::Grp& M) {
         }
         gptr[g + 1] = (int)gsrc.size();
     }
-    CK(cudaMalloc(&M.ptr, gptr.size() * sizeof(int)));
+    for (int* p : {M.ptr, M.src, M.tid})   // of an attempt that failed
+        if (p) cudaFree(p);
+    M.ptr = M.src = M.tid = nullptr;
     CK(cudaMalloc(&M.src, std::max<size_t>(gsrc.size(), 1) * sizeof(int)));
     CK(cudaMalloc(&M.tid, std::max<size_t>(gtid.size(), 4) * sizeof(int)));
-    CK(cudaMemcpy(M.ptr, gptr.data(), gptr.size() * sizeof(int), cudaMemcpyHostToDevice));
     if (!gsrc.empty()) {
         CK(cudaMemcpy(M.src, gsrc.data(), gsrc.size() * sizeof(int), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(M.tid, gtid.data(), gtid.size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
+    CK(cudaMalloc(&M.ptr, gptr.size() * sizeof(int)));   // last: a set pointer means complete lists
+    CK(cudaMemcpy(M.ptr, gptr.data(), gptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    return MLF_OK;
+}
+
+// lists for groups of 4 boxes, which only mlf_set_translation_group asks for
+static int quad_lists(Ctx* c) {
+    for (int n = 3; n <= c->nlev; ++n) {
+        Mixed32::Lv::Grp& g = c->m32.lv[n].grp[1];
+        if (g.ptr) continue;
+        const int st = group_lists(c, c->lv[n], 4, g);
+        if (st) return st;
     }
     return MLF_OK;
 }
@@ -281,7 +302,6 @@ int mixed_setup(Ctx* c) {
         if ((st = conv32(c, &M.T, L.dT, (size_t)L.ntrans * L.K))) return st;
         if ((st = up32(c, &M.wq, L.wq))) return st;
         if ((st = group_lists(c, L, 2, M.grp[0]))) return st;
-        if ((st = group_lists(c, L, 4, M.grp[1]))) return st;
         if (n < nl) {
             if ((st = up32(c, &M.wth, L.wth))) return st;
             if ((st = up32(c, &M.wph, L.wph))) return st;
@@ -309,6 +329,7 @@ int mixed_setup(Ctx* c) {
     // kernel-wide limit shared by all contexts: the device maximum (see configure_kernels)
     CK(cudaFuncSetAttribute(k_anterp_sep<float2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     CK(cudaFuncSetAttribute(k_interp_sep<float2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    if (c->tr_group == 4 && (st = quad_lists(c))) return st;
     CK(cudaStreamSynchronize(c->stream));
     c->m32.ready = 1;
     return MLF_OK;
@@ -399,35 +420,32 @@ static int matvec32_core(Ctx* c, const double2* x, const float2* x32, double2* y
     if (prof) cudaEventRecord(c->ev[2], s);
     for (int n = 3; n <= nl; ++n) {
         Level& L = c->lv[n];
-        const int bd = 128, nch = (L.K + bd - 1) / bd;
-        const int nr = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8;
-        const dim3 grid(L.nb * nch, (nrhs + nr - 1) / nr);
         const Mixed32::Lv& m = c->m32.lv[n];
-        const int G = c->tr_group ? c->tr_group : (nrhs == 1 ? 2 : 4);
-        if (G > 1 && m.grp[G / 4].ptr) {
-            // box groups: at most 8 sums of each box's two polarisations per thread
-            const Mixed32::Lv::Grp& gl = m.grp[G / 4];
-            const int nrg = std::min(nr, c->tr_cols ? c->tr_cols : (G == 4 ? 2 : 4));
-            const int ng = (L.nb + G - 1) / G;
-            const dim3 gg(ng * nch, (nrhs + nrg - 1) / nrg);
-#define TGRP(NR_, G_) k32_translate_grp<NR_, G_><<<gg, bd, 0, s>>>(L.K, L.nb, nrhs, nch, gl.ptr, gl.src, gl.tid, \
-                                                                  m.T, m.wq, m.C, m.B)
-            if (G == 4) {
-                if (nrg == 1) TGRP(1, 4); else if (nrg == 2) TGRP(2, 4); else TGRP(4, 4);
-            } else {
-                if (nrg == 1) TGRP(1, 2); else if (nrg == 2) TGRP(2, 2); else TGRP(4, 2);
-            }
+        const int G = c->tr_group ? c->tr_group : 2;
+        const int nr = std::min(nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : 4, c->tr_cols ? c->tr_cols : 2);
+        const int KP = L.K / 2, ng = (L.nb + G - 1) / G, ncol = (nrhs + nr - 1) / nr;
+        const int nch = (KP + 31) / 32;
+        const dim3 grid(ng * nch, ncol);
+        const int* gp = G == 1 ? L.dfar_ptr : m.grp[G / 4].ptr;
+        const int* gs = G == 1 ? L.dfar_src : m.grp[G / 4].src;
+        const int* gt = G == 1 ? L.dfar_tid : m.grp[G / 4].tid;
+#define TGRP(NR_, G_)                                                                                              \
+    k32_translate_grp<NR_, G_><<<grid, 32, 0, s>>>(KP, L.nb, nrhs, nch, gp, gs, gt,                          \
+                                                    reinterpret_cast<const float4*>(m.T),                          \
+                                                    reinterpret_cast<const float2*>(m.wq),                         \
+                                                    reinterpret_cast<const float4*>(m.C),                          \
+                                                    reinterpret_cast<float4*>(m.B))
+#define TNR(G_)                                                       \
+    do {                                                              \
+        if (nr == 1) TGRP(1, G_);                                     \
+        else if (nr == 2) TGRP(2, G_);                                \
+        else TGRP(4, G_);                                             \
+    } while (0)
+        if (G == 4) TNR(4);
+        else if (G == 2) TNR(2);
+        else TNR(1);
+#undef TNR
 #undef TGRP
-            continue;
-        }
-        if (nr == 1)
-            k32_translate<1><<<grid, bd, 0, s>>>(L.K, nrhs, nch, L.dfar_ptr, L.dfar_src, L.dfar_tid, m.T, m.wq, m.C, m.B);
-        else if (nr == 2)
-            k32_translate<2><<<grid, bd, 0, s>>>(L.K, nrhs, nch, L.dfar_ptr, L.dfar_src, L.dfar_tid, m.T, m.wq, m.C, m.B);
-        else if (nr == 4)
-            k32_translate<4><<<grid, bd, 0, s>>>(L.K, nrhs, nch, L.dfar_ptr, L.dfar_src, L.dfar_tid, m.T, m.wq, m.C, m.B);
-        else
-            k32_translate<8><<<grid, bd, 0, s>>>(L.K, nrhs, nch, L.dfar_ptr, L.dfar_src, L.dfar_tid, m.T, m.wq, m.C, m.B);
     }
     if (prof) cudaEventRecord(c->ev[3], s);
     for (int n = 4; n <= nl; ++n) {
@@ -1144,6 +1162,12 @@ int mlf_set_gs_passes(mlf_ctx* h, int passes) {
 int mlf_set_translation_group(mlf_ctx* h, int boxes, int cols) {
     if (!h || (boxes != 0 && boxes != 1 && boxes != 2 && boxes != 4) || (cols != 0 && cols != 1 && cols != 2 && cols != 4))
         return MLF_E_ARG;
+    if (boxes == 4 && h->c.m32.ready) {   // before any product that a caller may capture
+        Ctx* c = &h->c;
+        if (!cuda_ok(c, cudaSetDevice(c->dev), "cudaSetDevice")) return MLF_E_CUDA;
+        const int st = quad_lists(c);
+        if (st) return st;
+    }
     h->c.tr_group = boxes;
     h->c.tr_cols = cols;
     return MLF_OK;

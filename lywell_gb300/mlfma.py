@@ -408,9 +408,8 @@ class MLFMA:
 
     def set_translation_group(self, boxes: int = 0, cols: int = 0):
         """FP32 translation over the merged far lists of 2 or 4 consecutive
-        boxes per thread, 1 box at a time, or 0 (the default): 2 for one
-        column, 4 for blocks; cols = columns per thread with grouped boxes
-        (0: automatic)."""
+        boxes per thread, 1 box at a time, or 0 (the default): 2; cols =
+        columns per thread (0, the default: 2)."""
         _check(load().mlf_set_translation_group(self._h, int(boxes), int(cols)), self._h)
 
     def matvec32(self, x):
