@@ -189,6 +189,109 @@ k32_translate_grp(int KP, int nb, int nrhs, int nchunk, const int* __restrict__ 
     }
 }
 
+// FP32 interpolation between octree levels (the separable upward pass of
+// mlf_sep.cuh) for NS field slots (columns x polarisations of a box) a thread,
+// with packed FMAs on (Re, Im).  Slots past the last read the last one's values.
+//   Cp(ip, it) = sum over the children of shift * sum_b wph sum_a wth Cc
+// blockIdx.x = (parent, slot group, slab of `rows` coarse theta rows); thread =
+// coarse sample (ip, it), so its stencil indices and weights are loaded once for
+// all children and slots; slabs are cut so that their samples fill a CTA of at
+// most IN32_T threads.  Y (shared memory, two buffers, [fine phi][row] with the
+// NS slots side by side, padded to NS + 2: no bank conflicts at 16 bytes) =
+// theta pass of one child; the phi pass sums v Re(shift) and v Im(shift) over
+// the children in registers.  Latency bounds it, so warps in flight count:
+// four slots at 64 registers (1.06 ms on the 69120-RWG sphere, 16 columns)
+// against eight (1.11) and CTAs of 384 (1.48); with 8-row slabs, 256 threads
+// and the parent slab in shared memory it was 1.34 ms.  One column of the
+// 122880-RWG sphere: 0.163 -> 0.141 ms.
+constexpr int IN32_T = 256;
+template <int NS>
+__global__ void __launch_bounds__(IN32_T, NS == 2 ? 6 : 4)
+k32_interp(int Lp, int Lc, int nslot, int nsg, int nslab, int rows, const int* __restrict__ child_ptr,
+           const int* __restrict__ octant, const int* __restrict__ sth, const float* __restrict__ wth,
+           const int* __restrict__ sph, const float* __restrict__ wph, const float2* __restrict__ shift,
+           const float2* __restrict__ Cc, float2* __restrict__ Cp) {
+    extern __shared__ __align__(16) unsigned char sep_smem[];
+    constexpr int SS = NS + 2;   // float2 per intermediate sample
+    float2* Y = reinterpret_cast<float2*>(sep_smem);
+    const int slab = blockIdx.x % nslab, sg = blockIdx.x / nslab % nsg, P = blockIdx.x / nslab / nsg;
+    const int q0 = sg * NS, i0 = slab * rows, nr = min(rows, Lp - i0);
+    const int Kp = 2 * Lp * Lp, Kc = 2 * Lc * Lc;
+    const int hi = threadIdx.x / nr, li = threadIdx.x - hi * nr;   // column (fine phi, then coarse phi), row
+    const bool th_on = hi < 2 * Lc, ph_on = hi < 2 * Lp;
+    int fa[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
+    f32x2 wa[3], wb[3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        float w = 0.f;
+        if (th_on) { w = wth[3 * (i0 + li) + t]; fa[t] = sth[3 * (i0 + li) + t] + hi * Lc; }
+        wa[t] = pk2(w, w);
+        w = 0.f;
+        if (ph_on) { w = wph[3 * hi + t]; fb[t] = (sph[3 * hi + t] * rows + li) * SS; }
+        wb[t] = pk2(w, w);
+    }
+    const int ks = hi * Lp + i0 + li;   // coarse sample
+    f32x2 sr[NS], si[NS];
+#pragma unroll
+    for (int u = 0; u < NS; ++u) sr[u] = si[u] = 0;
+    const int c0 = child_ptr[P], c1 = child_ptr[P + 1], nbuf = 2 * Lc * rows * SS;
+    for (int cb = c0; cb < c1; ++cb) {
+        float2* Yb = Y + ((cb - c0) & 1) * nbuf;
+        if (th_on) {
+            const float2* src = Cc + ((size_t)cb * nslot + q0) * Kc;
+            f32x2 y[NS];
+#pragma unroll
+            for (int u = 0; u < NS; ++u) {
+                const float2* col = src + (size_t)min(u, nslot - 1 - q0) * Kc;
+                y[u] = 0;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    const float2 v = col[fa[t]];
+                    y[u] = fma2(pk2(v.x, v.y), wa[t], y[u]);
+                }
+            }
+            float4* d = reinterpret_cast<float4*>(Yb + (hi * rows + li) * SS);
+#pragma unroll
+            for (int u = 0; u < NS; u += 2) {
+                const float2 v0 = up2(y[u]), v1 = up2(y[u + 1]);
+                d[u / 2] = make_float4(v0.x, v0.y, v1.x, v1.y);
+            }
+        }
+        __syncthreads();   // two buffers: one barrier a child
+        if (ph_on) {
+            const float2 z = shift[(size_t)octant[cb] * Kp + ks];
+            const f32x2 zr = pk2(z.x, z.x), zi = pk2(z.y, z.y);
+            f32x2 v[NS];
+#pragma unroll
+            for (int u = 0; u < NS; ++u) v[u] = 0;
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const float4* yq = reinterpret_cast<const float4*>(Yb + fb[t]);
+#pragma unroll
+                for (int u = 0; u < NS; u += 2) {
+                    const float4 q = yq[u / 2];
+                    v[u] = fma2(pk2(q.x, q.y), wb[t], v[u]);
+                    v[u + 1] = fma2(pk2(q.z, q.w), wb[t], v[u + 1]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < NS; ++u) {
+                sr[u] = fma2(v[u], zr, sr[u]);
+                si[u] = fma2(v[u], zi, si[u]);
+            }
+        }
+    }
+    if (ph_on) {
+        float2* dst = Cp + ((size_t)P * nslot + q0) * Kp + ks;
+#pragma unroll
+        for (int u = 0; u < NS; ++u)
+            if (q0 + u < nslot) {
+                const float2 a = up2(sr[u]), b = up2(si[u]);
+                dst[(size_t)u * Kp] = make_float2(a.x - b.y, a.y + b.x);
+            }
+    }
+}
+
 __global__ void k32_receive_near(int K, int N, int nrhs, int ld, const int* __restrict__ perm,
                                  const int* __restrict__ box_of_sorted, const float2* __restrict__ R,
                                  const float2* __restrict__ A, const int* __restrict__ ia, const int* __restrict__ ja,
@@ -329,6 +432,8 @@ int mixed_setup(Ctx* c) {
     // kernel-wide limit shared by all contexts: the device maximum (see configure_kernels)
     CK(cudaFuncSetAttribute(k_anterp_sep<float2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     CK(cudaFuncSetAttribute(k_interp_sep<float2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    CK(cudaFuncSetAttribute(k32_interp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    CK(cudaFuncSetAttribute(k32_interp<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     if (c->tr_group == 4 && (st = quad_lists(c))) return st;
     CK(cudaStreamSynchronize(c->stream));
     c->m32.ready = 1;
@@ -366,7 +471,7 @@ int device_matvec32_from32(Ctx* c, const float2* x32, double2* y, int nrhs, cuda
     return matvec32_core(c, nullptr, x32, y, nrhs, c->N, s);
 }
 
-// Field slots (columns x polarisations) per CTA of the separable passes: the
+// Field slots (columns x polarisations) per CTA of the anterpolation: the
 // largest of 8, 4, 2 that divides 2 nrhs and keeps the CTA within 48 KB of
 // shared memory (four CTAs per SM), else 1.  The slots share every index and
 // weight load of the stencils.
@@ -407,15 +512,28 @@ static int matvec32_core(Ctx* c, const double2* x, const float2* x32, double2* y
     for (int n = nl; n >= 4; --n) {
         Level& Lc = c->lv[n];
         Level& Lp = c->lv[n - 1];
-        const int nslab = (Lp.L + SEP_SLAB - 1) / SEP_SLAB;
-        const size_t per = (size_t)SEP_SLAB * 2 * (Lc.L + Lp.L) * sizeof(float2);   // child rows + parent slab
         const Mixed32::Lv &mp = c->m32.lv[n - 1], &mc = c->m32.lv[n];
-        slots_dispatch(nrhs, per, [&](auto ns) {
-            constexpr int NS = decltype(ns)::value;
-            k_interp_sep<float2, NS><<<Lp.nb * (2 * nrhs / NS) * nslab, 256, NS * per, s>>>(
-                Lp.L, Lc.L, nrhs, nslab, Lp.dchild_ptr, Lc.doctant, Lp.dsth, mp.wth, Lp.dsph, mp.wph, mp.shift, mc.C,
-                mp.C);
-        });
+        if (Lc.L <= Lp.L && 2 * Lp.L <= IN32_T) {
+            // slabs of coarse theta rows whose samples fill the CTA
+            const int most = IN32_T / (2 * Lp.L), nslab = (Lp.L + most - 1) / most, rows = (Lp.L + nslab - 1) / nslab;
+            const int threads = (rows * 2 * Lp.L + 31) / 32 * 32;
+            auto launch = [&](auto ns) {
+                constexpr int NS = decltype(ns)::value;
+                const int nsg = (2 * nrhs + NS - 1) / NS;
+                const size_t smem = (size_t)2 * 2 * Lc.L * rows * (NS + 2) * sizeof(float2);
+                k32_interp<NS><<<Lp.nb * nsg * nslab, threads, smem, s>>>(
+                    Lp.L, Lc.L, 2 * nrhs, nsg, nslab, rows, Lp.dchild_ptr, Lc.doctant, Lp.dsth, mp.wth, Lp.dsph,
+                    mp.wph, mp.shift, mc.C, mp.C);
+            };
+            if (nrhs == 1) launch(std::integral_constant<int, 2>());
+            else launch(std::integral_constant<int, 4>());
+            continue;
+        }
+        const int nslab = (Lp.L + SEP_SLAB - 1) / SEP_SLAB;
+        const size_t smem = (size_t)SEP_SLAB * 2 * (Lc.L + Lp.L) * sizeof(float2);   // child rows + parent slab
+        k_interp_sep<float2, 1><<<Lp.nb * 2 * nrhs * nslab, 256, smem, s>>>(
+            Lp.L, Lc.L, nrhs, nslab, Lp.dchild_ptr, Lc.doctant, Lp.dsth, mp.wth, Lp.dsph, mp.wph, mp.shift, mc.C,
+            mp.C);
     }
     if (prof) cudaEventRecord(c->ev[2], s);
     for (int n = 3; n <= nl; ++n) {
