@@ -486,7 +486,10 @@ int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, c
     const int nl = c->nlev;
     Level& leaf = c->lv[nl];
     if (ev) cudaEventRecord(ev[0], s);
-    k_aggregate<<<leaf.nb * nrhs, 256, 0, s>>>(leaf.K, nrhs, ld, c->dbox_ptr, c->dperm, c->dR, x, Cf[nl]);
+    const bool split = split64_on(c, nrhs);   // full boxes and several columns: on the tensor cores
+    int st;
+    if (!split) k_aggregate<<<leaf.nb * nrhs, 256, 0, s>>>(leaf.K, nrhs, ld, c->dbox_ptr, c->dperm, c->dR, x, Cf[nl]);
+    else if ((st = split64_aggregate(c, x, nrhs, ld, Cf[nl], s))) return st;
     if (ev) cudaEventRecord(ev[1], s);
     for (int n = nl; n >= 4; --n) {
         Level& Lc = c->lv[n];
@@ -516,12 +519,15 @@ int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, c
     }
     if (ev) cudaEventRecord(ev[4], s);
     {
-        const int warps = c->N * nrhs;
         const double facy = c->ph.w * MU / (4. * PI);
-        k_receive_near_d<<<chunks(warps * 32, 256), 256, 0, s>>>(leaf.K, c->N, nrhs, ld, c->dperm,
-                                                                  c->dbox_of_sorted, c->dR,
-                                                                  nl == 3 ? Bf[nl] : Af[nl], c->dia,
-                                                                  c->dja, c->dZd, x, facy, y);
+        const double2* Al = nl == 3 ? Bf[nl] : Af[nl];
+        if (split) {
+            if ((st = split64_receive_near(c, x, Al, facy, nrhs, ld, y, s))) return st;
+        } else {
+            k_receive_near_d<<<chunks(c->N * nrhs * 32, 256), 256, 0, s>>>(leaf.K, c->N, nrhs, ld, c->dperm,
+                                                                           c->dbox_of_sorted, c->dR, Al, c->dia,
+                                                                           c->dja, c->dZd, x, facy, y);
+        }
     }
     if (ev) cudaEventRecord(ev[5], s);
     return launch_check(c, "matvec");
@@ -532,6 +538,7 @@ int device_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaSt
     if (c->mv_prec == 1) return device_matvec32(c, x, y, nrhs, ld, s);
     int st;
     if ((st = ensure_fields(c, nrhs))) return st;
+    if (split64_on(c, nrhs) && (st = split64_ready(c, nrhs))) return st;
     c->last_nrhs = nrhs;
     double2* Cf[32] = {nullptr};
     double2* Bf[32] = {nullptr};
@@ -585,7 +592,7 @@ void device_free(Ctx* c) {
     F(c->dR); F(c->dperm); F(c->dbox_ptr); F(c->dbox_of_sorted); F(c->dia); F(c->dja); F(c->dZ);
     F(c->dp_coord); F(c->dt_baric); F(c->dt_baric_sub); F(c->de_long); F(c->de_centro); F(c->de_t);
     F(c->de_po); F(c->dalu); F(c->djlu); F(c->dju); F(c->dlvl_rows_f); F(c->dlvl_rows_b);
-    F(c->dalu64); F(c->drcs_edge); F(c->drcs_ws);
+    F(c->dalu64); F(c->doz_tiles); F(c->doz_pat); F(c->doz_exp); F(c->doz_ws); F(c->drcs_edge); F(c->drcs_ws);
     F(c->dwork); F(c->dscal); F(c->dflags); F(c->dx_io); F(c->dy_io); F(c->dMinv); F(c->dZd); F(c->dboff); F(c->dMinv32); F(c->dpre_xs); F(c->dZdense); F(c->dMinv_base);
     mixed_free(c);
     near_blocks_free(c);

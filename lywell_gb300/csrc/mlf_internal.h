@@ -169,6 +169,14 @@ struct Ctx {
     int *dia = nullptr, *dja = nullptr;
     float2* dZ = nullptr;
     double2* dZd = nullptr;           // the same near values as complex(8)
+    // FP64 products on blocks of columns (mlf_split64.cu): row tiles (box, first
+    // row), the patterns' exponents, the call's exponents (x's rows, Z's rows,
+    // columns) and the near sums [split][column][box-sorted place]
+    int2* doz_tiles = nullptr;
+    int *doz_pat = nullptr, *doz_exp = nullptr;
+    int noz_tiles = 0, nsm = 0;
+    double2* doz_ws = nullptr;
+    size_t oz_cap = 0;
     // device geometry for set-up kernels and RCS
     double *dp_coord = nullptr, *dt_baric = nullptr, *dt_baric_sub = nullptr, *de_long = nullptr,
            *de_centro = nullptr;
@@ -247,6 +255,12 @@ int ensure_work(Ctx* c, size_t n_double2);
 int device_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s);
 int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s,
                        double2* const* Cf, double2* const* Bf, double2* const* Af, cudaEvent_t* ev);
+// FP64 near field, leaf aggregation and receive on blocks of columns (mlf_split64.cu)
+bool split64_on(const Ctx* c, int nrhs);
+int split64_ready(Ctx* c, int nrhs);
+int split64_aggregate(Ctx* c, const double2* x, int nrhs, int ld, double2* C, cudaStream_t s);
+int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy, int nrhs, int ld, double2* y,
+                         cudaStream_t s);
 int device_ilu_upload(Ctx* c);
 int device_ilu_solve(Ctx* c, const double2* y, double2* x, int nrhs, cudaStream_t s);
 int device_cgs(Ctx* c, const double2* b, const double2* x0, double tol, int maxit, int nrhs,

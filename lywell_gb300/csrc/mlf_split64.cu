@@ -1,0 +1,480 @@
+// FP64 near field, leaf aggregation and leaf receive on blocks of columns, on
+// the tensor cores, by exact splitting into 8-bit digits (Ozaki, Ogita, Oishi
+// and Rump 2012; on FP16 matrix units Mukunoki et al. 2020).
+//
+// All three are a complex GEMM per leaf box (llenar_campoCyB,
+// modMLFMA.f90:1805-1811; MatxVec_MLFMA, :1915-1942):
+//   near       y_m = sum_k Z_mk x_k     the box's bases over its near list S,
+//                                       which they share; Z complex(4)
+//   receive    y_m = sum_k conj(R_mk) A_k   its bases over the 2K directions
+//   aggregate  C_q = sum_k R_kq x_k     the directions over its bases
+// GB300 does 2 DFMA a clock and SM, which bounds them whatever the number of
+// columns; an FP16 product of two integers below 2^8 is exact, and so is its
+// FP32 sum.  Both operands become 62-bit integers relative to a power of two
+// above the largest value of the row or column, cut into eight signed digits in
+// [-128, 127] of weight 2^(8 (7 - i)).  The 36 digit products with i + j <= 7
+// are summed per s = i + j in FP32 over 64 real terms: at most 8 * 64 * 2^14 =
+// 2^23, exact; then the eight sums are joined in 64-bit integers over all terms,
+// and rounded to double once at the end.  In the near field each source k is
+// scaled by a power of two before that: x_k to magnitude one (over the block's
+// columns), Z's column k by the inverse, so that a row's integers are relative
+// to its largest term |Z_mk x_k|: what is lost lies below 2^-62 of that, whatever
+// the range of x or Z, where a sum in double precision loses 2^-53 of its
+// partial sums.  Measured on a 7680-unknown list against extended precision:
+// relative error 1.8e-16 (rms over rows), 1.7e-15 with FP64 FMAs; the same with
+// x over six decades.
+//
+// mma.sync keeps each digit sum in the registers of the warp that joins it.
+// 12000-RWG spheroid (49 M near entries), 24 columns, before -> now: near +
+// receive 8.66 -> 1.66 ms, aggregation 1.00 -> 0.18 ms.
+//
+// A row or column with an Inf or a NaN gives NaN in its results.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+#include "mlf_internal.h"
+
+namespace mlf {
+
+#define CK(call)                                             \
+    do {                                                     \
+        if (!cuda_ok(c, (call), #call)) return MLF_E_CUDA;   \
+    } while (0)
+
+constexpr int OZ_D = 8;            // digits
+constexpr int OZ_R = 64;           // rows (bases of one box) per CTA
+constexpr int OZ_C = 12;           // complex columns per CTA
+constexpr int OZ_K = 32;           // bases of S per step: 64 real terms
+constexpr int OZ_PITCH = 4 * OZ_K + 16;                    // bytes of a row of 64 FP16, padded: ldmatrix without conflicts
+constexpr int OZ_ABYTES = OZ_D * OZ_R * OZ_PITCH;          // Z digits  [digit][row][term]
+constexpr int OZ_BBYTES = OZ_D * 2 * OZ_C * OZ_PITCH;      // x digits  [digit][real column][term]
+constexpr int OZ_STAGE = OZ_ABYTES + OZ_BBYTES;
+constexpr int OZ_SMEM = 2 * OZ_STAGE + (OZ_R + OZ_C) * 4;
+constexpr int OZ_WARPS = 12;       // 4 tiles of 16 rows x 3 of 8 real columns
+constexpr int OZ_THREADS = 32 * OZ_WARPS;
+constexpr int OZ_WR = (OZ_R + OZ_WARPS - 1) / OZ_WARPS;   // rows that a warp converts
+static_assert(OZ_C == OZ_WARPS && 2 * OZ_C == 8 * (OZ_WARPS / 4), "a warp converts one column and multiplies one tile");
+constexpr int OZ_MAX_SPLIT = 4;
+
+// |v| < 2^e to an integer below 2^62, truncated: v = m 2^(e - 62)
+__device__ __forceinline__ long long oz_fix(unsigned long long m62, int t, uint32_t sign) {
+    const long long m = (long long)(m62 >> min(t, 63));
+    return sign ? -m : m;
+}
+__device__ __forceinline__ long long oz_fix(float v, int e) {
+    const uint32_t b = __float_as_uint(v);
+    const int ef = (b >> 23) & 0xff;
+    const uint32_t mant = (b & 0x7fffffu) | (ef ? 0x800000u : 0u);
+    return oz_fix((unsigned long long)mant << 38, e + 126 - max(ef, 1), b >> 31);
+}
+__device__ __forceinline__ long long oz_fix(double v, int e) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ef = (int)(b >> 52) & 0x7ff;
+    const unsigned long long mant = (b & 0xfffffffffffffull) | (ef ? 0x10000000000000ull : 0ull);
+    return oz_fix(mant << 9, e + 1022 - max(ef, 1), (uint32_t)(b >> 63));
+}
+
+// exponent e with |v| < 2^e of the larger of two magnitudes, OZ_ZERO for zeros,
+// OZ_BAD for an Inf or a NaN
+constexpr int OZ_ZERO = -100000, OZ_BAD = 100000;
+__device__ __forceinline__ int oz_exp(float2 v) {
+    const uint32_t m = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+    const int ef = (int)(m >> 23);
+    return m == 0 ? OZ_ZERO : ef == 0xff ? OZ_BAD : max(ef, 1) - 126;
+}
+__device__ __forceinline__ int oz_exp(double2 v) {
+    const uint32_t m = max((uint32_t)__double2hiint(v.x) & 0x7fffffffu, (uint32_t)__double2hiint(v.y) & 0x7fffffffu);
+    const int ef = (int)(m >> 20);
+    return ef == 0x7ff ? OZ_BAD : max(ef, 1) - 1022;   // zeros count as the smallest number
+}
+
+// sexp[n] = exponent of x's row n over the columns
+__global__ void k_row_exp(int N, int nrhs, int ld, const double2* __restrict__ x, int* __restrict__ sexp) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= N) return;
+    int e = OZ_ZERO;
+    for (int c = 0; c < nrhs; ++c) e = max(e, oz_exp(x[(size_t)c * ld + n]));
+    sexp[n] = e == OZ_BAD ? 0 : e;
+}
+
+// rexp[pos] = exponent of row perm[pos] of Z 2^sexp; a warp per row
+__global__ void k_near_exp(int N, const int* __restrict__ perm, const int* __restrict__ ia, const int* __restrict__ ja,
+                           const float2* __restrict__ Z, const int* __restrict__ sexp, int* __restrict__ rexp) {
+    const int pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (pos >= N) return;
+    const int n = perm[pos], q1 = ia[n + 1];
+    int e = OZ_ZERO;
+#pragma unroll 4
+    for (int q = ia[n] + lane; q < q1; q += 32) e = max(e, oz_exp(Z[q]) + sexp[ja[q]]);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) rexp[pos] = e;
+}
+
+enum { OZ_NEAR = 0, OZ_RECEIVE = 1, OZ_AGGREGATE = 2 };
+
+// cexp[box * nrhs + c] = exponent of column c of the box's right-hand operand:
+// x 2^-sexp over the near list, the field A over its 2K directions, or x over
+// the box's bases; a CTA per pair
+template <int MODE>
+__global__ void k_col_exp(int nrhs, int ld, int K2, const int* __restrict__ box_ptr, const int* __restrict__ perm,
+                          const int* __restrict__ ia, const int* __restrict__ ja, const double2* __restrict__ x,
+                          const int* __restrict__ sexp, int* __restrict__ cexp) {
+    const int b = blockIdx.x / nrhs, c = blockIdx.x % nrhs;
+    __shared__ int top;
+    if (threadIdx.x == 0) top = OZ_ZERO;
+    __syncthreads();
+    int e = OZ_ZERO;
+    if (MODE == OZ_NEAR) {
+        const int n = perm[box_ptr[b]], q1 = ia[n + 1];
+        for (int q = ia[n] + threadIdx.x; q < q1; q += blockDim.x)
+            e = max(e, oz_exp(x[(size_t)c * ld + ja[q]]) - sexp[ja[q]]);
+    } else if (MODE == OZ_RECEIVE) {
+        for (int q = threadIdx.x; q < K2; q += blockDim.x) e = max(e, oz_exp(x[(size_t)blockIdx.x * K2 + q]));
+    } else {
+        for (int q = box_ptr[b] + threadIdx.x; q < box_ptr[b + 1]; q += blockDim.x)
+            e = max(e, oz_exp(x[(size_t)c * ld + perm[q]]));
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&top, e);
+    __syncthreads();
+    if (threadIdx.x == 0) cexp[blockIdx.x] = top;
+}
+
+// exponents of the patterns, once per context: of each basis over the directions
+// (a warp per basis), and of each box's directions over its bases
+__global__ void k_pattern_exp(int N, int K2, const double2* __restrict__ R, int* __restrict__ rexp) {
+    const int pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (pos >= N) return;
+    int e = OZ_ZERO;
+    for (int q = lane; q < K2; q += 32) e = max(e, oz_exp(R[(size_t)pos * K2 + q]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) rexp[pos] = e;
+}
+__global__ void k_direction_exp(int K2, const int* __restrict__ box_ptr, const double2* __restrict__ R,
+                                int* __restrict__ qexp) {
+    const int b = blockIdx.x;
+    for (int q = threadIdx.x; q < K2; q += blockDim.x) {
+        int e = OZ_ZERO;
+        for (int t = box_ptr[b]; t < box_ptr[b + 1]; ++t) e = max(e, oz_exp(R[(size_t)t * K2 + q]));
+        qexp[(size_t)b * K2 + q] = e;
+    }
+}
+
+// The digits of (re, im) as FP16 pairs, most significant first: with 128 added
+// to every digit the bytes of the integer are the biased digits; 0x6400 | byte
+// is 1024 + byte in FP16.
+__device__ __forceinline__ void oz_digits(long long re, long long im, uint32_t (&d)[OZ_D]) {
+    const unsigned long long bias = 0x8080808080808080ull;
+    const unsigned long long r = (unsigned long long)re + bias, i = (unsigned long long)im + bias;
+    const uint32_t w[4] = {(uint32_t)(r >> 32), (uint32_t)(i >> 32), (uint32_t)r, (uint32_t)i};
+    const __half2 off = __float2half2_rn(-1152.f);
+#pragma unroll
+    for (int q = 0; q < OZ_D; ++q) {
+        const int byte = 3 - (q & 3);   // of the high words, then of the low ones
+        const uint32_t x = (__byte_perm(w[q / 4 * 2], w[q / 4 * 2 + 1], byte | (4 + byte) << 8) & 0x00ff00ffu) | 0x64006400u;
+        const __half2 h = __hadd2(*reinterpret_cast<const __half2*>(&x), off);
+        d[q] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// 2^(er + ec - 68) (hi 2^32 + lo): digit i weighs 2^(e - 62 + 8 (7 - i)), the sum
+// s of hi and lo 2^(8 (7 - s)) of 2^(er + ec - 124 + 56)
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int er, int ec) {
+    return ldexp(fma((double)hi, 4294967296.0, (double)lo), er + ec - 68);
+}
+
+struct OzArgs {
+    int N, nrhs, ld, K2;                // K2 = 2K, the leaf's samples of both polarisations
+    const int2* tiles;                  // (box, first row)
+    const int *box_ptr, *perm, *ia, *ja;
+    const float2* Z;
+    const double2 *R, *x;               // x: right-hand operand (receive: the field A)
+    const int *sexp, *rexp, *cexp;      // exponents of sources (near), rows and columns
+    double2* out;                       // near: [split][col][box-sorted place]; receive: y; aggregate: the field C
+    const double2* near;                // receive: the near field's parts
+    int nsplit;
+    double facy;
+};
+
+template <int MODE> struct OzLeft { typedef double2 T; };
+template <> struct OzLeft<OZ_NEAR> { typedef float2 T; };
+
+// blockIdx.x = (row tile, block of 12 columns), .y = part of the near list.  While one step's
+// digits are multiplied the next step's are made in the other stage, half of the
+// warps beginning with the one, half with the other, and the values of the step
+// after are on their way to registers.
+template <int MODE>
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
+    typedef typename OzLeft<MODE>::T ZT;
+    extern __shared__ __align__(16) unsigned char oz_smem[];
+    int* er = reinterpret_cast<int*>(oz_smem + 2 * OZ_STAGE);   // exponent of each row
+    int* ec = er + OZ_R;                                         // ... and of each column
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nqt = (g.K2 + OZ_R - 1) / OZ_R;
+    const int ncb = (g.nrhs + OZ_C - 1) / OZ_C, tile = blockIdx.x / ncb;
+    const int2 tl = MODE == OZ_AGGREGATE ? make_int2(tile / nqt, tile % nqt * OZ_R) : g.tiles[tile];
+    const int b0 = g.box_ptr[tl.x], nb = g.box_ptr[tl.x + 1] - b0;
+    const int p0 = b0 + tl.y;                                    // near, receive: rows p0 .. p0 + nr - 1
+    const int nr = min(OZ_R, (MODE == OZ_AGGREGATE ? g.K2 : nb) - tl.y);
+    const int c0 = blockIdx.x % ncb * OZ_C, nc = min(OZ_C, g.nrhs - c0);
+    const int s0 = MODE == OZ_NEAR ? g.ia[g.perm[b0]] : 0;
+    const int len = MODE == OZ_NEAR ? g.ia[g.perm[b0] + 1] - s0 : MODE == OZ_RECEIVE ? g.K2 : nb;
+    const int nstep = (len + OZ_K - 1) / OZ_K;
+    const int k0 = (int)((long long)nstep * blockIdx.y / gridDim.y) * OZ_K;
+    const int k1 = min(len, (int)((long long)nstep * (blockIdx.y + 1) / gridDim.y) * OZ_K);
+    const int* rexp = g.rexp + (MODE == OZ_AGGREGATE ? (size_t)tl.x * g.K2 + tl.y : (size_t)p0);
+    if (tid < OZ_R) er[tid] = tid < nr ? rexp[tid] : OZ_ZERO;
+    if (tid < OZ_C) ec[tid] = tid < nc ? g.cexp[(size_t)tl.x * g.nrhs + c0 + tid] : OZ_ZERO;
+    __syncthreads();
+    // warp w converts the rows w, w + 12, ... and the column w
+    const ZT* zrow[OZ_WR];
+#pragma unroll
+    for (int r = 0; r < OZ_WR; ++r) {
+        const int row = min(warp + OZ_WARPS * r, nr - 1);
+        if constexpr (MODE == OZ_NEAR) zrow[r] = g.Z + g.ia[g.perm[p0 + row]];
+        else if constexpr (MODE == OZ_RECEIVE) zrow[r] = g.R + (size_t)(p0 + row) * g.K2;
+        else zrow[r] = g.R + (size_t)b0 * g.K2 + tl.y + row;
+    }
+    const int col = c0 + min(warp, nc - 1);
+    const double2* xc = MODE == OZ_RECEIVE ? g.x + ((size_t)tl.x * g.nrhs + col) * g.K2 : g.x + (size_t)col * g.ld;
+    auto source = [&](int k) {   // of the right-hand operand; k includes the lane
+        if (k >= k1) return -1;
+        return MODE == OZ_NEAR ? g.ja[s0 + k] : MODE == OZ_RECEIVE ? k : g.perm[b0 + k];
+    };
+    auto shift = [&](int j) { return MODE == OZ_NEAR && j >= 0 ? g.sexp[j] : 0; };
+    ZT z[OZ_WR];
+    double2 xv;
+    auto load = [&](int k, int j) {
+#pragma unroll
+        for (int r = 0; r < OZ_WR; ++r) {
+            z[r].x = z[r].y = 0;
+            if (j >= 0 && warp + OZ_WARPS * r < nr) {
+                z[r] = zrow[r][MODE == OZ_AGGREGATE ? (size_t)k * g.K2 : (size_t)k];
+                if (MODE == OZ_RECEIVE) z[r].y = -z[r].y;
+            }
+        }
+        xv = j >= 0 && warp < nc ? xc[j] : make_double2(0, 0);
+    };
+    // the loaded values to digits in stage `st`
+    auto convert = [&](unsigned char* st, int se) {
+        uint32_t d[OZ_D];
+#pragma unroll
+        for (int r = 0; r < OZ_WR; ++r) {
+            const int row = warp + OZ_WARPS * r;
+            if (row >= OZ_R) break;
+            const int e = er[row] - se;
+            oz_digits(oz_fix(z[r].x, e), oz_fix(z[r].y, e), d);
+#pragma unroll
+            for (int q = 0; q < OZ_D; ++q)
+                *reinterpret_cast<uint32_t*>(st + (q * OZ_R + row) * OZ_PITCH + lane * 4) = d[q];
+        }
+        const int e = ec[warp] + se;
+        oz_digits(oz_fix(xv.x, e), oz_fix(xv.y, e), d);
+#pragma unroll
+        for (int q = 0; q < OZ_D; ++q) {   // (Re x, -Im x) for Re y, (Im x, Re x) for Im y
+            unsigned char* row = st + OZ_ABYTES + (q * 2 * OZ_C + 2 * warp) * OZ_PITCH + lane * 4;
+            *reinterpret_cast<uint32_t*>(row) = d[q] ^ 0x80000000u;
+            *reinterpret_cast<uint32_t*>(row + OZ_PITCH) = __byte_perm(d[q], 0, 0x1032);
+        }
+    };
+    const int mt = warp & 3, nt = warp >> 2;   // row tile, column tile
+    const bool mine = mt * 16 < nr && nt * 4 < nc;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(oz_smem);
+    const uint32_t a_addr = base + (mt * 16 + (lane & 15)) * OZ_PITCH + (lane >> 4) * 16;
+    const uint32_t b_addr = base + OZ_ABYTES + (lane >> 4) * (2 * OZ_C * OZ_PITCH) +
+                            (nt * 8 + (lane & 7)) * OZ_PITCH + ((lane >> 3) & 1) * 16;
+    long long hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0};
+    auto products = [&](uint32_t off) {
+        float acc[OZ_D][4];
+#pragma unroll
+        for (int s = 0; s < OZ_D; ++s)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[s][q] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 2 * OZ_K / 16; ++ks) {
+            uint32_t b[OZ_D / 2][4];   // digits 2 p and 2 p + 1
+#pragma unroll
+            for (int p = 0; p < OZ_D / 2; ++p) ldsm4(b[p], b_addr + off + 2 * p * (2 * OZ_C * OZ_PITCH) + ks * 32);
+#pragma unroll
+            for (int i = 0; i < OZ_D; ++i) {
+                uint32_t a[4];
+                ldsm4(a, a_addr + off + i * (OZ_R * OZ_PITCH) + ks * 32);
+#pragma unroll
+                for (int j = 0; i + j < OZ_D; ++j)
+                    mma_f16(acc[i + j], a, b[j / 2][2 * (j & 1)], b[j / 2][2 * (j & 1) + 1]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            long long v[OZ_D];
+#pragma unroll
+            for (int s = 0; s < OZ_D; ++s) v[s] = __float2int_rn(acc[s][q]);
+            hi[q] += v[0] * 16777216 + v[1] * 65536 + v[2] * 256 + v[3];
+            lo[q] += v[4] * 16777216 + v[5] * 65536 + v[6] * 256 + v[7];
+        }
+    };
+    int j = source(k0 + lane), jn = source(k0 + OZ_K + lane);   // of the next step to convert, and the one after
+    load(k0 + lane, j);
+    int se = shift(j);
+    convert(oz_smem, se);
+    auto turn = [&](int k) {   // the loads that the following steps need
+        j = jn;
+        load(k + lane, j);
+        se = shift(j);
+        jn = source(k + OZ_K + lane);
+    };
+    turn(k0 + OZ_K);
+    int st = 0;
+    for (int kb = k0; kb < k1; kb += OZ_K, st ^= 1) {
+        __syncthreads();   // this step's digits are there, the other stage has been multiplied
+        auto next = [&]() {
+            if (kb + OZ_K >= k1) return;
+            convert(oz_smem + (st ^ 1) * OZ_STAGE, se);
+            turn(kb + 2 * OZ_K);
+        };
+        if ((warp >> 2) & 1) next();
+        if (mine) products(st * OZ_STAGE);
+        if (!((warp >> 2) & 1)) next();
+    }
+    if (!mine) return;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    const int cc = nt * 4 + (lane & 3);
+    if (cc >= nc) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int row = mt * 16 + 8 * h + (lane >> 2);
+        if (row >= nr) continue;
+        const int e = er[row], f = ec[cc];
+        double2 v = make_double2(oz_value(hi[2 * h], lo[2 * h], e, f), oz_value(hi[2 * h + 1], lo[2 * h + 1], e, f));
+        if (e > OZ_BAD / 2 || f > OZ_BAD / 2) v = make_double2(nan, nan);
+        if (MODE == OZ_NEAR) {
+            g.out[((size_t)blockIdx.y * g.nrhs + c0 + cc) * g.N + p0 + row] = v;
+        } else if (MODE == OZ_AGGREGATE) {
+            g.out[((size_t)tl.x * g.nrhs + c0 + cc) * g.K2 + tl.y + row] = v;
+        } else {   // y = j facy v + near
+            double2 w = make_double2(0, 0);
+            for (int p = 0; p < g.nsplit; ++p) {
+                const double2 t = g.near[((size_t)p * g.nrhs + c0 + cc) * g.N + p0 + row];
+                w.x += t.x;
+                w.y += t.y;
+            }
+            g.out[(size_t)(c0 + cc) * g.ld + g.perm[p0 + row]] = make_double2(fma(-g.facy, v.y, w.x), fma(g.facy, v.x, w.y));
+        }
+    }
+}
+
+// Parts of S: enough CTAs for about four waves of one per SM
+static int near64_split(const Ctx* c, int nrhs) {
+    const int ctas = c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C);
+    return std::max(1, std::min(OZ_MAX_SPLIT, (4 * c->nsm + ctas - 1) / ctas));
+}
+
+// Where the products run here: a CTA's tile is 64 rows of one box by 12 columns,
+// so boxes and blocks must fill it to some part.  Aggregation, receive and near
+// field in ms, FP64 FMAs against here, by bases per box x columns: 4 x 24: 1.95,
+// 4.48; 14 x 2: 0.39, 0.97; 14 x 8: 1.42, 1.19; 35 x 2: 0.43, 0.53; 35 x 8: 1.36,
+// 0.62; 61 x 24: 8.59, 2.29; 240 x 2: 0.62, 0.38.  One column stays with the
+// FMAs, whose order of sums single solves keep.
+bool split64_on(const Ctx* c, int nrhs) {
+    const long long nb = (long long)c->box_ptr.size() - 1;
+    return nrhs >= 2 && c->N >= 12 * nb && (long long)c->N * nrhs >= 112 * nb;
+}
+
+// The tile list and the patterns' exponents (once per context), and the
+// workspace, grown so that a smaller block never needs more (a caller may
+// capture it).
+int split64_ready(Ctx* c, int nrhs) {
+    const size_t nb = c->box_ptr.size() - 1, K2 = 2 * (size_t)c->lv[c->nlev].K;
+    if (!c->doz_tiles) {
+        std::vector<int2> t;
+        for (size_t b = 0; b < nb; ++b)
+            for (int r = 0; r < c->box_ptr[b + 1] - c->box_ptr[b]; r += OZ_R) t.push_back(make_int2((int)b, r));
+        CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->dev));
+        // limits of the kernels, the same for every context
+        CK(cudaFuncSetAttribute(k_split64<OZ_NEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+        CK(cudaFuncSetAttribute(k_split64<OZ_RECEIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+        CK(cudaFuncSetAttribute(k_split64<OZ_AGGREGATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+        if (!c->doz_pat) CK(cudaMalloc(&c->doz_pat, (c->N + nb * K2) * sizeof(int)));
+        k_pattern_exp<<<(c->N + 7) / 8, 256, 0, c->stream>>>(c->N, (int)K2, c->dR, c->doz_pat);
+        k_direction_exp<<<(unsigned)nb, 256, 0, c->stream>>>((int)K2, c->dbox_ptr, c->dR, c->doz_pat + c->N);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(c->stream));   // products may run on another stream
+        int2* d = nullptr;
+        CK(cudaMalloc(&d, t.size() * sizeof(int2)));
+        if (!cuda_ok(c, cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice), "tiles")) {
+            cudaFree(d);
+            return MLF_E_CUDA;
+        }
+        c->doz_tiles = d;
+        c->noz_tiles = (int)t.size();
+    }
+    size_t need = 0;
+    for (int n = 2; n <= nrhs; ++n) need = std::max(need, (size_t)near64_split(c, n) * n * c->N);
+    if (c->oz_cap < need) {
+        if (c->doz_ws) cudaFree(c->doz_ws);
+        if (c->doz_exp) cudaFree(c->doz_exp);
+        c->doz_ws = nullptr;
+        c->doz_exp = nullptr;
+        c->oz_cap = 0;
+        CK(cudaMalloc(&c->doz_ws, need * sizeof(double2)));
+        CK(cudaMalloc(&c->doz_exp, (2 * (size_t)c->N + nb * nrhs) * sizeof(int)));
+        c->oz_cap = need;
+    }
+    return MLF_OK;
+}
+
+static OzArgs oz_args(const Ctx* c, int nrhs, int ld) {
+    OzArgs g{};
+    g.N = c->N; g.nrhs = nrhs; g.ld = ld; g.K2 = 2 * c->lv[c->nlev].K;
+    g.tiles = c->doz_tiles;
+    g.box_ptr = c->dbox_ptr; g.perm = c->dperm; g.ia = c->dia; g.ja = c->dja;
+    g.Z = c->dZ; g.R = c->dR;
+    return g;
+}
+
+// C (leaf fields) = R^T x
+int split64_aggregate(Ctx* c, const double2* x, int nrhs, int ld, double2* C, cudaStream_t s) {
+    const int nb = (int)c->box_ptr.size() - 1;
+    OzArgs g = oz_args(c, nrhs, ld);
+    int* cexp = c->doz_exp + 2 * (size_t)c->N;
+    k_col_exp<OZ_AGGREGATE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, nullptr, cexp);
+    g.x = x; g.rexp = c->doz_pat + c->N; g.cexp = cexp; g.out = C;
+    k_split64<OZ_AGGREGATE><<<(unsigned)((size_t)nb * ((g.K2 + OZ_R - 1) / OZ_R) * ((nrhs + OZ_C - 1) / OZ_C)), OZ_THREADS,
+                              OZ_SMEM, s>>>(g);
+    return cuda_ok(c, cudaGetLastError(), "aggregation (split)") ? MLF_OK : MLF_E_CUDA;
+}
+
+// y = Z_near x + j facy conj(R) A
+int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy, int nrhs, int ld, double2* y,
+                         cudaStream_t s) {
+    const int nb = (int)c->box_ptr.size() - 1, ncb = (nrhs + OZ_C - 1) / OZ_C;
+    OzArgs g = oz_args(c, nrhs, ld);
+    int *sexp = c->doz_exp, *rexp = sexp + c->N, *cexp = rexp + c->N;
+    k_row_exp<<<(c->N + 255) / 256, 256, 0, s>>>(c->N, nrhs, ld, x, sexp);
+    k_near_exp<<<(c->N + 7) / 8, 256, 0, s>>>(c->N, c->dperm, c->dia, c->dja, c->dZ, sexp, rexp);
+    k_col_exp<OZ_NEAR><<<nb * nrhs, 256, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, sexp, cexp);
+    const int nsplit = near64_split(c, nrhs);
+    g.x = x; g.sexp = sexp; g.rexp = rexp; g.cexp = cexp; g.out = c->doz_ws;
+    k_split64<OZ_NEAR><<<dim3(ncb * c->noz_tiles, nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
+    k_col_exp<OZ_RECEIVE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, A, nullptr, cexp);
+    g.x = A; g.rexp = c->doz_pat; g.out = y; g.near = c->doz_ws; g.nsplit = nsplit; g.facy = facy;
+    k_split64<OZ_RECEIVE><<<ncb * c->noz_tiles, OZ_THREADS, OZ_SMEM, s>>>(g);
+    return cuda_ok(c, cudaGetLastError(), "near + receive (split)") ? MLF_OK : MLF_E_CUDA;
+}
+
+}  // namespace mlf
