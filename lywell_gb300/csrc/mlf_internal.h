@@ -170,7 +170,7 @@ struct Ctx {
     float2* dZ = nullptr;
     double2* dZd = nullptr;           // the same near values as complex(8)
     // FP64 products on blocks of columns (mlf_split64.cu): row tiles (box, first
-    // row), the patterns' exponents, the call's exponents (x's rows, Z's rows,
+    // row), exponents of the patterns (or of the dense matrix), the call's exponents (x's rows, Z's rows,
     // columns) and the near sums [split][column][box-sorted place]
     int2* doz_tiles = nullptr;
     int *doz_pat = nullptr, *doz_exp = nullptr;
@@ -257,6 +257,7 @@ int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, c
                        double2* const* Cf, double2* const* Bf, double2* const* Af, cudaEvent_t* ev);
 // FP64 near field, leaf aggregation and receive on blocks of columns (mlf_split64.cu)
 bool split64_on(const Ctx* c, int nrhs);
+int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s);
 int split64_ready(Ctx* c, int nrhs);
 int split64_aggregate(Ctx* c, const double2* x, int nrhs, int ld, double2* C, cudaStream_t s);
 int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy, int nrhs, int ld, double2* y,

@@ -1,7 +1,7 @@
 // Dense method-of-moments operator on the GPU (modMoM.f90:85-128 fill,
 // MatxVec_MoM modMoM.f90:273-277): the full N x N impedance matrix in FP64,
 // filled on the device by the same Z_mn element as the near field, and a
-// matvec that streams it once per group of four right-hand sides.  A
+// matvec that streams it once per group of twelve right-hand sides.  A
 // context made with MLF_FLAG_DENSE_MOM holds this operator instead of the
 // octree; CGS, excitation and RCS run on it unchanged.  At N = 30720 the
 // matrix is 15 GB, within HBM, so it also serves as the exact reference for
@@ -30,38 +30,32 @@ __global__ void k_mom_fill(int N, const double* __restrict__ t_baric, const doub
         Z[(size_t)m * N + n] = zmn_mom(m, n, t_baric, t_baric_sub, p_coord, e_t, e_po, e_long, w, w_smue, c72);
 }
 
-// y(m, c) = sum_n Z[m][n] x(n, c): one warp per row, four columns per pass
-__global__ void k_mom_gemv(int N, int nrhs, int ld, const double2* __restrict__ Z, const double2* __restrict__ x,
+// y(m) = sum_n Z[m][n] x(n) for column blockIdx.y: one warp per row, four entries
+// a lane in flight, summed in the order of n.  The FP64 pipe bounds it (0.33 ms of
+// DFMA at 6750 unknowns, one column): 0.34 ms; one entry in flight, behind a loop
+// over four columns, took 1.47 ms.
+__global__ void k_mom_gemv(int N, int ld, const double2* __restrict__ Z, const double2* __restrict__ x,
                            double2* __restrict__ y) {
+    x += (size_t)blockIdx.y * ld;
+    y += (size_t)blockIdx.y * ld;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (gw >= N) return;
     const int m = (int)gw;
     const double2* zr = Z + (size_t)m * N;
-    for (int c0 = 0; c0 < nrhs; c0 += 4) {
-        double ar[4] = {0, 0, 0, 0}, ai[4] = {0, 0, 0, 0};
-        for (int n = lane; n < N; n += 32) {
-            const double2 z = zr[n];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (c0 + u < nrhs) {
-                    const double2 v = x[(size_t)(c0 + u) * ld + n];
-                    ar[u] = fma(z.x, v.x, ar[u]); ar[u] = fma(-z.y, v.y, ar[u]);
-                    ai[u] = fma(z.x, v.y, ai[u]); ai[u] = fma(z.y, v.x, ai[u]);
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                ar[u] += __shfl_xor_sync(0xffffffff, ar[u], o);
-                ai[u] += __shfl_xor_sync(0xffffffff, ai[u], o);
-            }
-        }
-        if (lane == 0)
-            for (int u = 0; u < 4 && c0 + u < nrhs; ++u) y[(size_t)(c0 + u) * ld + m] = make_double2(ar[u], ai[u]);
+    double ar = 0, ai = 0;
+#pragma unroll 4
+    for (int n = lane; n < N; n += 32) {
+        const double2 z = zr[n], v = x[n];
+        ar = fma(z.x, v.x, ar); ar = fma(-z.y, v.y, ar);
+        ai = fma(z.x, v.y, ai); ai = fma(z.y, v.x, ai);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ar += __shfl_xor_sync(0xffffffff, ar, o);
+        ai += __shfl_xor_sync(0xffffffff, ai, o);
+    }
+    if (lane == 0) y[m] = make_double2(ar, ai);
 }
 
 int dense_setup(Ctx* c) {
@@ -86,8 +80,11 @@ int dense_setup(Ctx* c) {
 }
 
 int dense_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
+    // blocks of columns go to the digit splits, but for small matrices, where their
+    // six launches (about 30 us) cost more: 1080 unknowns x 2 is 36 us either way
+    if (nrhs > 1 && (double)c->N * c->N * nrhs > 2.5e6) return dense64_matvec(c, x, y, nrhs, ld, s);
     const long long threads = (long long)c->N * 32;
-    k_mom_gemv<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(c->N, nrhs, ld, c->dZdense, x, y);
+    k_mom_gemv<<<dim3((unsigned)((threads + 255) / 256), nrhs), 256, 0, s>>>(c->N, ld, c->dZdense, x, y);
     return cuda_ok(c, cudaGetLastError(), "dense matvec") ? MLF_OK : MLF_E_CUDA;
 }
 

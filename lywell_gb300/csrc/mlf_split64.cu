@@ -2,12 +2,14 @@
 // the tensor cores, by exact splitting into 8-bit digits (Ozaki, Ogita, Oishi
 // and Rump 2012; on FP16 matrix units Mukunoki et al. 2020).
 //
-// All three are a complex GEMM per leaf box (llenar_campoCyB,
+// The three are a complex GEMM per leaf box (llenar_campoCyB,
 // modMLFMA.f90:1805-1811; MatxVec_MLFMA, :1915-1942):
 //   near       y_m = sum_k Z_mk x_k     the box's bases over its near list S,
 //                                       which they share; Z complex(4)
 //   receive    y_m = sum_k conj(R_mk) A_k   its bases over the 2K directions
 //   aggregate  C_q = sum_k R_kq x_k     the directions over its bases
+// and the dense method-of-moments operator (MatxVec_MoM, modMoM.f90:273-277) is
+// one over all unknowns.
 // GB300 does 2 DFMA a clock and SM, which bounds them whatever the number of
 // columns; an FP16 product of two integers below 2^8 is exact, and so is its
 // FP32 sum.  Both operands become 62-bit integers relative to a power of two
@@ -58,7 +60,7 @@ constexpr int OZ_WARPS = 12;       // 4 tiles of 16 rows x 3 of 8 real columns
 constexpr int OZ_THREADS = 32 * OZ_WARPS;
 constexpr int OZ_WR = (OZ_R + OZ_WARPS - 1) / OZ_WARPS;   // rows that a warp converts
 static_assert(OZ_C == OZ_WARPS && 2 * OZ_C == 8 * (OZ_WARPS / 4), "a warp converts one column and multiplies one tile");
-constexpr int OZ_MAX_SPLIT = 4;
+constexpr int OZ_MAX_SPLIT = 4, OZ_MAX_DENSE_SPLIT = 8;
 
 // |v| < 2^e to an integer below 2^62, truncated: v = m 2^(e - 62)
 __device__ __forceinline__ long long oz_fix(unsigned long long m62, int t, uint32_t sign) {
@@ -114,7 +116,7 @@ __global__ void k_near_exp(int N, const int* __restrict__ perm, const int* __res
     if (lane == 0) rexp[pos] = e;
 }
 
-enum { OZ_NEAR = 0, OZ_RECEIVE = 1, OZ_AGGREGATE = 2 };
+enum { OZ_NEAR = 0, OZ_RECEIVE = 1, OZ_AGGREGATE = 2, OZ_DENSE = 3 };
 
 // cexp[box * nrhs + c] = exponent of column c of the box's right-hand operand:
 // x 2^-sexp over the near list, the field A over its 2K directions, or x over
@@ -198,12 +200,68 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int er, i
     return ldexp(fma((double)hi, 4294967296.0, (double)lo), er + ec - 68);
 }
 
+// Dense operator.  bexp[row * nblk + b] = exponent of the row over the 32 unknowns
+// of block b, once per context; a warp per row
+__global__ void k_dense_block_exp(int N, int nblk, const double2* __restrict__ Z, short* __restrict__ bexp) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= N) return;
+    for (int b = 0; b < nblk; ++b) {
+        const int k = 32 * b + lane;
+        const int e = __reduce_max_sync(0xffffffffu, k < N ? oz_exp(Z[(size_t)row * N + k]) : -1022);
+        if (lane == 0) bexp[(size_t)row * nblk + b] = (short)min(max(e, -2000), 2000);   // 2000: not finite
+    }
+}
+// bmax[b] = largest sexp of block b; cexp[c] = exponent of column c of x 2^-sexp
+__global__ void k_dense_col_exp(int N, int nrhs, int ld, int nblk, const double2* __restrict__ x,
+                                const int* __restrict__ sexp, int* __restrict__ bmax, int* __restrict__ cexp) {
+    const int lane = threadIdx.x & 31;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nblk; b += (gridDim.x * blockDim.x) >> 5) {
+        const int k = 32 * b + lane;
+        const int s = k < N ? sexp[k] : OZ_ZERO, e = __reduce_max_sync(0xffffffffu, s);
+        if (lane == 0) bmax[b] = e;
+        for (int c = 0; c < nrhs; ++c) {
+            const int v = __reduce_max_sync(0xffffffffu, k < N ? oz_exp(x[(size_t)c * ld + k]) - s : OZ_ZERO);
+            if (lane == 0) atomicMax(&cexp[c], v);
+        }
+    }
+}
+// rexp[row] = bound of the exponent of row of Z 2^sexp, by blocks
+__global__ void k_dense_row_exp(int N, int nblk, const short* __restrict__ bexp, const int* __restrict__ bmax,
+                                int* __restrict__ rexp) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= N) return;
+    int e = OZ_ZERO;
+    for (int b = lane; b < nblk; b += 32) {
+        const int v = bexp[(size_t)row * nblk + b];
+        e = max(e, v == 2000 ? OZ_BAD : v + bmax[b]);
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) rexp[row] = e;
+}
+__global__ void k_set_int(int n, int v, int* __restrict__ a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) a[i] = v;
+}
+// y = sum of the parts, in order
+__global__ void k_sum_parts(int N, int nrhs, int ld, int nsplit, const double2* __restrict__ ws,
+                            double2* __restrict__ y) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (i >= N) return;
+    double2 t = make_double2(0, 0);
+    for (int p = 0; p < nsplit; ++p) {
+        const double2 v = ws[((size_t)p * nrhs + c) * N + i];
+        t.x += v.x;
+        t.y += v.y;
+    }
+    y[(size_t)c * ld + i] = t;
+}
+
 struct OzArgs {
     int N, nrhs, ld, K2;                // K2 = 2K, the leaf's samples of both polarisations
     const int2* tiles;                  // (box, first row)
     const int *box_ptr, *perm, *ia, *ja;
     const float2* Z;
-    const double2 *R, *x;               // x: right-hand operand (receive: the field A)
+    const double2 *R, *x;               // R: patterns, or the dense matrix; x: right-hand operand (receive: the field A)
     const int *sexp, *rexp, *cexp;      // exponents of sources (near), rows and columns
     double2* out;                       // near: [split][col][box-sorted place]; receive: y; aggregate: the field C
     const double2* near;                // receive: the near field's parts
@@ -227,8 +285,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nqt = (g.K2 + OZ_R - 1) / OZ_R;
     const int ncb = (g.nrhs + OZ_C - 1) / OZ_C, tile = blockIdx.x / ncb;
-    const int2 tl = MODE == OZ_AGGREGATE ? make_int2(tile / nqt, tile % nqt * OZ_R) : g.tiles[tile];
-    const int b0 = g.box_ptr[tl.x], nb = g.box_ptr[tl.x + 1] - b0;
+    const int2 tl = MODE == OZ_DENSE ? make_int2(0, tile * OZ_R) : MODE == OZ_AGGREGATE ? make_int2(tile / nqt, tile % nqt * OZ_R) : g.tiles[tile];
+    const int b0 = MODE == OZ_DENSE ? 0 : g.box_ptr[tl.x], nb = MODE == OZ_DENSE ? g.N : g.box_ptr[tl.x + 1] - b0;
     const int p0 = b0 + tl.y;                                    // near, receive: rows p0 .. p0 + nr - 1
     const int nr = min(OZ_R, (MODE == OZ_AGGREGATE ? g.K2 : nb) - tl.y);
     const int c0 = blockIdx.x % ncb * OZ_C, nc = min(OZ_C, g.nrhs - c0);
@@ -248,15 +306,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
         const int row = min(warp + OZ_WARPS * r, nr - 1);
         if constexpr (MODE == OZ_NEAR) zrow[r] = g.Z + g.ia[g.perm[p0 + row]];
         else if constexpr (MODE == OZ_RECEIVE) zrow[r] = g.R + (size_t)(p0 + row) * g.K2;
+        else if constexpr (MODE == OZ_DENSE) zrow[r] = g.R + (size_t)(p0 + row) * g.N;
         else zrow[r] = g.R + (size_t)b0 * g.K2 + tl.y + row;
     }
     const int col = c0 + min(warp, nc - 1);
     const double2* xc = MODE == OZ_RECEIVE ? g.x + ((size_t)tl.x * g.nrhs + col) * g.K2 : g.x + (size_t)col * g.ld;
     auto source = [&](int k) {   // of the right-hand operand; k includes the lane
         if (k >= k1) return -1;
-        return MODE == OZ_NEAR ? g.ja[s0 + k] : MODE == OZ_RECEIVE ? k : g.perm[b0 + k];
+        return MODE == OZ_NEAR ? g.ja[s0 + k] : MODE == OZ_AGGREGATE ? g.perm[b0 + k] : k;
     };
-    auto shift = [&](int j) { return MODE == OZ_NEAR && j >= 0 ? g.sexp[j] : 0; };
+    auto shift = [&](int j) { return (MODE == OZ_NEAR || MODE == OZ_DENSE) && j >= 0 ? g.sexp[j] : 0; };
     ZT z[OZ_WR];
     double2 xv;
     auto load = [&](int k, int j) {
@@ -362,7 +421,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
         const int e = er[row], f = ec[cc];
         double2 v = make_double2(oz_value(hi[2 * h], lo[2 * h], e, f), oz_value(hi[2 * h + 1], lo[2 * h + 1], e, f));
         if (e > OZ_BAD / 2 || f > OZ_BAD / 2) v = make_double2(nan, nan);
-        if (MODE == OZ_NEAR) {
+        if (MODE == OZ_NEAR || MODE == OZ_DENSE) {
             g.out[((size_t)blockIdx.y * g.nrhs + c0 + cc) * g.N + p0 + row] = v;
         } else if (MODE == OZ_AGGREGATE) {
             g.out[((size_t)tl.x * g.nrhs + c0 + cc) * g.K2 + tl.y + row] = v;
@@ -378,10 +437,26 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
     }
 }
 
-// Parts of S: enough CTAs for about four waves of one per SM
+// Parts of the terms: enough CTAs for about four waves of one per SM
 static int near64_split(const Ctx* c, int nrhs) {
     const int ctas = c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C);
-    return std::max(1, std::min(OZ_MAX_SPLIT, (4 * c->nsm + ctas - 1) / ctas));
+    return std::max(1, std::min(c->dense ? OZ_MAX_DENSE_SPLIT : OZ_MAX_SPLIT, (4 * c->nsm + ctas - 1) / ctas));
+}
+
+// workspace for blocks of up to nrhs columns, with `ints` exponents beside it
+static int oz_workspace(Ctx* c, int nrhs, size_t ints) {
+    size_t need = 0;
+    for (int n = 2; n <= nrhs; ++n) need = std::max(need, (size_t)near64_split(c, n) * n * c->N);
+    if (c->oz_cap >= need) return MLF_OK;
+    if (c->doz_ws) cudaFree(c->doz_ws);
+    if (c->doz_exp) cudaFree(c->doz_exp);
+    c->doz_ws = nullptr;
+    c->doz_exp = nullptr;
+    c->oz_cap = 0;
+    CK(cudaMalloc(&c->doz_ws, need * sizeof(double2)));
+    CK(cudaMalloc(&c->doz_exp, ints * sizeof(int)));
+    c->oz_cap = need;
+    return MLF_OK;
 }
 
 // Where the products run here: a CTA's tile is 64 rows of one box by 12 columns,
@@ -423,19 +498,7 @@ int split64_ready(Ctx* c, int nrhs) {
         c->doz_tiles = d;
         c->noz_tiles = (int)t.size();
     }
-    size_t need = 0;
-    for (int n = 2; n <= nrhs; ++n) need = std::max(need, (size_t)near64_split(c, n) * n * c->N);
-    if (c->oz_cap < need) {
-        if (c->doz_ws) cudaFree(c->doz_ws);
-        if (c->doz_exp) cudaFree(c->doz_exp);
-        c->doz_ws = nullptr;
-        c->doz_exp = nullptr;
-        c->oz_cap = 0;
-        CK(cudaMalloc(&c->doz_ws, need * sizeof(double2)));
-        CK(cudaMalloc(&c->doz_exp, (2 * (size_t)c->N + nb * nrhs) * sizeof(int)));
-        c->oz_cap = need;
-    }
-    return MLF_OK;
+    return oz_workspace(c, nrhs, 2 * (size_t)c->N + nb * nrhs);
 }
 
 static OzArgs oz_args(const Ctx* c, int nrhs, int ld) {
@@ -475,6 +538,48 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
     g.x = A; g.rexp = c->doz_pat; g.out = y; g.near = c->doz_ws; g.nsplit = nsplit; g.facy = facy;
     k_split64<OZ_RECEIVE><<<ncb * c->noz_tiles, OZ_THREADS, OZ_SMEM, s>>>(g);
     return cuda_ok(c, cudaGetLastError(), "near + receive (split)") ? MLF_OK : MLF_E_CUDA;
+}
+
+// Dense operator: y = Z x for blocks of columns.  The row exponents are bounds by
+// blocks of 32 unknowns, so that a product reads the matrix once.  FP64 FMAs, four
+// columns a pass, against here: 6750 unknowns x 3: 1399, 467 us; x 24: 7678, 1297;
+// 3000 x 2: 339, 120; 1920 x 4: 131, 59; 1080 x 6: 86, 39.
+static int dense64_ready(Ctx* c, int nrhs) {
+    const int N = c->N, nblk = (N + 31) / 32;
+    if (!c->doz_pat) {
+        CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->dev));
+        CK(cudaFuncSetAttribute(k_split64<OZ_DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+        c->noz_tiles = (N + OZ_R - 1) / OZ_R;
+        int* p = nullptr;
+        CK(cudaMalloc(&p, (size_t)N * nblk * sizeof(short)));
+        k_dense_block_exp<<<(N + 7) / 8, 256, 0, c->stream>>>(N, nblk, c->dZdense, reinterpret_cast<short*>(p));
+        if (!cuda_ok(c, cudaGetLastError(), "k_dense_block_exp") ||
+            !cuda_ok(c, cudaStreamSynchronize(c->stream), "k_dense_block_exp")) {   // products may run on another stream
+            cudaFree(p);
+            return MLF_E_CUDA;
+        }
+        c->doz_pat = p;
+    }
+    return oz_workspace(c, nrhs, 2 * (size_t)N + nblk + nrhs);
+}
+
+int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
+    int st;
+    if ((st = dense64_ready(c, nrhs))) return st;
+    const int N = c->N, nblk = (N + 31) / 32, nsplit = near64_split(c, nrhs);
+    int *sexp = c->doz_exp, *rexp = sexp + N, *bmax = rexp + N, *cexp = bmax + nblk;
+    k_row_exp<<<(N + 255) / 256, 256, 0, s>>>(N, nrhs, ld, x, sexp);
+    k_set_int<<<(nrhs + 255) / 256, 256, 0, s>>>(nrhs, OZ_ZERO, cexp);
+    k_dense_col_exp<<<std::min((nblk + 7) / 8, 256), 256, 0, s>>>(N, nrhs, ld, nblk, x, sexp, bmax, cexp);
+    k_dense_row_exp<<<(N + 7) / 8, 256, 0, s>>>(N, nblk, reinterpret_cast<const short*>(c->doz_pat), bmax, rexp);
+    OzArgs g{};
+    g.N = N; g.nrhs = nrhs; g.ld = ld; g.K2 = 1;
+    g.R = c->dZdense; g.x = x;
+    g.sexp = sexp; g.rexp = rexp; g.cexp = cexp;
+    g.out = c->doz_ws;
+    k_split64<OZ_DENSE><<<dim3((unsigned)c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C), nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
+    k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, y);
+    return cuda_ok(c, cudaGetLastError(), "dense matvec (split)") ? MLF_OK : MLF_E_CUDA;
 }
 
 }  // namespace mlf

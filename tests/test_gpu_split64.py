@@ -74,3 +74,18 @@ def test_not_finite_stays_in_its_column(spheroid, bad):
     assert not np.isfinite(Z[:, 2]).all()
     for c in (0, 1, 3):
         assert _off(Z[:, c], Y[:, c]) < 1e-14
+
+
+@pytest.mark.parametrize("level,nrhs", [(0, 2), (1, 3), (2, 13), (2, 2), (3, 2), (3, 25)])
+def test_dense_blocks(level, nrhs, gpu_lib):
+    """The dense operator: fewer rows than a tile, ragged last blocks of 32 unknowns."""
+    from lywell_gb300 import RWG, MoM, meshes
+    with MoM(RWG(meshes.icosphere(level, 0.6))) as m:
+        X = _columns(m, nrhs, level)
+        if nrhs == 13:
+            X[:, 3] *= 1e100
+            X[:, 4] = 0
+        Y = m.matvec(X)
+        for c in range(nrhs):
+            ref = m.matvec(X[:, c])
+            assert np.linalg.norm(Y[:, c] - ref) <= 1e-12 * np.linalg.norm(ref)
