@@ -312,10 +312,11 @@ int mlf_nearinv(mlf_ctx* ctx, int* bad_box);
 int mlf_set_nearinv_precision(mlf_ctx* ctx, int bits);
 
 /* The FP32 LU gives each box one CTA, so the largest neighbourhoods would set
- * the set-up time alone.  Boxes of at least min_unknowns unknowns whose work
- * (n^3) exceeds three times the remaining boxes' share per CTA are factorised on many CTAs
- * each instead (panel on one CTA; row swaps, U12 and the trailing update over
- * the GPU), on side streams next to the one-CTA-per-box kernel.
+ * the set-up time alone.  Boxes of at least min_unknowns unknowns that hold
+ * 1600 unknowns or more, or whose work (n^3) exceeds the remaining boxes' share
+ * per CTA, are factorised on many CTAs each instead (panel on one CTA; U12 and
+ * the trailing update over the GPU), in groups of boxes in step, on side streams
+ * next to the one-CTA-per-box kernel; the results are the same.
  * min_unknowns = 0 turns this off; the default is 1024.  mlf_get_lu_split
  * reads the setting and how many boxes took the many-CTA path in the last
  * build.  No counterpart in the reference. */
