@@ -678,11 +678,13 @@ __global__ void k_mdot(int N, int nrhs, const double2* __restrict__ V, size_t vs
     if (threadIdx.x == 0) partial[((size_t)i * nrhs + col) * gridDim.x + blockIdx.x] = make_double2(rs[0], is[0]);
 }
 
-// out[k] = sum_b partial[k*GM_BLOCKS + b], fixed order
+// out[k] = sum_b partial[k*GM_BLOCKS + b], fixed order; a thread's loads are the
+// time (19 us one after the other), so 16 are in flight
 __global__ void k_reduce_partials(int nk, const double2* __restrict__ partial, double2* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nk) return;
     double2 s = make_double2(0, 0);
+#pragma unroll 16
     for (int b = 0; b < GM_BLOCKS; ++b) {
         s.x += partial[(size_t)k * GM_BLOCKS + b].x;
         s.y += partial[(size_t)k * GM_BLOCKS + b].y;
@@ -800,6 +802,7 @@ __global__ void k_reduce_partials_n(int nk, int nb, const double2* __restrict__ 
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nk) return;
     double2 s = make_double2(0, 0);
+#pragma unroll 16
     for (int b = 0; b < nb; ++b) {
         s.x += partial[(size_t)k * nb + b].x;
         s.y += partial[(size_t)k * nb + b].y;

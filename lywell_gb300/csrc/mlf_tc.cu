@@ -36,7 +36,8 @@
 // 1024 bytes).
 //
 // A persistent CTA (8 warps) per SM walks work items (tile of at most 160
-// rows, 64 columns).  Thread 0 issues the TMA loads of a 3-stage ring; thread
+// rows, 64 columns; a part of the near list where tiles are few, the parts' sums
+// added by k_tc_sum).  Thread 0 issues the TMA loads of a 3- or 4-stage ring; thread
 // 32 issues the MMAs: per chunk of 32 real K, 4 K-steps x 3 products (A_lo
 // B_hi, A_hi B_lo, A_hi B_hi) into a 128 x N FP32 accumulator in TMEM, and
 // tcgen05.commit frees a stage once its MMAs are done.  Warps 4-7 read their
@@ -66,16 +67,21 @@ namespace mlf {
         if (!cuda_ok(c, (call), #call)) return MLF_E_CUDA;   \
     } while (0)
 
-constexpr int TC_STAGES = 3;
 constexpr int TC_ROWS = 160;                 // bases of box i per tile (MMA N <= 160 here)
 constexpr int TC_KCH = 16;                   // complex contraction values per 128-byte TF32 row (receive)
 constexpr int TC_KCH_H = 32;                 // complex contraction values per 128-byte FP16 row (near, aggregation)
 constexpr int TC_COLS = 64;                  // right-hand sides per column tile (MMA M = 128)
 constexpr int TC_ZBOX = 32;                  // rows per TMA box of the Z operand
 constexpr int TC_ABYTES = 128 * 128;         // one A tile: 128 rows x 128 bytes
-constexpr int TC_BBYTES = TC_ROWS * 128;     // one B tile at most
-constexpr int TC_STAGE_BYTES = 2 * TC_ABYTES + 2 * TC_BBYTES;
-constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE_BYTES + 1024;   // + alignment of the ring
+// The ring: three stages of 72 KB for tiles of up to 160 rows, or four of 56 KB
+// where no tile has more than 96 (bytes in flight bound the kernel).
+template <int ST> struct TcRing {
+    static constexpr int ROWS = ST == 4 ? 96 : TC_ROWS;
+    static constexpr int BBYTES = ROWS * 128;               // one B tile at most
+    static constexpr int STAGE = 2 * TC_ABYTES + 2 * BBYTES;
+    static constexpr size_t SMEM = (size_t)ST * STAGE + 1024;   // + alignment of the ring
+};
+constexpr int TC_MAX_SPLIT = 8;              // parts of a tile's near list at most
 constexpr uint32_t TC_TMEM_COLS = 256;
 constexpr uint32_t TC_SPIN = 1u << 20;       // mbarrier polls before a wait gives up
 
@@ -95,6 +101,15 @@ struct TcState {
     int nsm = 0;                    // SMs: CTAs of the persistent GEMM
     int4* dtiles = nullptr;         // (box, first row, rows, -), by decreasing work
     int* dtchunks = nullptr;        // per tile: chunks over its near boxes
+    int maxrows = 0;                // rows of the largest tile
+    // near field and preconditioner: the tiles again, in nsplit parts of their near
+    // lists where tiles are few: (box, first row, rows, part), chunks and first
+    // block entry of each part
+    int nsplit = 1, nstiles = 0;
+    int4* dstiles = nullptr;
+    int *dstchunks = nullptr, *dsfirst = nullptr;
+    float2* dws = nullptr;          // their sums [part][box-sorted basis][column]
+    size_t ws_cap = 0;
     int* dzrow = nullptr;           // per block entry e: first Z-operand row (chunk 0)
     int* dcbase = nullptr;          // per box: its first chunk
     int2* dchunk = nullptr;         // per chunk: (first box-sorted position, bases in it)
@@ -111,7 +126,7 @@ struct TcState {
     // leaf aggregation and receive (built from the FP32 patterns R on first use)
     const float2* Rsrc = nullptr;   // the patterns the operands below hold
     int K2 = 0;                     // 2K directions of the leaf level
-    int natiles = 0;
+    int natiles = 0, arows = 0;     // tiles of the aggregation, rows of the largest
     int4* datiles = nullptr;        // aggregation tiles (box, first direction, directions, -)
     int* datchunks = nullptr;       // per aggregation tile: chunks of the box's bases
     int* dabase = nullptr;          // per box: first row of the aggregation operand
@@ -195,15 +210,18 @@ __global__ void k_tc_fill_zh(const int* __restrict__ entry_box, const int* __res
 }
 
 // cmax[col] = max over column col of xs (box-sorted rows, row-major N x nrhs)
-// of |re|, |im|; grid (N / 256, nrhs / 64), 64 columns x 4 row groups per CTA
+// of |re|, |im|; grid (N / 64, nrhs / 64), 64 columns x 4 row groups per CTA.
+// A thread's rows are a chain of loads: 16 of them, eight in flight, where 64 on
+// a quarter of the CTAs took 10.2 us for 15360 x 32.
 __global__ void __launch_bounds__(256) k_tc_colmax(int N, int nrhs, const float2* __restrict__ xs,
                                                    unsigned* __restrict__ cmax) {
     __shared__ float red[4][TC_COLS];
     const int tx = threadIdx.x & (TC_COLS - 1), ty = threadIdx.x / TC_COLS;
     const int col = blockIdx.y * TC_COLS + tx;
-    const int r0 = blockIdx.x * 256 + ty * 64, r1 = min(r0 + 64, N);
+    const int r0 = blockIdx.x * 64 + ty * 16, r1 = min(r0 + 16, N);
     float m = 0.f;
     if (col < nrhs)
+#pragma unroll 8
         for (int r = r0; r < r1; ++r) {
             const float2 v = xs[(size_t)r * nrhs + col];
             m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
@@ -336,6 +354,7 @@ struct TcArgs {
     const int* nbox_list;
     const int* zrow;     // near: per block entry; aggregation, receive: per box -- first B row
     const int* cbase;    // per box: its first chunk of the X operand
+    const int* first;    // near: per tile, first block entry of its part
     int nchunk, nrhs, ld, K2;
     float facy;
     const float* rinv;   // FP16 modes: per output row (near: box-sorted basis; aggregation: box x 2K), 1 / scale
@@ -344,6 +363,8 @@ struct TcArgs {
     double2* y;
     float2* out32;
     float2* C;
+    float2* ws;          // near: the parts' sums, to be added by k_tc_sum (null: one part, written at once)
+    int N;
     int* err;
 };
 
@@ -362,15 +383,16 @@ struct TcFmt {
     static constexpr int KCH = H ? TC_KCH_H : TC_KCH;
 };
 
-template <int MODE>
+template <int MODE, int ST>
 __global__ void __launch_bounds__(256, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mbhi, const __grid_constant__ CUtensorMap mblo,
               const __grid_constant__ CUtensorMap mxhi, const __grid_constant__ CUtensorMap mxlo, const TcArgs a) {
     constexpr bool NEAR = MODE == TCM_NEAR_ADD || MODE == TCM_NEAR_SET;
     constexpr bool RAW = MODE == TCM_RECV;
+    constexpr int STAGE = TcRing<ST>::STAGE, BBYTES = TcRing<ST>::BBYTES;
     constexpr uint32_t RAW_BYTES = TC_COLS * 128;   // 64 field rows of 16 complex values
     extern __shared__ unsigned char tc_raw[];
-    __shared__ __align__(8) uint64_t full[TC_STAGES], empty[TC_STAGES], conv[TC_STAGES], accf[2], acce[2], done;
+    __shared__ __align__(8) uint64_t full[ST], empty[ST], conv[ST], accf[2], acce[2], done;
     __shared__ uint32_t tmem_base;
     __shared__ int fail_s, cvok_s, issued_s, consumed_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -379,7 +401,7 @@ __global__ void __launch_bounds__(256, 1)
     const int nitems = a.ntiles * a.nct;
     volatile int* vfail = &fail_s;
     if (tid == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) {
+        for (int s = 0; s < ST; ++s) {
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
             tc::mbar_init(&conv[s], 64);
@@ -425,14 +447,14 @@ __global__ void __launch_bounds__(256, 1)
                 const int nch = tc_item_chunks<MODE>(a, tile);
                 const int nB = (nrow + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX;          // B rows staged
                 const uint32_t bytes = (RAW ? RAW_BYTES : 2u * TC_ABYTES) + 2u * (uint32_t)nB * 128u;
-                int le = NEAR ? a.nbox_ptr[i] : 0, lkc = 0;
+                int le = NEAR ? a.first[tile] : 0, lkc = 0;
                 for (int cI = 0; cI < nch; ++cI, ++g) {
-                    const int s = g % TC_STAGES;
-                    if ((g >= TC_STAGES && !tc::mbar_wait(&empty[s], ((g / TC_STAGES) - 1) & 1, TC_SPIN)) || *vfail) {
+                    const int s = g % ST;
+                    if ((g >= ST && !tc::mbar_wait(&empty[s], ((g / ST) - 1) & 1, TC_SPIN)) || *vfail) {
                         ok = false;   // the consumers then give up on this stage's full barrier too
                         break;
                     }
-                    unsigned char* st = ring + (size_t)s * TC_STAGE_BYTES;
+                    unsigned char* st = ring + (size_t)s * STAGE;
                     tc::mbar_arrive_expect_tx(&full[s], bytes);
                     int zr;
                     if (NEAR) {
@@ -460,7 +482,7 @@ __global__ void __launch_bounds__(256, 1)
                         // the aggregation's and receive's pattern operands are read by the
                         // tiles of one box (and the column tiles) only: streamed too
                         tc::tma_load_2d_hint(st + 2 * TC_ABYTES + qq * 128, &mbhi, 0, zr + qq, &full[s], pol_b);
-                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + TC_BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s],
+                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s],
                                              pol_b);
                     }
                 }
@@ -486,15 +508,15 @@ __global__ void __launch_bounds__(256, 1)
                 const uint32_t d = tmem + buf * TC_TMEM_COLS;
                 const uint32_t idesc = tc::instr_desc_f32acc(TcFmt<MODE>::FMT, 128, (a.tiles[tile].z + 15) / 16 * 16);
                 for (int cI = 0; cI < nch; ++cI, ++g) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t par = (g / TC_STAGES) & 1;
+                    const int s = g % ST;
+                    const uint32_t par = (g / ST) & 1;
                     if (!tc::mbar_wait(&full[s], par, TC_SPIN) || (RAW && !tc::mbar_wait(&conv[s], par, TC_SPIN))) {
                         ok = false;
                         break;
                     }
                     tc::tc_fence_after_sync();
-                    const uint32_t st = tc::smem_u32(ring + (size_t)s * TC_STAGE_BYTES);
-                    const uint32_t ahi = st, alo = st + TC_ABYTES, bhi = st + 2 * TC_ABYTES, blo = bhi + TC_BBYTES;
+                    const uint32_t st = tc::smem_u32(ring + (size_t)s * STAGE);
+                    const uint32_t ahi = st, alo = st + TC_ABYTES, bhi = st + 2 * TC_ABYTES, blo = bhi + BBYTES;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {   // K steps of 32 bytes of the 128-byte rows
                         const uint32_t ko = 32u * k;
@@ -532,8 +554,8 @@ __global__ void __launch_bounds__(256, 1)
             for (int q = blockIdx.x; q < nitems && go; q += gridDim.x) {
                 const int nch = tc_item_chunks<MODE>(a, q / a.nct);
                 for (int cI = 0; cI < nch; ++cI, ++g) {
-                    const int s = g % TC_STAGES;
-                    const uint32_t par = (g / TC_STAGES) & 1;
+                    const int s = g % ST;
+                    const uint32_t par = (g / ST) & 1;
                     if (cl == 0) cvok_s = (!*vfail && tc::mbar_wait(&full[s], par, TC_SPIN)) ? 1 : 0;
                     tc::named_bar_sync(1, 64);
                     if (!cvok_s) {   // the same decision in all 64 threads
@@ -541,7 +563,7 @@ __global__ void __launch_bounds__(256, 1)
                         break;
                     }
                     tc::mbar_wait(&full[s], par, TC_SPIN);   // complete already: acquires the landed bytes
-                    unsigned char* st = ring + (size_t)s * TC_STAGE_BYTES;
+                    unsigned char* st = ring + (size_t)s * STAGE;
                     // the raw rows arrive 128-byte swizzled: chunk k of row cl sits at
                     // k ^ (cl & 7), so the 8 lanes of a shared-memory wavefront read 8
                     // different bank groups
@@ -594,6 +616,10 @@ __global__ void __launch_bounds__(256, 1)
                 // a box without bases radiates nothing
                 if (MODE == TCM_AGG && writer)
                     for (int p = 0; p < nrow; ++p) a.C[((size_t)i * a.nrhs + col) * a.K2 + r0 + p] = make_float2(0.f, 0.f);
+                // nor does a part that got no box add anything
+                if (NEAR && a.ws && writer)
+                    for (int p = 0; p < nrow; ++p)
+                        a.ws[((size_t)tl.w * a.N + i0 + r0 + p) * a.nrhs + col] = make_float2(0.f, 0.f);
                 continue;
             }
             const uint32_t buf = na & 1;
@@ -613,8 +639,12 @@ __global__ void __launch_bounds__(256, 1)
                     const float im = __shfl_xor_sync(0xffffffffu, v[u], 1);
                     const int p = n0 + u;
                     if (writer && p < nrow) {
-                        if (MODE == TCM_NEAR_ADD) {
+                        if (NEAR && a.ws) {
                             const float rs = a.rinv[i0 + r0 + p];   // powers of two: exact
+                            a.ws[((size_t)tl.w * a.N + i0 + r0 + p) * a.nrhs + col] =
+                                make_float2(v[u] * rs * cs, im * rs * cs);
+                        } else if (MODE == TCM_NEAR_ADD) {
+                            const float rs = a.rinv[i0 + r0 + p];
                             double2* yp = a.y + (size_t)col * a.ld + a.perm[i0 + r0 + p];
                             const double2 o = *yp;
                             *yp = make_double2(o.x + (double)(v[u] * rs * cs), o.y + (double)(im * rs * cs));
@@ -643,12 +673,45 @@ __global__ void __launch_bounds__(256, 1)
         // loads already issued land before the shared memory is given up: at most
         // STAGES chunks beyond the last one the MMA thread consumed
         const uint32_t c0 = (uint32_t)consumed_s, c1 = (uint32_t)issued_s;
-        for (uint32_t g = c0; g < c1 && g < c0 + TC_STAGES; ++g)
-            tc::mbar_wait(&full[g % TC_STAGES], (g / TC_STAGES) & 1, TC_SPIN);
+        for (uint32_t g = c0; g < c1 && g < c0 + ST; ++g)
+            tc::mbar_wait(&full[g % ST], (g / ST) & 1, TC_SPIN);
     }
     tc::tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 2 * TC_TMEM_COLS);
+}
+
+// y += (ADD, FP64) or out32 = the sum of the parts ws[part][pos][col], in order, to
+// row perm[pos]; tiles of 32 bases x 32 columns turned in shared memory
+template <bool ADD>
+__global__ void __launch_bounds__(256) k_tc_sum(int N, int nrhs, int ld, int nsplit, const int* __restrict__ perm,
+                                                const float2* __restrict__ ws, double2* __restrict__ y,
+                                                float2* __restrict__ out32) {
+    __shared__ float2 t[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    for (int r = ty; r < 32; r += 8) {
+        float2 v = make_float2(0.f, 0.f);
+        if (p0 + r < N && c0 + tx < nrhs)
+            for (int q = 0; q < nsplit; ++q) {
+                const float2 w = ws[((size_t)q * N + p0 + r) * nrhs + c0 + tx];
+                v.x += w.x;
+                v.y += w.y;
+            }
+        t[r][tx] = v;
+    }
+    __syncthreads();
+    if (p0 + tx >= N) return;
+    const int n = perm[p0 + tx];
+    for (int c = ty; c < 32 && c0 + c < nrhs; c += 8) {
+        const float2 v = t[tx][c];
+        const size_t o = (size_t)(c0 + c) * ld + n;
+        if (ADD) {
+            const double2 w = y[o];
+            y[o] = make_double2(w.x + (double)v.x, w.y + (double)v.y);
+        } else {
+            out32[o] = v;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -726,7 +789,7 @@ void tc_free(Ctx* c) {
     F(t->Z.hi); F(t->Z.lo); F(t->Z.rinv); F(t->M.hi); F(t->M.lo); F(t->M.rinv); F(t->xhi); F(t->xlo);
     F(t->dcmax); F(t->dcinv); F(t->drowmax); F(t->RA.rinv);
     F(t->datiles); F(t->dabase); F(t->drbase); F(t->RA.hi); F(t->RA.lo); F(t->RR.hi); F(t->RR.lo);
-    F(t->dtchunks); F(t->datchunks);
+    F(t->dtchunks); F(t->datchunks); F(t->dstiles); F(t->dstchunks); F(t->dsfirst); F(t->dws);
     delete t;
     c->tc = nullptr;
 }
@@ -837,6 +900,56 @@ static int tc_setup_build(Ctx* c) {
     t->nsm = std::max(nsm, 1);
     c->tc = t;
     t->ntiles = (int)tiles.size();
+    for (const int4& q : tiles) t->maxrows = std::max(t->maxrows, q.z);
+    // parts of the near lists, whole near boxes each and about equal in chunks, so
+    // that the items of one column tile come to about four and a half per SM (184
+    // tiles of the 30720-RWG spheroid's boxes left most of the second round idle, 46
+    // tiles of the 7680-RWG one most of the SMs).  The 30720-RWG product with 64
+    // columns: 708 -> 636 us; a solve of 17280 unknowns x 32 columns: 104 -> 90 ms.
+    // The shorter FP32 accumulations are more accurate too: 1.5e-5 -> 2.3e-6 from
+    // FP64 at 7680.  Past eight parts their sums cost what they gain
+    t->nsplit = tiles.empty() ? 1 : std::max(1, std::min(TC_MAX_SPLIT, (9 * t->nsm / 2) / (int)tiles.size()));
+    std::vector<int4> stiles;
+    std::vector<int> stch, sfirst;
+    for (const int4& q : tiles) {
+        const int e1 = c->nbox_ptr[q.x + 1];
+        int e = c->nbox_ptr[q.x], total = 0;
+        for (int k = e; k < e1; ++k) total += cbase[c->nbox_list[k] + 1] - cbase[c->nbox_list[k]];
+        for (int part = 0, done = 0; part < t->nsplit; ++part) {   // every part, so that its sums are written
+            const int goal = (int)((long long)total * (part + 1) / t->nsplit);
+            stiles.push_back(make_int4(q.x, q.y, q.z, part));
+            sfirst.push_back(e);
+            int ch = 0;
+            while (e < e1 && (part + 1 == t->nsplit || done + ch < goal)) {
+                ch += cbase[c->nbox_list[e] + 1] - cbase[c->nbox_list[e]];
+                ++e;
+            }
+            done += ch;
+            stch.push_back(ch);
+        }
+    }
+    {
+        std::vector<int> idx(stiles.size());
+        for (size_t k = 0; k < idx.size(); ++k) idx[k] = (int)k;
+        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return stch[x] > stch[y]; });
+        std::vector<int4> t2;
+        std::vector<int> n2, f2;
+        for (int k : idx) {
+            t2.push_back(stiles[k]);
+            n2.push_back(stch[k]);
+            f2.push_back(sfirst[k]);
+        }
+        stiles.swap(t2);
+        stch.swap(n2);
+        sfirst.swap(f2);
+    }
+    t->nstiles = (int)stiles.size();
+    CK(cudaMalloc(&t->dstiles, std::max<size_t>(stiles.size(), 1) * sizeof(int4)));
+    CK(cudaMalloc(&t->dstchunks, std::max<size_t>(stch.size(), 1) * sizeof(int)));
+    CK(cudaMalloc(&t->dsfirst, std::max<size_t>(sfirst.size(), 1) * sizeof(int)));
+    CK(cudaMemcpy(t->dstiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(t->dstchunks, stch.data(), stch.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(t->dsfirst, sfirst.data(), sfirst.size() * sizeof(int), cudaMemcpyHostToDevice));
     t->nchunk = (int)chunk.size();
     t->zrows = rows;
     CK(cudaMalloc(&t->dtiles, std::max<size_t>(tiles.size(), 1) * sizeof(int4)));
@@ -853,10 +966,14 @@ static int tc_setup_build(Ctx* c) {
     CK(cudaMemcpy(t->dchunk, chunk.data(), chunk.size() * sizeof(int2), cudaMemcpyHostToDevice));
     CK(cudaMemset(t->derr, 0, sizeof(int)));
     if ((st = tc_near_operand(c, c->dZblk, &t->Z, c->stream))) return st;
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_SET>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_ADD, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_SET, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_ADD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_SET, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
     CK(cudaStreamSynchronize(c->stream));
     return MLF_OK;
 }
@@ -866,6 +983,15 @@ static int tc_x_buffers(Ctx* c, int nrhs) {
     TcState* t = c->tc;
     const int nct = (nrhs + TC_COLS - 1) / TC_COLS;
     const long long rows = (long long)nct * t->nchunk * 128;
+    // whole column tiles, as the operand: a block that fits the one fits the other
+    const size_t parts = t->nsplit > 1 ? (size_t)t->nsplit * c->N * nct * TC_COLS : 0;
+    if (parts > t->ws_cap) {
+        if (t->dws) cudaFree(t->dws);
+        t->dws = nullptr;
+        t->ws_cap = 0;
+        CK(cudaMalloc(&t->dws, parts * sizeof(float2)));
+        t->ws_cap = parts;
+    }
     if (rows <= t->xrows_cap && nct * TC_COLS <= t->cols_cap) return MLF_OK;
     auto F = [](void* p) { if (p) cudaFree(p); };
     F(t->xhi); F(t->xlo); F(t->dcmax); F(t->dcinv);
@@ -891,7 +1017,7 @@ static int tc_pack_x(Ctx* c, const float2* xs, int nrhs, cudaStream_t s) {
     TcState* t = c->tc;
     const int nct = (nrhs + TC_COLS - 1) / TC_COLS;
     CK(cudaMemsetAsync(t->dcmax, 0, (size_t)nrhs * sizeof(unsigned), s));
-    k_tc_colmax<<<dim3((c->N + 255) / 256, nct), 256, 0, s>>>(c->N, nrhs, xs, t->dcmax);
+    k_tc_colmax<<<dim3((c->N + 63) / 64, nct), 256, 0, s>>>(c->N, nrhs, xs, t->dcmax);
     k_tc_pack_xh<<<dim3(t->nchunk, nct), 256, 0, s>>>(t->nchunk, nrhs, t->dchunk, xs, t->dcmax,
                                                       static_cast<__half2*>(t->xhi), static_cast<__half2*>(t->xlo),
                                                       t->dcinv);
@@ -915,13 +1041,33 @@ static TcArgs tc_args(const Ctx* c, int nrhs) {
     a.nrhs = nrhs;
     a.perm = c->dperm;
     a.cinv = t->dcinv;
+    a.N = c->N;
     a.err = t->derr;
     return a;
+}
+
+// the near field's or preconditioner's items: the tiles in parts
+static void tc_near_args(const Ctx* c, TcArgs& a) {
+    const TcState* t = c->tc;
+    a.tiles = t->dstiles;
+    a.tchunks = t->dstchunks;
+    a.first = t->dsfirst;
+    a.ntiles = t->nstiles;
+    a.ws = t->nsplit > 1 ? t->dws : nullptr;
 }
 
 // persistent grid: one CTA per SM, at most one per work item
 static unsigned tc_grid(const TcState* t, const TcArgs& a) {
     return (unsigned)std::max(1, std::min(t->nsm, a.ntiles * a.nct));
+}
+
+template <int MODE>
+static void tc_launch(const TcState* t, int rows, const CUtensorMap& bhi, const CUtensorMap& blo, const CUtensorMap& xhi,
+                      const CUtensorMap& xlo, const TcArgs& a, cudaStream_t s) {
+    if (rows <= TcRing<4>::ROWS)
+        k_tc_gemm<MODE, 4><<<tc_grid(t, a), 256, TcRing<4>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
+    else
+        k_tc_gemm<MODE, 3><<<tc_grid(t, a), 256, TcRing<3>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
 }
 
 // y(:, 0:nrhs) += Z_near xs on the tensor cores (engine 4); x_packed: the X
@@ -936,7 +1082,11 @@ int device_near_tc(Ctx* c, const float2* xs, int ld, int nrhs, double2* y, cudaS
     a.ld = ld;
     a.y = y;
     a.rinv = t->Z.rinv;
-    k_tc_gemm<TCM_NEAR_ADD><<<tc_grid(t, a), 256, TC_SMEM, s>>>(t->Z.mhi, t->Z.mlo, t->mxhi, t->mxlo, a);
+    tc_near_args(c, a);
+    tc_launch<TCM_NEAR_ADD>(t, t->maxrows, t->Z.mhi, t->Z.mlo, t->mxhi, t->mxlo, a, s);
+    if (a.ws)
+        k_tc_sum<true><<<dim3((c->N + 31) / 32, (nrhs + 31) / 32), 256, 0, s>>>(c->N, nrhs, ld, t->nsplit, c->dperm, a.ws,
+                                                                                y, nullptr);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near field") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -954,7 +1104,11 @@ int device_near_pattern_tc(Ctx* c, const float2* Mblk, const float2* xs, int nrh
     a.ld = c->N;
     a.out32 = out;
     a.rinv = t->M.rinv;
-    k_tc_gemm<TCM_NEAR_SET><<<tc_grid(t, a), 256, TC_SMEM, s>>>(t->M.mhi, t->M.mlo, t->mxhi, t->mxlo, a);
+    tc_near_args(c, a);
+    tc_launch<TCM_NEAR_SET>(t, t->maxrows, t->M.mhi, t->M.mlo, t->mxhi, t->mxlo, a, s);
+    if (a.ws)
+        k_tc_sum<false><<<dim3((c->N + 31) / 32, (nrhs + 31) / 32), 256, 0, s>>>(c->N, nrhs, c->N, t->nsplit, c->dperm,
+                                                                                 a.ws, nullptr, out);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near-pattern preconditioner") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -1010,6 +1164,7 @@ static int tc_leaf_setup(Ctx* c, const float2* R, int K2) {
     abase[nb] = (int)arows;
     rbase[nb] = (int)rrows;
     t->natiles = (int)tiles.size();
+    t->arows = std::min(per, K2);
     CK(cudaMalloc(&t->datiles, std::max<size_t>(tiles.size(), 1) * sizeof(int4)));
     CK(cudaMalloc(&t->datchunks, std::max<size_t>(tch.size(), 1) * sizeof(int)));
     CK(cudaMalloc(&t->dabase, abase.size() * sizeof(int)));
@@ -1057,7 +1212,7 @@ int device_agg_tc(Ctx* c, const float2* R, int K, const float2* xs, int nrhs, fl
     a.K2 = 2 * K;
     a.C = C;
     a.rinv = t->RA.rinv;
-    k_tc_gemm<TCM_AGG><<<tc_grid(t, a), 256, TC_SMEM, s>>>(t->RA.mhi, t->RA.mlo, t->mxhi, t->mxlo, a);
+    tc_launch<TCM_AGG>(t, t->arows, t->RA.mhi, t->RA.mlo, t->mxhi, t->mxlo, a, s);
     return cuda_ok(c, cudaGetLastError(), "tensor-core aggregation") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -1080,7 +1235,7 @@ int device_recv_tc(Ctx* c, const float2* R, int K, const float2* A, float facy, 
     a.facy = facy;
     a.ld = ld;
     a.y = y;
-    k_tc_gemm<TCM_RECV><<<tc_grid(t, a), 256, TC_SMEM, s>>>(t->RR.mhi, t->RR.mlo, raw, raw, a);
+    tc_launch<TCM_RECV>(t, t->maxrows, t->RR.mhi, t->RR.mlo, raw, raw, a, s);
     return cuda_ok(c, cudaGetLastError(), "tensor-core receive") ? MLF_OK : MLF_E_CUDA;
 }
 
