@@ -198,6 +198,116 @@ k_ilu_cta(int N, const int* __restrict__ jlu, const int* __restrict__ ju, const 
     for (int i = threadIdx.x; i < N; i += blockDim.x) xc[i] = fail ? make_double2(nan, nan) : xs[i];
 }
 
+// The same sweeps for the narrowest levels (ILUT's: 1.8 rows), where one chain of
+// rows is the time: a warp's FP64 instruction holds its pipe for 64 cycles however
+// few lanes it has, so what counts is the instructions between the arrival of a
+// row's last value and the store of its own.  Lanes 0-15 carry Re and lanes 16-31
+// Im of 16 entries, the entries 0-15 and 16-31 of a batch in sums of their own
+// (the two lanes' sums of the sweeps above): two instructions a step where
+// one lane a batch took four, and the half that waits goes last.  The first
+// reduction step adds the halves, the last operations do Re and Im together.
+// A row that is not there yet holds a signalling NaN, which no operation returns,
+// in place of a flag, a fence and a second read.  12 warps: the polls of more
+// of them slow the chain.  Same sums, bit for bit.
+// Measured against k_ilu_cta: ILUT of 1080 unknowns 1.45 -> 1.11 ms, of 1470 2.33
+// -> 1.93 ms; ILU0 of 1920 (10.7 rows a level) 0.66 -> 0.78 ms, of 13230 5.2 ->
+// 6.6 ms.  8 warps 1.23, 10 1.20, 16 1.27 ms; three batches ahead 1.21 ms.
+constexpr int ILU_N_WARPS = 12;
+constexpr unsigned long long ILU_ABSENT = 0x7ff4dead5eed0001ull;
+
+template <bool FWD>
+__device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* __restrict__ ju,
+                                 const double2* __restrict__ alu, unsigned xa, const double2* rhs,
+                                 volatile int* fail) {
+    constexpr int NU = 4;   // batches loaded ahead
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, v = lane & 15;
+    const bool im = lane >= 16;
+    for (int t = warp; t < N; t += ILU_N_WARPS) {
+        if (__any_sync(0xffffffffu, *fail)) break;
+        const int i = FWD ? t : N - 1 - t;
+        const int k0 = FWD ? jlu[i + 1] : ju[i + 1], k1 = FWD ? ju[i + 1] : jlu[i + 2];
+        const double2 b2 = rhs[i], d = FWD ? make_double2(0, 0) : alu[i + 1];
+        double s[2] = {0, 0};
+        for (int kb = k0; kb < k1; kb += 32 * NU) {
+            unsigned c[2][NU];   // shared address of the entry's x, ~0: no entry
+            double2 a[2][NU];
+#pragma unroll
+            for (int u = 0; u < NU; ++u)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = kb + 32 * u + 16 * h + v;
+                    c[h][u] = k < k1 ? xa + 16u * (unsigned)(jlu[k] - 1) : ~0u;
+                    a[h][u] = k < k1 ? alu[k] : make_double2(0, 0);
+                }
+            // batch u's half h, if its values are there or once they are
+            auto step = [&](int h, int u, bool wait) {
+                const bool has = c[h][u] != ~0u;
+                unsigned long long xr = 0, xi = 0;
+                for (int n = 1;; ++n) {
+                    if (has) asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(xr), "=l"(xi) : "r"(c[h][u]));
+                    if (__all_sync(0xffffffffu, xr != ILU_ABSENT && xi != ILU_ABSENT)) break;
+                    if (!wait) return false;
+                    if ((n & 1023) == 0 && __any_sync(0xffffffffu, n > ILU_SPIN || *fail)) {   // one decision a warp
+                        *fail = 1;
+                        break;
+                    }
+                }
+                if (has) {
+                    s[h] = fma(a[h][u].x, __longlong_as_double(im ? xi : xr), s[h]);
+                    s[h] = fma(im ? a[h][u].y : -a[h][u].y, __longlong_as_double(im ? xr : xi), s[h]);
+                }
+                return true;
+            };
+            int at = NU;   // first batch whose half 0 waits
+#pragma unroll
+            for (int u = 0; u < NU; ++u)
+                if (kb + 32 * u < k1 && u < at && !step(0, u, false)) at = u;
+#pragma unroll
+            for (int u = 0; u < NU; ++u)
+                if (kb + 32 * u + 16 < k1) step(1, u, true);
+#pragma unroll
+            for (int u = 0; u < NU; ++u)
+                if (kb + 32 * u < k1 && u >= at) step(0, u, true);
+        }
+        double q = s[0] + s[1];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        double x = (im ? b2.y : b2.x) - q;
+        if (!FWD) {   // the fused forms of ilu_cta_sweep
+            const double xo = __shfl_xor_sync(0xffffffffu, x, 16);
+            x = fma(d.x, x, __dmul_rn(im ? d.y : -d.y, xo));
+        }
+        if (v == 0) asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(xa + 16u * (unsigned)i + (im ? 8u : 0u)), "d"(x));
+    }
+}
+
+// blockIdx.x = column; dynamic shared memory: x (N double2)
+__global__ void __launch_bounds__(32 * ILU_N_WARPS)
+k_ilu_narrow(int N, const int* __restrict__ jlu, const int* __restrict__ ju, const double2* __restrict__ alu,
+             const double2* __restrict__ y, double2* x) {
+    extern __shared__ __align__(16) unsigned char ilu_smem[];
+    __shared__ int fail;
+    double2* xs = reinterpret_cast<double2*>(ilu_smem);
+    const unsigned xa = (unsigned)__cvta_generic_to_shared(ilu_smem);
+    const double absent = __longlong_as_double((long long)ILU_ABSENT);
+    const double2* yc = y + (size_t)blockIdx.x * N;
+    double2* xc = x + (size_t)blockIdx.x * N;
+    if (threadIdx.x == 0) fail = 0;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) xs[i] = make_double2(absent, absent);
+    __syncthreads();
+    ilu_narrow_sweep<true>(N, jlu, ju, alu, xa, yc, &fail);
+    __syncthreads();
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {   // the forward result is the other sweep's right-hand side
+        xc[i] = xs[i];
+        xs[i] = make_double2(absent, absent);
+    }
+    __syncthreads();
+    ilu_narrow_sweep<false>(N, jlu, ju, alu, xa, xc, &fail);
+    __syncthreads();
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) xc[i] = fail ? make_double2(nan, nan) : xs[i];
+}
+
 // Whether k_ilu_cta takes the factors: x must fit in one CTA's shared memory
 // (13 900 unknowns), and levels must be narrow: one SM takes up to 0.2 us a row
 // (measured 0.15 to 0.20 with ILU0's 180 to 600 levels), a launch per level
@@ -207,6 +317,12 @@ static bool ilu_in_cta(const Ctx* c, int optin) {
     if ((size_t)c->N * (sizeof(double2) + 1) + 1024 > (size_t)optin) return false;
     const double levels = (double)(c->lvl_ptr_f.size() + c->lvl_ptr_b.size() - 2);
     return 2 * ROW_US * c->N < LEVEL_US * levels;
+}
+
+// Whether those rows go to k_ilu_narrow: fewer than four a level (both sides in
+// its comment, at 1.8 and 10.7).
+static bool ilu_narrow(const Ctx* c) {
+    return 2 * (size_t)c->N < 4 * (c->lvl_ptr_f.size() + c->lvl_ptr_b.size() - 2);
 }
 
 int device_ilu_upload(Ctx* c) {
@@ -229,6 +345,7 @@ int device_ilu_upload(Ctx* c) {
         if ((st = up(&c->dalu64, a64))) return st;
         // a limit of the kernel, shared by every context: the device's maximum
         CK(cudaFuncSetAttribute(k_ilu_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+        CK(cudaFuncSetAttribute(k_ilu_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
         return MLF_OK;
     }
     if ((st = up(&c->dalu, c->alu)) || (st = up(&c->dlvl_rows_f, c->lvl_rows_f)) ||
@@ -244,8 +361,12 @@ int device_ilu_solve(Ctx* c, const double2* y, double2* x, int nrhs, cudaStream_
         return MLF_E_STATE;
     }
     if (c->dalu64) {
-        k_ilu_cta<<<nrhs, 32 * ILU_WARPS, (size_t)c->N * (sizeof(double2) + 1), s>>>(c->N, c->djlu, c->dju, c->dalu64,
-                                                                                     y, x);
+        if (ilu_narrow(c))
+            k_ilu_narrow<<<nrhs, 32 * ILU_N_WARPS, (size_t)c->N * sizeof(double2), s>>>(c->N, c->djlu, c->dju, c->dalu64,
+                                                                                       y, x);
+        else
+            k_ilu_cta<<<nrhs, 32 * ILU_WARPS, (size_t)c->N * (sizeof(double2) + 1), s>>>(c->N, c->djlu, c->dju,
+                                                                                         c->dalu64, y, x);
         return cuda_ok(c, cudaGetLastError(), "ilu sweeps") ? MLF_OK : MLF_E_CUDA;
     }
     const int nlf = (int)c->lvl_ptr_f.size() - 1, nlb = (int)c->lvl_ptr_b.size() - 1;

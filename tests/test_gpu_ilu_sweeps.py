@@ -51,3 +51,23 @@ def test_sweeps_carry_nan(gpu_lib):
         assert np.isnan(x).any()
         y[m.N // 2] = 1.0
         assert np.isfinite(m.lusol0C(y)).all()
+
+
+@pytest.mark.parametrize("level,radius,fill,droptol", [(2, 0.6, 1.0, 1e-2), (2, 0.6, 60.0, 1e-6), (3, 1.0, 5.0, 1e-3),
+                                                       (3, 1.0, 20.0, 1e-5)])
+def test_narrow_levels(level, radius, fill, droptol, gpu_lib):
+    """ILUT factors of few rows a level: rows of less than half a batch of 32
+    entries up to rows of several loads of four batches; NaN is carried."""
+    from lywell_gb300 import MLFMA, RWG, meshes
+    with MLFMA(RWG(meshes.icosphere(level, radius)), lam=1.0, ladomax=0.25) as m:
+        assert m.ilut(fill, droptol) == 0
+        alu, jlu, ju = m.ilu0_factors()
+        rng = np.random.default_rng(level)
+        y = rng.standard_normal((m.N, 2)) + 1j * rng.standard_normal((m.N, 2))
+        x = m.lusol0C(y)
+        for c in range(2):
+            ref = _lusol(alu, jlu, ju, y[:, c])   # same bound as above
+            assert np.linalg.norm(x[:, c] - ref) < 1e-10 * np.linalg.norm(ref)
+        y[m.N // 2, 0] = np.nan
+        z = m.lusol0C(y)
+        assert np.isnan(z[:, 0]).any() and np.array_equal(z[:, 1], x[:, 1])
