@@ -209,11 +209,11 @@ k_ilu_cta(int N, const int* __restrict__ jlu, const int* __restrict__ ju, const 
 // A row that is not there yet holds a signalling NaN, which no operation returns,
 // in place of a flag, a fence and a second read.  12 warps: the polls of more
 // of them slow the chain.  Same sums, bit for bit.
-// Measured against k_ilu_cta: ILUT of 1080 unknowns 1.45 -> 1.11 ms, of 1470 2.33
-// -> 1.93 ms; ILU0 of 1920 (10.7 rows a level) 0.66 -> 0.78 ms, of 13230 5.2 ->
-// 6.6 ms.  8 warps 1.23, 10 1.20, 16 1.27 ms; three batches ahead 1.21 ms.
+// Measured against k_ilu_cta: ILUT of 1080 unknowns 1.45 -> 1.04 ms, of 1470 2.33
+// -> 1.82 ms; ILU0 of 1920 (10.7 rows a level) 0.66 -> 0.78 ms, of 13230 5.2 ->
+// 6.6 ms.  8 warps 1.14, 16 1.17 ms; three batches ahead 1.21 ms.
 constexpr int ILU_N_WARPS = 12;
-constexpr unsigned long long ILU_ABSENT = 0x7ff4dead5eed0001ull;
+constexpr unsigned ILU_ABSENT_HI = 0x7ff4deadu;   // high word of it
 
 template <bool FWD>
 __device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* __restrict__ ju,
@@ -238,14 +238,23 @@ __device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* 
                     const int k = kb + 32 * u + 16 * h + v;
                     c[h][u] = k < k1 ? xa + 16u * (unsigned)(jlu[k] - 1) : ~0u;
                     a[h][u] = k < k1 ? alu[k] : make_double2(0, 0);
+                    if (!im) a[h][u].y = -a[h][u].y;
                 }
+            // the entry's x, own part and other part; false: not there yet
+            auto load = [&](unsigned at, double& own, double& oth) {
+                unsigned rl, rh, il, ih;
+                asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(rl), "=r"(rh), "=r"(il), "=r"(ih) : "r"(at));
+                const double r = __hiloint2double((int)rh, (int)rl), i = __hiloint2double((int)ih, (int)il);
+                own = im ? i : r;
+                oth = im ? r : i;
+                return rh != ILU_ABSENT_HI && ih != ILU_ABSENT_HI;
+            };
             // batch u's half h, if its values are there or once they are
             auto step = [&](int h, int u, bool wait) {
                 const bool has = c[h][u] != ~0u;
-                unsigned long long xr = 0, xi = 0;
-                for (int n = 1;; ++n) {
-                    if (has) asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(xr), "=l"(xi) : "r"(c[h][u]));
-                    if (__all_sync(0xffffffffu, xr != ILU_ABSENT && xi != ILU_ABSENT)) break;
+                double own = 0, oth = 0;
+                for (int n = 1; !__all_sync(0xffffffffu, !has || load(c[h][u], own, oth)); ++n) {
                     if (!wait) return false;
                     if ((n & 1023) == 0 && __any_sync(0xffffffffu, n > ILU_SPIN || *fail)) {   // one decision a warp
                         *fail = 1;
@@ -253,8 +262,8 @@ __device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* 
                     }
                 }
                 if (has) {
-                    s[h] = fma(a[h][u].x, __longlong_as_double(im ? xi : xr), s[h]);
-                    s[h] = fma(im ? a[h][u].y : -a[h][u].y, __longlong_as_double(im ? xr : xi), s[h]);
+                    s[h] = fma(a[h][u].x, own, s[h]);
+                    s[h] = fma(a[h][u].y, oth, s[h]);
                 }
                 return true;
             };
@@ -265,9 +274,26 @@ __device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* 
 #pragma unroll
             for (int u = 0; u < NU; ++u)
                 if (kb + 32 * u + 16 < k1) step(1, u, true);
+            if (at == NU) continue;
+            // half 0 from there, what is there behind the awaited batch read beforehand
+            double own[NU], oth[NU];
+            unsigned there = 0;
+#pragma unroll
+            for (int u = 1; u < NU; ++u)
+                if (u > at && kb + 32 * u < k1) {
+                    own[u] = oth[u] = 0;
+                    if (__all_sync(0xffffffffu, c[0][u] == ~0u || load(c[0][u], own[u], oth[u]))) there |= 1u << u;
+                }
 #pragma unroll
             for (int u = 0; u < NU; ++u)
-                if (kb + 32 * u < k1 && u >= at) step(0, u, true);
+                if (u >= at && kb + 32 * u < k1) {
+                    if (!(there >> u & 1)) {
+                        step(0, u, true);
+                    } else if (c[0][u] != ~0u) {
+                        s[0] = fma(a[0][u].x, own[u], s[0]);
+                        s[0] = fma(a[0][u].y, oth[u], s[0]);
+                    }
+                }
         }
         double q = s[0] + s[1];
 #pragma unroll
@@ -289,7 +315,7 @@ k_ilu_narrow(int N, const int* __restrict__ jlu, const int* __restrict__ ju, con
     __shared__ int fail;
     double2* xs = reinterpret_cast<double2*>(ilu_smem);
     const unsigned xa = (unsigned)__cvta_generic_to_shared(ilu_smem);
-    const double absent = __longlong_as_double((long long)ILU_ABSENT);
+    const double absent = __hiloint2double((int)ILU_ABSENT_HI, 1);
     const double2* yc = y + (size_t)blockIdx.x * N;
     double2* xc = x + (size_t)blockIdx.x * N;
     if (threadIdx.x == 0) fail = 0;
