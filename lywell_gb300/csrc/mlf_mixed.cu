@@ -595,8 +595,8 @@ static int matvec32_core(Ctx* c, const double2* x, const float2* x32, double2* y
             const float2* Aleaf = nl == 3 ? c->m32.lv[nl].B : c->m32.lv[nl].A;
             if (blk_engine_of(c) == 4) {
                 // the X operand was packed by the aggregation of this product
-                if ((st = device_recv_tc(c, c->m32.R, leaf.K, Aleaf, facy, nrhs, ld, y, s))) return st;
-                st = device_near_tc(c, c->m32.xT, ld, nrhs, y, s, true);
+                if ((st = device_recv_tc(c, c->m32.R, leaf.K, Aleaf, facy, nrhs, s))) return st;
+                st = device_near_tc(c, ld, nrhs, y, s);
             } else {
                 if ((st = device_recv_blocks32(c, c->m32.R, leaf.K, Aleaf, facy, nrhs, ld, y, s))) return st;
                 st = device_near_blocks32(c, c->m32.xT, ld, nrhs, y, s);

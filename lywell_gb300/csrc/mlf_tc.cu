@@ -35,9 +35,9 @@
 // canonical K-major SWIZZLE_128B layout tcgen05.mma reads (8-row atoms of
 // 1024 bytes).
 //
-// A persistent CTA (8 warps) per SM walks work items (tile of at most 160
-// rows, 64 columns; a part of the near list where tiles are few, the parts' sums
-// added by k_tc_sum).  Thread 0 issues the TMA loads of a 3- or 4-stage ring; thread
+// A persistent CTA (8 warps, the receive's 10) per SM walks its share of the work
+// (tiles of at most 160 rows, 64 columns, cut into parts where shares meet, the
+// parts' sums added by k_tc_sum).  Thread 0 issues the TMA loads of a 3- or 4-stage ring; thread
 // 32 issues the MMAs: per chunk of 32 real K, 4 K-steps x 3 products (A_lo
 // B_hi, A_hi B_lo, A_hi B_hi) into a 128 x N FP32 accumulator in TMEM, and
 // tcgen05.commit frees a stage once its MMAs are done.  Warps 4-7 read their
@@ -54,6 +54,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <vector>
 
@@ -71,7 +72,7 @@ constexpr int TC_ROWS = 160;                 // bases of box i per tile (MMA N <
 constexpr int TC_KCH = 16;                   // complex contraction values per 128-byte TF32 row (receive)
 constexpr int TC_KCH_H = 32;                 // complex contraction values per 128-byte FP16 row (near, aggregation)
 constexpr int TC_COLS = 64;                  // right-hand sides per column tile (MMA M = 128)
-constexpr int TC_ZBOX = 32;                  // rows per TMA box of the Z operand
+constexpr int TC_ZBOX = 32;                  // rows per TMA box of the B operands
 constexpr int TC_ABYTES = 128 * 128;         // one A tile: 128 rows x 128 bytes
 // The ring: three stages of 72 KB for tiles of up to 160 rows, or four of 56 KB
 // where no tile has more than 96 (bytes in flight bound the kernel).
@@ -81,7 +82,7 @@ template <int ST> struct TcRing {
     static constexpr int STAGE = 2 * TC_ABYTES + 2 * BBYTES;
     static constexpr size_t SMEM = (size_t)ST * STAGE + 1024;   // + alignment of the ring
 };
-constexpr int TC_MAX_SPLIT = 8;              // parts of a tile's near list at most
+constexpr int TC_PARTS = 15;                 // parts of a tile at most (about)
 constexpr uint32_t TC_TMEM_COLS = 256;
 constexpr uint32_t TC_SPIN = 1u << 20;       // mbarrier polls before a wait gives up
 
@@ -95,22 +96,28 @@ struct TcOperand {
     CUtensorMap mhi, mlo;
 };
 
+// A GEMM's work in shares for the persistent CTAs: items (tile, run of its chunks)
+struct TcSlots {
+    int n = 0;                      // shares
+    int* ptr = nullptr;             // share -> its items
+    int4* item = nullptr;           // (box, first row, rows, part of the tile)
+    int2* ch = nullptr;             // first chunk, chunks
+    int parts = 0;                  // parts of a tile at most
+    unsigned char* np = nullptr;    // per box-sorted basis: parts of its tile
+};
+
 struct TcState {
-    int ntiles = 0, nchunk = 0;     // tiles of the near GEMM; chunks of 32 bases over all boxes
+    int nchunk = 0;                 // chunks of 32 bases over all boxes
     long long zrows = 0;            // rows of the Z-operand layout
     int nsm = 0;                    // SMs: CTAs of the persistent GEMM
-    int4* dtiles = nullptr;         // (box, first row, rows, -), by decreasing work
-    int* dtchunks = nullptr;        // per tile: chunks over its near boxes
-    int maxrows = 0;                // rows of the largest tile
-    // near field and preconditioner: the tiles again, in nsplit parts of their near
-    // lists where tiles are few: (box, first row, rows, part), chunks and first
-    // block entry of each part
-    int nsplit = 1, nstiles = 0;
-    int4* dstiles = nullptr;
-    int *dstchunks = nullptr, *dsfirst = nullptr;
-    float2* dws = nullptr;          // their sums [part][box-sorted basis][column]
+    std::vector<int4> tiles;        // (box, first row, rows, -)
+    int maxrows = 0;                // rows of the largest
+    TcSlots near, recv, agg;
+    int2* dlist = nullptr;          // near chunks of each box in order: (chunk of the X operand, Z-operand row)
+    float2* dws = nullptr;          // parts' sums [part][box-sorted basis][column], the near field's, then the receive's
     size_t ws_cap = 0;
     int* dzrow = nullptr;           // per block entry e: first Z-operand row (chunk 0)
+    int* dpos = nullptr;            // box-sorted position of each basis
     int* dcbase = nullptr;          // per box: its first chunk
     int2* dchunk = nullptr;         // per chunk: (first box-sorted position, bases in it)
     int* derr = nullptr;            // set by a CTA whose wait gave up
@@ -126,9 +133,7 @@ struct TcState {
     // leaf aggregation and receive (built from the FP32 patterns R on first use)
     const float2* Rsrc = nullptr;   // the patterns the operands below hold
     int K2 = 0;                     // 2K directions of the leaf level
-    int natiles = 0, arows = 0;     // tiles of the aggregation, rows of the largest
-    int4* datiles = nullptr;        // aggregation tiles (box, first direction, directions, -)
-    int* datchunks = nullptr;       // per aggregation tile: chunks of the box's bases
+    int arows = 0;                  // rows of the largest aggregation tile
     int* dabase = nullptr;          // per box: first row of the aggregation operand
     int* drbase = nullptr;          // per box: first row of the receive operand
     TcOperand RA;                   // R^T per box and chunk of 32 bases: 2K rows of 32 FP16 (re, im)
@@ -324,54 +329,44 @@ __global__ void k_tc_fill_rr(int K2, const int* __restrict__ box_ptr, const int*
 // ---------------------------------------------------------------------------
 
 // What one launch computes (B the operand streamed by TMA, X the right-hand
-// side operand, tile = (box i, first row r0, rows, instruction descriptor)):
-//   TCM_NEAR_ADD  y (FP64 columns, ld) += Z X over the near boxes j of box i
-//   TCM_NEAR_SET  out32 (FP32 columns, ld) = M X, M on the near pattern
+// side operand, item = (box i, first row r0, rows, part)):
+//   TCM_NEAR      part of Z X (or M X, M on the near pattern) over the near boxes j
+//                 of box i, to ws
 //   TCM_AGG       C(q, col, i) = sum_t R(t, q) x(t, col), t over box i's bases,
 //                 q = r0 .. r0 + rows - 1 of the 2K directions
-//   TCM_RECV      y(basis, col) = j facy sum_q conj R(basis, q) A(q, col, i)
+//   TCM_RECV      part of j facy sum_q conj R(basis, q) A(q, col, i), to ws
 // The aggregation takes the near field's packed X operand (the box's own
 // chunks); the receive stages raw rows of the A field (64 columns x 16
-// directions, 128-byte swizzled) by TMA and warps 2-3 expand them in shared memory
+// directions, 128-byte swizzled) by TMA and warps 2, 3, 8, 9 expand them in shared memory
 // into the [re, -im] / [im, re] row pairs, split into TF32 hi and lo.
 //
-// Persistent: one CTA per SM walks the work items q = blockIdx.x + k gridDim.x,
-// item q = (tile q / nct, column tile q % nct), the tiles ordered by
-// decreasing work.  Warp roles: warp 0 lane 0 issues the TMA loads, warp 1
-// lane 0 the MMAs, warps 2-3 expand the receive's raw rows, warps 4-7 read
+// Persistent: one CTA per SM takes the shares (tc_slots) and column tiles q =
+// blockIdx.x + k gridDim.x, the column tiles of a share on neighbouring CTAs, which
+// read the same B rows.  Warp roles: warp 0 lane 0 issues the TMA loads, warp 1
+// lane 0 the MMAs, warps 2, 3, 8, 9 expand the receive's raw rows, warps 4-7 read
 // the accumulators out (warp 4 + w owns TMEM lanes 32 w .. 32 w + 31).  Two
 // TMEM accumulators of 256 columns alternate between items, so the loads and
 // MMAs of the next item run under the epilogue of the previous one; the
 // shared-memory ring and its barrier phases run on across items.
-enum : int { TCM_NEAR_ADD = 0, TCM_NEAR_SET = 1, TCM_AGG = 2, TCM_RECV = 3 };
+enum : int { TCM_NEAR = 0, TCM_AGG = 1, TCM_RECV = 2 };
 
 struct TcArgs {
-    const int4* tiles;
-    const int* tchunks;  // per tile: chunks of its contraction (near, aggregation)
-    int ntiles, nct;     // tiles, column tiles of 64
+    int nslots, nct;         // shares of the work, column tiles of 64
+    const int* slot;         // TcSlots ptr, item, ch
+    const int4* item;
+    const int2* ch;
     const int* box_ptr;
-    const int* nbox_ptr;
-    const int* nbox_list;
-    const int* zrow;     // near: per block entry; aggregation, receive: per box -- first B row
-    const int* cbase;    // per box: its first chunk of the X operand
-    const int* first;    // near: per tile, first block entry of its part
-    int nchunk, nrhs, ld, K2;
+    const int2* list;        // near: chunks of the boxes' near lists
+    const int* zrow;         // aggregation, receive: per box -- first B row
+    const int* cbase;        // aggregation: per box, its first chunk of the X operand
+    int nchunk, nrhs, K2, N;
     float facy;
-    const float* rinv;   // FP16 modes: per output row (near: box-sorted basis; aggregation: box x 2K), 1 / scale
-    const float* cinv;   // FP16 modes: per column, 1 / scale
-    const int* perm;
-    double2* y;
-    float2* out32;
-    float2* C;
-    float2* ws;          // near: the parts' sums, to be added by k_tc_sum (null: one part, written at once)
-    int N;
+    const float* rinv;       // FP16 modes: per output row (near: box-sorted basis; aggregation: box x 2K), 1 / scale
+    const float* cinv;       // FP16 modes: per column, 1 / scale
+    float2* C;               // aggregation
+    float2* ws;              // near, receive: parts' sums, for k_tc_sum
     int* err;
 };
-
-template <int MODE>
-__device__ __forceinline__ int tc_item_chunks(const TcArgs& a, int tile) {
-    return MODE == TCM_RECV ? (a.K2 + TC_KCH - 1) / TC_KCH : a.tchunks[tile];
-}
 
 // Operands of the near field, its preconditioner and the aggregation are FP16
 // (kind::f16, 32 complex values per 128-byte row); the receive's are TF32
@@ -383,11 +378,14 @@ struct TcFmt {
     static constexpr int KCH = H ? TC_KCH_H : TC_KCH;
 };
 
+template <int MODE>
+constexpr int TC_THREADS = MODE == TCM_RECV ? 320 : 256;
+
 template <int MODE, int ST>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mbhi, const __grid_constant__ CUtensorMap mblo,
               const __grid_constant__ CUtensorMap mxhi, const __grid_constant__ CUtensorMap mxlo, const TcArgs a) {
-    constexpr bool NEAR = MODE == TCM_NEAR_ADD || MODE == TCM_NEAR_SET;
+    constexpr bool NEAR = MODE == TCM_NEAR;
     constexpr bool RAW = MODE == TCM_RECV;
     constexpr int STAGE = TcRing<ST>::STAGE, BBYTES = TcRing<ST>::BBYTES;
     constexpr uint32_t RAW_BYTES = TC_COLS * 128;   // 64 field rows of 16 complex values
@@ -398,13 +396,13 @@ __global__ void __launch_bounds__(256, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t raw = tc::smem_u32(tc_raw);
     unsigned char* ring = tc_raw + (((raw + 1023u) & ~1023u) - raw);   // 1024-aligned swizzle atoms
-    const int nitems = a.ntiles * a.nct;
+    const int nwork = a.nslots * a.nct;
     volatile int* vfail = &fail_s;
     if (tid == 0) {
         for (int s = 0; s < ST; ++s) {
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
-            tc::mbar_init(&conv[s], 64);
+            tc::mbar_init(&conv[s], 128);
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&accf[b], 1);
@@ -439,15 +437,16 @@ __global__ void __launch_bounds__(256, 1)
             const uint64_t pol_b = tc::l2_evict_first();
             uint32_t g = 0;
             bool ok = true;
-            for (int q = blockIdx.x; q < nitems && ok; q += gridDim.x) {
-                const int tile = q / a.nct, ct = q - tile * a.nct;
-                const int4 tl = a.tiles[tile];
-                const int i = tl.x, r0 = tl.y, nrow = tl.z;
+            for (int q = blockIdx.x; q < nwork && ok; q += gridDim.x) {
+            const int sl = q / a.nct, ct = q - sl * a.nct, t1 = a.slot[sl + 1];
+            for (int it = a.slot[sl]; it < t1 && ok; ++it) {
+                const int4 tl = a.item[it];
+                const int2 ch = a.ch[it];
+                const int i = tl.x, r0 = tl.y, nrow = tl.z, nch = ch.y;
                 const int ni = a.box_ptr[i + 1] - a.box_ptr[i];
-                const int nch = tc_item_chunks<MODE>(a, tile);
                 const int nB = (nrow + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX;          // B rows staged
                 const uint32_t bytes = (RAW ? RAW_BYTES : 2u * TC_ABYTES) + 2u * (uint32_t)nB * 128u;
-                int le = NEAR ? a.first[tile] : 0, lkc = 0;
+                int2 next = NEAR && nch ? a.list[ch.x] : make_int2(0, 0);   // a chunk ahead of its use
                 for (int cI = 0; cI < nch; ++cI, ++g) {
                     const int s = g % ST;
                     if ((g >= ST && !tc::mbar_wait(&empty[s], ((g / ST) - 1) & 1, TC_SPIN)) || *vfail) {
@@ -458,15 +457,11 @@ __global__ void __launch_bounds__(256, 1)
                     tc::mbar_arrive_expect_tx(&full[s], bytes);
                     int zr;
                     if (NEAR) {
-                        const int j = a.nbox_list[le];
-                        const int xr = (ct * a.nchunk + a.cbase[j] + lkc) * 128;
+                        const int xr = (ct * a.nchunk + next.x) * 128;
+                        zr = next.y + r0;
                         tc::tma_load_2d(st, &mxhi, 0, xr, &full[s]);
                         tc::tma_load_2d(st + TC_ABYTES, &mxlo, 0, xr, &full[s]);
-                        zr = a.zrow[le] + lkc * ni + r0;
-                        if (++lkc * TcFmt<MODE>::KCH >= a.box_ptr[j + 1] - a.box_ptr[j]) {
-                            lkc = 0;
-                            ++le;
-                        }
+                        if (cI + 1 < nch) next = a.list[ch.x + cI + 1];
                     } else if (MODE == TCM_AGG) {
                         const int xr = (ct * a.nchunk + a.cbase[i] + cI) * 128;
                         tc::tma_load_2d(st, &mxhi, 0, xr, &full[s]);
@@ -474,18 +469,18 @@ __global__ void __launch_bounds__(256, 1)
                         zr = a.zrow[i] + cI * a.K2 + r0;
                     } else {
                         // raw field rows (box i, columns of this tile) into the lo tile's first 8 KB
-                        tc::tma_load_2d_hint(st + TC_ABYTES, &mxhi, 2 * TC_KCH * cI, i * a.nrhs + ct * TC_COLS,
+                        tc::tma_load_2d_hint(st + TC_ABYTES, &mxhi, 2 * TC_KCH * (ch.x + cI), i * a.nrhs + ct * TC_COLS,
                                              &full[s], pol_b);
-                        zr = a.zrow[i] + cI * ni + r0;
+                        zr = a.zrow[i] + (ch.x + cI) * ni + r0;
                     }
+                    // the aggregation's and receive's pattern operands are read by the
+                    // tiles of one box (and the column tiles) only: streamed too
                     for (int qq = 0; qq < nB; qq += TC_ZBOX) {
-                        // the aggregation's and receive's pattern operands are read by the
-                        // tiles of one box (and the column tiles) only: streamed too
                         tc::tma_load_2d_hint(st + 2 * TC_ABYTES + qq * 128, &mbhi, 0, zr + qq, &full[s], pol_b);
-                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s],
-                                             pol_b);
+                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s], pol_b);
                     }
                 }
+            }
             }
             issued_s = (int)g;
             if (!ok) *vfail = 1;
@@ -495,9 +490,10 @@ __global__ void __launch_bounds__(256, 1)
             // MMA issuer: per chunk 4 K steps x 3 products into the item's TMEM accumulator
             uint32_t g = 0, na = 0;
             bool ok = true;
-            for (int q = blockIdx.x; q < nitems && ok; q += gridDim.x) {
-                const int tile = q / a.nct;
-                const int nch = tc_item_chunks<MODE>(a, tile);
+            for (int q = blockIdx.x; q < nwork && ok; q += gridDim.x) {
+            const int sl = q / a.nct, t1 = a.slot[sl + 1];
+            for (int it = a.slot[sl]; it < t1; ++it) {
+                const int nch = a.ch[it].y;
                 if (nch == 0) continue;
                 const uint32_t buf = na & 1;
                 if (na >= 2 && !tc::mbar_wait(&acce[buf], ((na >> 1) - 1) & 1, TC_SPIN)) {
@@ -506,7 +502,7 @@ __global__ void __launch_bounds__(256, 1)
                 }
                 tc::tc_fence_after_sync();
                 const uint32_t d = tmem + buf * TC_TMEM_COLS;
-                const uint32_t idesc = tc::instr_desc_f32acc(TcFmt<MODE>::FMT, 128, (a.tiles[tile].z + 15) / 16 * 16);
+                const uint32_t idesc = tc::instr_desc_f32acc(TcFmt<MODE>::FMT, 128, (a.item[it].z + 15) / 16 * 16);
                 for (int cI = 0; cI < nch; ++cI, ++g) {
                     const int s = g % ST;
                     const uint32_t par = (g / ST) & 1;
@@ -538,6 +534,7 @@ __global__ void __launch_bounds__(256, 1)
                 tc::mma_commit(&accf[buf]);   // the item's accumulator is complete
                 ++na;
             }
+            }
             if (g > 0) {
                 tc::mma_commit(&done);   // every MMA issued above
                 if (!tc::mbar_wait(&done, 0, TC_SPIN)) ok = false;
@@ -545,20 +542,24 @@ __global__ void __launch_bounds__(256, 1)
             consumed_s = (int)g;
             if (!ok) *vfail = 1;
         }
-    } else if (warp < 4) {
+    } else if (warp < 4 || warp >= 8) {
         if (RAW && !skip_all) {
-            // converters: thread cl expands field row cl (column ct 64 + cl) of each chunk
-            const int cl = tid - 64;
+            // converters (warps 2, 3, 8, 9): threads cl and 64 + cl expand half of field row
+            // cl (column ct 64 + cl) of each chunk each; with one thread a row this was the
+            // receive's time (2350 cycles a chunk)
+            const int cid = warp < 4 ? tid - 64 : tid - 192, cl = cid & 63, kh = cid >> 6 << 2;
             uint32_t g = 0;
             bool go = true;
-            for (int q = blockIdx.x; q < nitems && go; q += gridDim.x) {
-                const int nch = tc_item_chunks<MODE>(a, q / a.nct);
+            for (int q = blockIdx.x; q < nwork && go; q += gridDim.x) {
+            const int sl = q / a.nct, t1 = a.slot[sl + 1];
+            for (int it = a.slot[sl]; it < t1 && go; ++it) {
+                const int nch = a.ch[it].y;
                 for (int cI = 0; cI < nch; ++cI, ++g) {
                     const int s = g % ST;
                     const uint32_t par = (g / ST) & 1;
-                    if (cl == 0) cvok_s = (!*vfail && tc::mbar_wait(&full[s], par, TC_SPIN)) ? 1 : 0;
-                    tc::named_bar_sync(1, 64);
-                    if (!cvok_s) {   // the same decision in all 64 threads
+                    if (cid == 0) cvok_s = (!*vfail && tc::mbar_wait(&full[s], par, TC_SPIN)) ? 1 : 0;
+                    tc::named_bar_sync(1, 128);
+                    if (!cvok_s) {   // the same decision in all 128 threads
                         go = false;
                         break;
                     }
@@ -567,18 +568,18 @@ __global__ void __launch_bounds__(256, 1)
                     // the raw rows arrive 128-byte swizzled: chunk k of row cl sits at
                     // k ^ (cl & 7), so the 8 lanes of a shared-memory wavefront read 8
                     // different bank groups
-                    float4 v[8];
+                    float4 v[4];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        v[k] = *reinterpret_cast<const float4*>(st + TC_ABYTES + tc::sw128_offset(cl, k));
-                    tc::named_bar_sync(1, 64);   // every raw row is read before the lo tile overwrites them
+                    for (int k = 0; k < 4; ++k)
+                        v[k] = *reinterpret_cast<const float4*>(st + TC_ABYTES + tc::sw128_offset(cl, kh + k));
+                    tc::named_bar_sync(1, 128);   // every raw row is read before the lo tile overwrites them
                     // rows 2cl and 2cl+1 place chunk k at k ^ (2cl & 7) (resp. +1): lanes
                     // with cl & 4 take the chunks in the order k ^ 1 so that the 8 lanes
                     // of a wavefront again store to 8 different bank groups
                     const int flip = (cl >> 2) & 1;
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {   // 16-byte chunk k: complex values 2k, 2k+1
-                        const int k = kk ^ flip;
+                    for (int kk = 0; kk < 4; ++kk) {   // 16-byte chunk k: complex values 2k, 2k+1
+                        const int k = kh + (kk ^ flip);
                         const float4 w = flip ? v[kk ^ 1] : v[kk];
                         // row 2cl: (re, -im) pairs; row 2cl+1: (im, re) -- the same values, so
                         // its hi and lo parts follow from row 2cl's (the rounding is symmetric)
@@ -598,35 +599,35 @@ __global__ void __launch_bounds__(256, 1)
                     tc::mbar_arrive(&conv[s]);
                 }
             }
+            }
         }
     } else if (!skip_all) {
         // epilogue: warp 4 + ew reads accumulator rows (TMEM lanes) 32 ew .. 32 ew + 31
         const int ew = warp - 4;
         const int m = 32 * ew + lane;                   // D row = TMEM lane
         uint32_t na = 0;
-        for (int q = blockIdx.x; q < nitems; q += gridDim.x) {
-            const int tile = q / a.nct, ct = q - tile * a.nct;
-            const int4 tl = a.tiles[tile];
+        bool go = true;
+        for (int q = blockIdx.x; q < nwork && go; q += gridDim.x) {
+        const int sl = q / a.nct, ct = q - sl * a.nct, t1 = a.slot[sl + 1];
+        const int col = ct * TC_COLS + (m >> 1), odd = lane & 1;
+        const bool writer = col < a.nrhs;
+        const float cs = (TcFmt<MODE>::H && writer) ? a.cinv[col] : 1.f;
+        for (int it = a.slot[sl]; it < t1; ++it) {
+            const int4 tl = a.item[it];
             const int i = tl.x, r0 = tl.y, nrow = tl.z;
-            const int i0 = a.box_ptr[i];
-            const int col = ct * TC_COLS + (m >> 1);
-            const bool writer = (lane & 1) == 0 && col < a.nrhs;
-            const float cs = (TcFmt<MODE>::H && writer) ? a.cinv[col] : 1.f;
-            if (tc_item_chunks<MODE>(a, tile) == 0) {
+            if (a.ch[it].y == 0) {
                 // a box without bases radiates nothing
-                if (MODE == TCM_AGG && writer)
+                if (MODE == TCM_AGG && writer && !odd)
                     for (int p = 0; p < nrow; ++p) a.C[((size_t)i * a.nrhs + col) * a.K2 + r0 + p] = make_float2(0.f, 0.f);
-                // nor does a part that got no box add anything
-                if (NEAR && a.ws && writer)
-                    for (int p = 0; p < nrow; ++p)
-                        a.ws[((size_t)tl.w * a.N + i0 + r0 + p) * a.nrhs + col] = make_float2(0.f, 0.f);
                 continue;
             }
+            const int i0 = a.box_ptr[i];
             const uint32_t buf = na & 1;
             // a warp-uniform decision: tcgen05.ld below is a whole-warp instruction
             const bool got = __all_sync(0xffffffffu, tc::mbar_wait(&accf[buf], (na >> 1) & 1, TC_SPIN) ? 1 : 0);
             if (!got) {
                 *vfail = 1;
+                go = false;
                 break;
             }
             tc::tc_fence_after_sync();
@@ -634,29 +635,38 @@ __global__ void __launch_bounds__(256, 1)
             for (int n0 = 0; n0 < nrow; n0 += 32) {
                 float v[32];
                 tc::tmem_ld_32x32b_x32(d + (uint32_t)n0, v);
+                // lane 2c holds Re and lane 2c + 1 Im of column c
+                if (MODE == TCM_AGG) {
+                    // of four rows the even lane writes two, the odd lane two: 32 bytes of
+                    // the column's field a pair (8-byte stores by even lanes were a
+                    // sector each: 27 000 cycles an item, most of the kernel)
 #pragma unroll
-                for (int u = 0; u < 32; ++u) {
-                    const float im = __shfl_xor_sync(0xffffffffu, v[u], 1);
-                    const int p = n0 + u;
-                    if (writer && p < nrow) {
-                        if (NEAR && a.ws) {
-                            const float rs = a.rinv[i0 + r0 + p];   // powers of two: exact
-                            a.ws[((size_t)tl.w * a.N + i0 + r0 + p) * a.nrhs + col] =
-                                make_float2(v[u] * rs * cs, im * rs * cs);
-                        } else if (MODE == TCM_NEAR_ADD) {
-                            const float rs = a.rinv[i0 + r0 + p];
-                            double2* yp = a.y + (size_t)col * a.ld + a.perm[i0 + r0 + p];
-                            const double2 o = *yp;
-                            *yp = make_double2(o.x + (double)(v[u] * rs * cs), o.y + (double)(im * rs * cs));
-                        } else if (MODE == TCM_NEAR_SET) {
-                            const float rs = a.rinv[i0 + r0 + p];
-                            a.out32[(size_t)col * a.ld + a.perm[i0 + r0 + p]] = make_float2(v[u] * rs * cs, im * rs * cs);
-                        } else if (MODE == TCM_AGG) {
-                            const float rs = a.rinv[(size_t)i * a.K2 + r0 + p];
-                            a.C[((size_t)i * a.nrhs + col) * a.K2 + r0 + p] = make_float2(v[u] * rs * cs, im * rs * cs);
-                        } else {
-                            a.y[(size_t)col * a.ld + a.perm[i0 + r0 + p]] =
-                                make_double2(-(double)(a.facy * im), (double)(a.facy * v[u]));
+                    for (int u = 0; u < 32; u += 4) {
+                        const float e0 = __shfl_xor_sync(0xffffffffu, odd ? v[u] : v[u + 2], 1);
+                        const float e1 = __shfl_xor_sync(0xffffffffu, odd ? v[u + 1] : v[u + 3], 1);
+                        const int p = n0 + u + 2 * odd;
+                        if (writer && p < nrow) {   // rows and 2K are even
+                            const float2 rs = *reinterpret_cast<const float2*>(a.rinv + (size_t)i * a.K2 + r0 + p);
+                            const float4 w = odd ? make_float4(e0, v[u + 2], e1, v[u + 3])
+                                                 : make_float4(v[u], e0, v[u + 1], e1);
+                            // powers of two: exact
+                            *reinterpret_cast<float4*>(a.C + ((size_t)i * a.nrhs + col) * a.K2 + r0 + p) =
+                                make_float4(w.x * rs.x * cs, w.y * rs.x * cs, w.z * rs.y * cs, w.w * rs.y * cs);
+                        }
+                    }
+                } else {
+                    // of two rows the even lane writes one, the odd lane the other
+#pragma unroll
+                    for (int u = 0; u < 32; u += 2) {
+                        const float e = __shfl_xor_sync(0xffffffffu, odd ? v[u] : v[u + 1], 1);
+                        const float re = odd ? e : v[u], im = odd ? v[u + 1] : e;
+                        const int p = n0 + u + odd;
+                        if (writer && p < nrow) {
+                            const int pos = i0 + r0 + p;
+                            const float rs = NEAR ? a.rinv[pos] : 1.f;
+                            a.ws[((size_t)tl.w * a.N + pos) * a.nrhs + col] =
+                                NEAR ? make_float2(re * rs * cs, im * rs * cs)
+                                     : make_float2(-(a.facy * im), a.facy * re);
                         }
                     }
                 }
@@ -664,6 +674,7 @@ __global__ void __launch_bounds__(256, 1)
             tc::tc_fence_before_sync();
             tc::mbar_arrive(&acce[buf]);   // the MMAs may overwrite this accumulator
             ++na;
+        }
         }
     }
     __syncthreads();
@@ -681,36 +692,56 @@ __global__ void __launch_bounds__(256, 1)
     if (warp == 0) tc::tmem_dealloc(tmem, 2 * TC_TMEM_COLS);
 }
 
-// y += (ADD, FP64) or out32 = the sum of the parts ws[part][pos][col], in order, to
-// row perm[pos]; tiles of 32 bases x 32 columns turned in shared memory
-template <bool ADD>
-__global__ void __launch_bounds__(256) k_tc_sum(int N, int nrhs, int ld, int nsplit, const int* __restrict__ perm,
-                                                const float2* __restrict__ ws, double2* __restrict__ y,
-                                                float2* __restrict__ out32) {
-    __shared__ float2 t[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+// (double)f; a normal number by moving its fields, as a conversion instruction
+// takes a slot of the FP64 pipe (one warp instruction in 19 cycles an SM)
+__device__ __forceinline__ double f2d(float f) {
+    const unsigned u = __float_as_uint(f), ex = u >> 23 & 255u;
+    if (ex == 0 || ex == 255) return (double)f;
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
+// Row n of y = the receive's parts + the near field's, or of out32 = the near
+// parts alone: the parts ws[part][pos[n]][col] of each added in order in FP32, as
+// they were accumulated, the two sums in FP64.  Tiles of 32 rows x 32 columns
+// turned in shared memory, so that both sides move whole sectors.  30720 x 64:
+// 70 us with the parts converted and added in FP64 -> 38 us
+template <class T2>
+__global__ void __launch_bounds__(256) k_tc_sum(int N, int nrhs, int ld, const int* __restrict__ pos,
+                                                const unsigned char* __restrict__ npn, const float2* __restrict__ wsn,
+                                                const unsigned char* __restrict__ npr, const float2* __restrict__ wsr,
+                                                T2* __restrict__ out) {
+    constexpr bool Y = sizeof(T2) == sizeof(double2);
+    __shared__ float2 t[Y ? 2 : 1][32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, n0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+#pragma unroll
     for (int r = ty; r < 32; r += 8) {
-        float2 v = make_float2(0.f, 0.f);
-        if (p0 + r < N && c0 + tx < nrhs)
-            for (int q = 0; q < nsplit; ++q) {
-                const float2 w = ws[((size_t)q * N + p0 + r) * nrhs + c0 + tx];
+        if (n0 + r >= N || c0 + tx >= nrhs) continue;
+        const int p = pos[n0 + r];
+        auto sum = [&](int n, const float2* __restrict__ ws) {
+            float2 v = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int q = 0; q < n; ++q) {
+                const float2 w = ws[((size_t)q * N + p) * nrhs + c0 + tx];
                 v.x += w.x;
                 v.y += w.y;
             }
-        t[r][tx] = v;
+            return v;
+        };
+        t[0][r][tx] = sum(npn[p], wsn);
+        if (Y) t[Y][r][tx] = sum(npr[p], wsr);
     }
     __syncthreads();
-    if (p0 + tx >= N) return;
-    const int n = perm[p0 + tx];
+    if (n0 + tx >= N) return;
     for (int c = ty; c < 32 && c0 + c < nrhs; c += 8) {
-        const float2 v = t[tx][c];
-        const size_t o = (size_t)(c0 + c) * ld + n;
-        if (ADD) {
-            const double2 w = y[o];
-            y[o] = make_double2(w.x + (double)v.x, w.y + (double)v.y);
-        } else {
-            out32[o] = v;
+        const float2 v = t[0][tx][c], w = t[Y][tx][c];
+        T2 o;
+        o.x = v.x;
+        o.y = v.y;
+        if constexpr (Y) {
+            o.x = f2d(w.x) + f2d(v.x);
+            o.y = f2d(w.y) + f2d(v.y);
         }
+        out[(size_t)(c0 + c) * ld + n0 + tx] = o;
     }
 }
 
@@ -765,31 +796,98 @@ int make_rows_map(Ctx* c, CUtensorMap* m, const void* base, long long rows, int 
 
 }  // namespace
 
-// tiles in order of decreasing work (chunks), ties in box order: the
-// persistent CTAs take them round-robin, longest first
-static void order_by_work(std::vector<int4>& tiles, std::vector<int>& nch) {
-    std::vector<int> idx(tiles.size());
-    for (size_t k = 0; k < idx.size(); ++k) idx[k] = (int)k;
-    std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return nch[x] > nch[y]; });
-    std::vector<int4> t2(tiles.size());
-    std::vector<int> n2(tiles.size());
-    for (size_t k = 0; k < idx.size(); ++k) {
-        t2[k] = tiles[idx[k]];
-        n2[k] = nch[idx[k]];
+static void tc_slots_free(TcSlots* w) {
+    auto F = [](void* p) { if (p) cudaFree(p); };
+    F(w->ptr); F(w->item); F(w->ch); F(w->np);
+    *w = TcSlots();
+}
+
+// The chunks ch[k] (first, number) of the tiles in equal shares, one per SM,
+// consecutive in tile order; with split a tile whose chunks fall into several
+// shares becomes as many parts (runs of under three chunks join their neighbour).
+// Whole tiles per CTA left SMs idle: 184 tiles of the 30720-RWG spheroid's boxes
+// need two rounds on 152 SMs, 46 tiles of the 7680-RWG one under a third.  A share
+// holds eight chunks or more, a tile about TC_PARTS parts at most.  The FP32
+// accumulations are shorter in parts: 7680 RWG are 6.2e-6
+// from FP64 instead of 1.5e-5.
+// 30720 RWG x 64 columns: near field 167 -> 136 us, receive 80 -> 54, the whole
+// product 708 -> 592 (with k_tc_sum and the aggregation's stores); a mixed solve of
+// 17280 unknowns x 32 columns 104 -> 84 ms.
+static int tc_slots(Ctx* c, TcSlots* w, const std::vector<int4>& tiles, const std::vector<int2>& ch, bool split) {
+    tc_slots_free(w);
+    auto cost = [&](size_t k) { return 128.0 + (tiles[k].z + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX; };   // rows staged a chunk
+    double all = 0, most = 0;
+    long long chunks = 0;
+    for (size_t k = 0; k < tiles.size(); ++k) {
+        all += cost(k) * ch[k].y;
+        most = std::max(most, cost(k) * ch[k].y);
+        chunks += ch[k].y;
     }
-    tiles.swap(t2);
-    nch.swap(n2);
+    int n = c->tc->nsm;
+    if (split) {
+        n = (int)std::min<long long>(n, std::max(1LL, chunks / 8));
+        if (most > 0) n = std::max(1, std::min(n, (int)(all * TC_PARTS / most)));
+    }
+    w->n = n;
+    std::vector<int> ptr(n + 1, 0);
+    std::vector<int4> item;
+    std::vector<int2> run;
+    std::vector<unsigned char> np(std::max(c->N, 1), 0);
+    double before = 0;
+    int s = 0;
+    auto put = [&](size_t k, int part, int a, int e) {
+        item.push_back(make_int4(tiles[k].x, tiles[k].y, tiles[k].z, part));
+        run.push_back(make_int2(ch[k].x + a, e - a));
+        ptr[s + 1]++;
+    };
+    for (size_t k = 0; k < tiles.size(); ++k) {
+        const double ck = cost(k);
+        const int nch = ch[k].y;
+        int part = 0;
+        if (!split) {
+            s = all > 0 ? std::max(s, std::min(n - 1, (int)((before + 0.5 * ck * nch) * n / all))) : 0;
+            put(k, part++, 0, nch);
+        }
+        for (int a = 0; split && a < nch;) {
+            int e = s == n - 1 ? nch : std::min(nch, (int)std::lround((all * (s + 1) / n - before) / ck));
+            if (nch - e <= 2) e = nch;
+            if (e <= a || (e < nch && e - a <= 2)) {
+                ++s;
+                continue;
+            }
+            put(k, part++, a, e);
+            a = e;
+            if (e < nch) ++s;
+        }
+        before += ck * nch;
+        w->parts = std::max(w->parts, part);
+        if (split)
+            for (int r = 0; r < tiles[k].z; ++r) np[c->box_ptr[tiles[k].x] + tiles[k].y + r] = (unsigned char)part;
+    }
+    for (int q = 0; q < n; ++q) ptr[q + 1] += ptr[q];
+    CK(cudaMalloc(&w->ptr, ptr.size() * sizeof(int)));
+    CK(cudaMalloc(&w->item, std::max<size_t>(item.size(), 1) * sizeof(int4)));
+    CK(cudaMalloc(&w->ch, std::max<size_t>(run.size(), 1) * sizeof(int2)));
+    CK(cudaMalloc(&w->np, np.size()));
+    CK(cudaMemcpy(w->ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(w->item, item.data(), item.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(w->ch, run.data(), run.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(w->np, np.data(), np.size(), cudaMemcpyHostToDevice));
+    return MLF_OK;
 }
 
 void tc_free(Ctx* c) {
     TcState* t = c->tc;
     if (!t) return;
     auto F = [](void* p) { if (p) cudaFree(p); };
-    F(t->dtiles); F(t->dzrow); F(t->dcbase); F(t->dchunk); F(t->derr);
+    F(t->dlist); F(t->dpos); F(t->dzrow); F(t->dcbase); F(t->dchunk); F(t->derr);
     F(t->Z.hi); F(t->Z.lo); F(t->Z.rinv); F(t->M.hi); F(t->M.lo); F(t->M.rinv); F(t->xhi); F(t->xlo);
     F(t->dcmax); F(t->dcinv); F(t->drowmax); F(t->RA.rinv);
-    F(t->datiles); F(t->dabase); F(t->drbase); F(t->RA.hi); F(t->RA.lo); F(t->RR.hi); F(t->RR.lo);
-    F(t->dtchunks); F(t->datchunks); F(t->dstiles); F(t->dstchunks); F(t->dsfirst); F(t->dws);
+    F(t->dabase); F(t->drbase); F(t->RA.hi); F(t->RA.lo); F(t->RR.hi); F(t->RR.lo);
+    F(t->dws);
+    tc_slots_free(&t->near);
+    tc_slots_free(&t->recv);
+    tc_slots_free(&t->agg);
     delete t;
     c->tc = nullptr;
 }
@@ -889,89 +987,49 @@ static int tc_setup_build(Ctx* c) {
         c->err = "tensor-core near field: operand layout exceeds 2^31 rows";
         return MLF_E_STATE;
     }
-    std::vector<int> tch(tiles.size(), 0);
-    for (size_t k = 0; k < tiles.size(); ++k)
-        for (int e = c->nbox_ptr[tiles[k].x]; e < c->nbox_ptr[tiles[k].x + 1]; ++e)
-            tch[k] += cbase[c->nbox_list[e] + 1] - cbase[c->nbox_list[e]];
-    order_by_work(tiles, tch);
+    // near chunks of each box in order
+    std::vector<int2> list;
+    std::vector<int> lptr(nb + 1, 0);
+    for (int i = 0; i < nb; ++i) {
+        const int ni = c->box_ptr[i + 1] - c->box_ptr[i];
+        for (int e = c->nbox_ptr[i]; ni > 0 && e < c->nbox_ptr[i + 1]; ++e) {
+            const int j = c->nbox_list[e];
+            for (int k = cbase[j]; k < cbase[j + 1]; ++k) list.push_back(make_int2(k, zrow[e] + (k - cbase[j]) * ni));
+        }
+        lptr[i + 1] = (int)list.size();
+    }
+    std::vector<int2> tch;   // per tile: its first chunk in the list, chunks
+    for (const int4& q : tiles) tch.push_back(make_int2(lptr[q.x], lptr[q.x + 1] - lptr[q.x]));
     int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->dev));
     TcState* t = new TcState();
     t->nsm = std::max(nsm, 1);
     c->tc = t;
-    t->ntiles = (int)tiles.size();
+    t->tiles = tiles;
     for (const int4& q : tiles) t->maxrows = std::max(t->maxrows, q.z);
-    // parts of the near lists, whole near boxes each and about equal in chunks, so
-    // that the items of one column tile come to about four and a half per SM (184
-    // tiles of the 30720-RWG spheroid's boxes left most of the second round idle, 46
-    // tiles of the 7680-RWG one most of the SMs).  The 30720-RWG product with 64
-    // columns: 708 -> 636 us; a solve of 17280 unknowns x 32 columns: 104 -> 90 ms.
-    // The shorter FP32 accumulations are more accurate too: 1.5e-5 -> 2.3e-6 from
-    // FP64 at 7680.  Past eight parts their sums cost what they gain
-    t->nsplit = tiles.empty() ? 1 : std::max(1, std::min(TC_MAX_SPLIT, (9 * t->nsm / 2) / (int)tiles.size()));
-    std::vector<int4> stiles;
-    std::vector<int> stch, sfirst;
-    for (const int4& q : tiles) {
-        const int e1 = c->nbox_ptr[q.x + 1];
-        int e = c->nbox_ptr[q.x], total = 0;
-        for (int k = e; k < e1; ++k) total += cbase[c->nbox_list[k] + 1] - cbase[c->nbox_list[k]];
-        for (int part = 0, done = 0; part < t->nsplit; ++part) {   // every part, so that its sums are written
-            const int goal = (int)((long long)total * (part + 1) / t->nsplit);
-            stiles.push_back(make_int4(q.x, q.y, q.z, part));
-            sfirst.push_back(e);
-            int ch = 0;
-            while (e < e1 && (part + 1 == t->nsplit || done + ch < goal)) {
-                ch += cbase[c->nbox_list[e] + 1] - cbase[c->nbox_list[e]];
-                ++e;
-            }
-            done += ch;
-            stch.push_back(ch);
-        }
-    }
-    {
-        std::vector<int> idx(stiles.size());
-        for (size_t k = 0; k < idx.size(); ++k) idx[k] = (int)k;
-        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return stch[x] > stch[y]; });
-        std::vector<int4> t2;
-        std::vector<int> n2, f2;
-        for (int k : idx) {
-            t2.push_back(stiles[k]);
-            n2.push_back(stch[k]);
-            f2.push_back(sfirst[k]);
-        }
-        stiles.swap(t2);
-        stch.swap(n2);
-        sfirst.swap(f2);
-    }
-    t->nstiles = (int)stiles.size();
-    CK(cudaMalloc(&t->dstiles, std::max<size_t>(stiles.size(), 1) * sizeof(int4)));
-    CK(cudaMalloc(&t->dstchunks, std::max<size_t>(stch.size(), 1) * sizeof(int)));
-    CK(cudaMalloc(&t->dsfirst, std::max<size_t>(sfirst.size(), 1) * sizeof(int)));
-    CK(cudaMemcpy(t->dstiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t->dstchunks, stch.data(), stch.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t->dsfirst, sfirst.data(), sfirst.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if ((st = tc_slots(c, &t->near, tiles, tch, true))) return st;
+    std::vector<int> pos(std::max(c->N, 1), 0);
+    for (int p = 0; p < c->N; ++p) pos[c->box_bases[p]] = p;
+    CK(cudaMalloc(&t->dpos, pos.size() * sizeof(int)));
+    CK(cudaMemcpy(t->dpos, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMalloc(&t->dlist, std::max<size_t>(list.size(), 1) * sizeof(int2)));
+    CK(cudaMemcpy(t->dlist, list.data(), list.size() * sizeof(int2), cudaMemcpyHostToDevice));
     t->nchunk = (int)chunk.size();
     t->zrows = rows;
-    CK(cudaMalloc(&t->dtiles, std::max<size_t>(tiles.size(), 1) * sizeof(int4)));
-    CK(cudaMalloc(&t->dtchunks, std::max<size_t>(tch.size(), 1) * sizeof(int)));
     CK(cudaMalloc(&t->dzrow, zrow.size() * sizeof(int)));
     CK(cudaMalloc(&t->dcbase, cbase.size() * sizeof(int)));
     CK(cudaMalloc(&t->dchunk, std::max<size_t>(chunk.size(), 1) * sizeof(int2)));
     CK(cudaMalloc(&t->derr, sizeof(int)));
     CK(cudaMalloc(&t->drowmax, std::max(c->N, 1) * sizeof(unsigned)));
-    CK(cudaMemcpy(t->dtiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t->dtchunks, tch.data(), tch.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(t->dzrow, zrow.data(), zrow.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(t->dcbase, cbase.data(), cbase.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(t->dchunk, chunk.data(), chunk.size() * sizeof(int2), cudaMemcpyHostToDevice));
     CK(cudaMemset(t->derr, 0, sizeof(int)));
     if ((st = tc_near_operand(c, c->dZblk, &t->Z, c->stream))) return st;
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_ADD, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_SET, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
     CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
     CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_ADD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR_SET, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
+    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
     CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
     CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
     CK(cudaStreamSynchronize(c->stream));
@@ -984,7 +1042,7 @@ static int tc_x_buffers(Ctx* c, int nrhs) {
     const int nct = (nrhs + TC_COLS - 1) / TC_COLS;
     const long long rows = (long long)nct * t->nchunk * 128;
     // whole column tiles, as the operand: a block that fits the one fits the other
-    const size_t parts = t->nsplit > 1 ? (size_t)t->nsplit * c->N * nct * TC_COLS : 0;
+    const size_t parts = (size_t)(t->near.parts + t->recv.parts) * c->N * nct * TC_COLS;
     if (parts > t->ws_cap) {
         if (t->dws) cudaFree(t->dws);
         t->dws = nullptr;
@@ -1028,65 +1086,48 @@ static int tc_pack_x(Ctx* c, const float2* xs, int nrhs, cudaStream_t s) {
 static TcArgs tc_args(const Ctx* c, int nrhs) {
     const TcState* t = c->tc;
     TcArgs a{};
-    a.tiles = t->dtiles;
-    a.tchunks = t->dtchunks;
-    a.ntiles = t->ntiles;
     a.nct = (nrhs + TC_COLS - 1) / TC_COLS;
     a.box_ptr = c->dbox_ptr;
-    a.nbox_ptr = c->dnbox_ptr;
-    a.nbox_list = c->dnbox_list;
-    a.zrow = t->dzrow;
+    a.list = t->dlist;
     a.cbase = t->dcbase;
     a.nchunk = t->nchunk;
     a.nrhs = nrhs;
-    a.perm = c->dperm;
     a.cinv = t->dcinv;
     a.N = c->N;
+    a.ws = t->dws;
     a.err = t->derr;
     return a;
 }
 
-// the near field's or preconditioner's items: the tiles in parts
-static void tc_near_args(const Ctx* c, TcArgs& a) {
-    const TcState* t = c->tc;
-    a.tiles = t->dstiles;
-    a.tchunks = t->dstchunks;
-    a.first = t->dsfirst;
-    a.ntiles = t->nstiles;
-    a.ws = t->nsplit > 1 ? t->dws : nullptr;
-}
-
-// persistent grid: one CTA per SM, at most one per work item
-static unsigned tc_grid(const TcState* t, const TcArgs& a) {
-    return (unsigned)std::max(1, std::min(t->nsm, a.ntiles * a.nct));
-}
-
+// persistent grid: one CTA per SM, at most one per share and column tile
 template <int MODE>
-static void tc_launch(const TcState* t, int rows, const CUtensorMap& bhi, const CUtensorMap& blo, const CUtensorMap& xhi,
-                      const CUtensorMap& xlo, const TcArgs& a, cudaStream_t s) {
+static void tc_launch(const TcState* t, const TcSlots& w, int rows, const CUtensorMap& bhi, const CUtensorMap& blo,
+                      const CUtensorMap& xhi, const CUtensorMap& xlo, TcArgs a, cudaStream_t s) {
+    a.nslots = w.n;
+    a.slot = w.ptr;
+    a.item = w.item;
+    a.ch = w.ch;
+    const unsigned grid = (unsigned)std::max(1, std::min(t->nsm, w.n * a.nct));
     if (rows <= TcRing<4>::ROWS)
-        k_tc_gemm<MODE, 4><<<tc_grid(t, a), 256, TcRing<4>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
+        k_tc_gemm<MODE, 4><<<grid, TC_THREADS<MODE>, TcRing<4>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
     else
-        k_tc_gemm<MODE, 3><<<tc_grid(t, a), 256, TcRing<3>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
+        k_tc_gemm<MODE, 3><<<grid, TC_THREADS<MODE>, TcRing<3>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
 }
 
-// y(:, 0:nrhs) += Z_near xs on the tensor cores (engine 4); x_packed: the X
-// operand already holds xs (packed by the aggregation of the same product)
-int device_near_tc(Ctx* c, const float2* xs, int ld, int nrhs, double2* y, cudaStream_t s, bool x_packed) {
-    int st;
-    if ((st = tc_setup(c))) return st;
-    if ((st = tc_x_buffers(c, nrhs))) return st;
+static dim3 tc_sum_grid(const Ctx* c, int nrhs) { return dim3((c->N + 31) / 32, (nrhs + 31) / 32); }
+
+// the receive's parts follow the near field's
+static float2* tc_recv_ws(const Ctx* c, int nrhs) { return c->tc->dws + (size_t)c->tc->near.parts * c->N * nrhs; }
+
+// y(:, 0:nrhs) = Z_near xs + the receive of the same product on the tensor cores
+// (engine 4); the X operand holds xs, packed by the product's aggregation
+int device_near_tc(Ctx* c, int ld, int nrhs, double2* y, cudaStream_t s) {
     TcState* t = c->tc;
-    if (!x_packed && (st = tc_pack_x(c, xs, nrhs, s))) return st;
     TcArgs a = tc_args(c, nrhs);
-    a.ld = ld;
-    a.y = y;
     a.rinv = t->Z.rinv;
-    tc_near_args(c, a);
-    tc_launch<TCM_NEAR_ADD>(t, t->maxrows, t->Z.mhi, t->Z.mlo, t->mxhi, t->mxlo, a, s);
-    if (a.ws)
-        k_tc_sum<true><<<dim3((c->N + 31) / 32, (nrhs + 31) / 32), 256, 0, s>>>(c->N, nrhs, ld, t->nsplit, c->dperm, a.ws,
-                                                                                y, nullptr);
+    tc_launch<TCM_NEAR>(t, t->near, t->maxrows, t->Z.mhi, t->Z.mlo, t->mxhi, t->mxlo, a, s);
+    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, ld, t->dpos, t->near.np, t->dws, t->recv.np,
+                                                  tc_recv_ws(c, nrhs), y);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near field") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -1101,14 +1142,11 @@ int device_near_pattern_tc(Ctx* c, const float2* Mblk, const float2* xs, int nrh
     if (!t->M.hi && (st = tc_near_operand(c, Mblk, &t->M, s))) return st;
     if ((st = tc_pack_x(c, xs, nrhs, s))) return st;
     TcArgs a = tc_args(c, nrhs);
-    a.ld = c->N;
-    a.out32 = out;
     a.rinv = t->M.rinv;
-    tc_near_args(c, a);
-    tc_launch<TCM_NEAR_SET>(t, t->maxrows, t->M.mhi, t->M.mlo, t->mxhi, t->mxlo, a, s);
-    if (a.ws)
-        k_tc_sum<false><<<dim3((c->N + 31) / 32, (nrhs + 31) / 32), 256, 0, s>>>(c->N, nrhs, c->N, t->nsplit, c->dperm,
-                                                                                 a.ws, nullptr, out);
+    tc_launch<TCM_NEAR>(t, t->near, t->maxrows, t->M.mhi, t->M.mlo, t->mxhi, t->mxlo, a, s);
+    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, c->N, t->dpos, t->near.np, t->dws,
+                                                  static_cast<const unsigned char*>(nullptr),
+                                                  static_cast<const float2*>(nullptr), out);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near-pattern preconditioner") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -1125,9 +1163,9 @@ static int tc_leaf_setup(Ctx* c, const float2* R, int K2) {
     TcState* t = c->tc;
     if (t->RA.hi && t->Rsrc == R && t->K2 == K2) return MLF_OK;
     auto F = [](void* p) { if (p) cudaFree(p); };
-    F(t->datiles); F(t->datchunks); F(t->dabase); F(t->drbase);
+    F(t->dabase); F(t->drbase);
     F(t->RA.hi); F(t->RA.lo); F(t->RA.rinv); F(t->RR.hi); F(t->RR.lo);
-    t->datiles = nullptr; t->datchunks = nullptr; t->dabase = t->drbase = nullptr;
+    t->dabase = t->drbase = nullptr;
     t->RA.hi = t->RA.lo = t->RR.hi = t->RR.lo = nullptr;
     t->RA.rinv = nullptr;
     t->Rsrc = nullptr;
@@ -1136,7 +1174,7 @@ static int tc_leaf_setup(Ctx* c, const float2* R, int K2) {
     const int nt = (K2 + TC_ROWS - 1) / TC_ROWS;
     const int per = ((K2 + nt - 1) / nt + 15) / 16 * 16;   // directions per tile, multiple of 16, <= 160
     std::vector<int4> tiles;
-    std::vector<int> tch;
+    std::vector<int2> tch;
     std::vector<int> abase(nb + 1, 0), rbase(nb + 1, 0);
     long long arows = 0, rrows = 0;
     for (int b = 0; b < nb; ++b) {
@@ -1157,20 +1195,16 @@ static int tc_leaf_setup(Ctx* c, const float2* R, int K2) {
                 return MLF_E_STATE;
             }
             tiles.push_back(make_int4(b, r0, nrow, 0));
-            tch.push_back(nkc);
+            tch.push_back(make_int2(0, nkc));
         }
     }
-    order_by_work(tiles, tch);
     abase[nb] = (int)arows;
     rbase[nb] = (int)rrows;
-    t->natiles = (int)tiles.size();
     t->arows = std::min(per, K2);
-    CK(cudaMalloc(&t->datiles, std::max<size_t>(tiles.size(), 1) * sizeof(int4)));
-    CK(cudaMalloc(&t->datchunks, std::max<size_t>(tch.size(), 1) * sizeof(int)));
+    if ((st = tc_slots(c, &t->agg, tiles, tch, false))) return st;
+    if ((st = tc_slots(c, &t->recv, t->tiles, std::vector<int2>(t->tiles.size(), make_int2(0, nqc)), true))) return st;
     CK(cudaMalloc(&t->dabase, abase.size() * sizeof(int)));
     CK(cudaMalloc(&t->drbase, rbase.size() * sizeof(int)));
-    CK(cudaMemcpy(t->datiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t->datchunks, tch.data(), tch.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(t->dabase, abase.data(), abase.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(t->drbase, rbase.data(), rbase.size() * sizeof(int), cudaMemcpyHostToDevice));
     const size_t ab = (size_t)std::max<long long>(arows, 1) * 128, rb = (size_t)std::max<long long>(rrows, 1) * 128;
@@ -1205,21 +1239,18 @@ int device_agg_tc(Ctx* c, const float2* R, int K, const float2* xs, int nrhs, fl
     TcState* t = c->tc;
     if ((st = tc_pack_x(c, xs, nrhs, s))) return st;
     TcArgs a = tc_args(c, nrhs);
-    a.tiles = t->datiles;
-    a.tchunks = t->datchunks;
-    a.ntiles = t->natiles;
     a.zrow = t->dabase;
     a.K2 = 2 * K;
     a.C = C;
     a.rinv = t->RA.rinv;
-    tc_launch<TCM_AGG>(t, t->arows, t->RA.mhi, t->RA.mlo, t->mxhi, t->mxlo, a, s);
+    tc_launch<TCM_AGG>(t, t->agg, t->arows, t->RA.mhi, t->RA.mlo, t->mxhi, t->mxlo, a, s);
     return cuda_ok(c, cudaGetLastError(), "tensor-core aggregation") ? MLF_OK : MLF_E_CUDA;
 }
 
-// y = j facy conj(R) A per leaf box (written, not added) on the tensor cores;
-// A the leaf fields [box][column][2K], staged raw by TMA and expanded in the CTA
-int device_recv_tc(Ctx* c, const float2* R, int K, const float2* A, float facy, int nrhs, int ld, double2* y,
-                   cudaStream_t s) {
+// j facy conj(R) A per leaf box on the tensor cores, left as parts for
+// device_near_tc; A the leaf fields [box][column][2K], staged raw by TMA and
+// expanded in the CTA
+int device_recv_tc(Ctx* c, const float2* R, int K, const float2* A, float facy, int nrhs, cudaStream_t s) {
     int st;
     const int K2 = 2 * K;
     if ((st = tc_leaf_setup(c, R, K2))) return st;
@@ -1233,9 +1264,8 @@ int device_recv_tc(Ctx* c, const float2* R, int K, const float2* A, float facy, 
     a.zrow = t->drbase;
     a.K2 = K2;
     a.facy = facy;
-    a.ld = ld;
-    a.y = y;
-    tc_launch<TCM_RECV>(t, t->maxrows, t->RR.mhi, t->RR.mlo, raw, raw, a, s);
+    a.ws = tc_recv_ws(c, nrhs);
+    tc_launch<TCM_RECV>(t, t->recv, t->maxrows, t->RR.mhi, t->RR.mlo, raw, raw, a, s);
     return cuda_ok(c, cudaGetLastError(), "tensor-core receive") ? MLF_OK : MLF_E_CUDA;
 }
 

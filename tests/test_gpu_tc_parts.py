@@ -1,8 +1,9 @@
-"""The tcgen05 engine with its near lists cut into parts, in rings of three and
-four stages, against the FP64 operator.
+"""The tcgen05 engine, its tiles cut into parts by equal shares of the chunks, in
+rings of three and four stages, against the FP64 operator.
 
-Bodies: about 46 tiles of 145 rows (eight parts, three stages), 184 tiles of 42
-rows (three parts, four stages) and 736 tiles of 42 rows (uncut, four stages).
+Bodies: about 46 tiles of 145 rows (four or five parts each, three stages), 184
+tiles of 42 rows (one or two parts, four stages) and 736 tiles of 42 rows (most
+in one part, four stages).
 Columns: the fewest, one over half a column tile, one over a whole one, and back
 to few in the workspaces of the larger block.
 
