@@ -332,6 +332,9 @@ int device_setup(Ctx* c) {
     for (int b = 0; b < leaf.nb; ++b)
         for (int j = c->box_ptr[b]; j < c->box_ptr[b + 1]; ++j) box_of_sorted[j] = b;
     if ((st = upload(c, &c->dperm, c->box_bases))) return st;
+    std::vector<int> pos(N);
+    for (int j = 0; j < N; ++j) pos[c->box_bases[j]] = j;
+    if ((st = upload(c, &c->dpos, pos))) return st;
     if ((st = upload(c, &c->dbox_ptr, c->box_ptr))) return st;
     if ((st = upload(c, &c->dbox_of_sorted, box_of_sorted))) return st;
     if ((st = upload(c, &c->dia, c->ia))) return st;
@@ -589,7 +592,7 @@ void device_free(Ctx* c) {
         F(L.dsth); F(L.dsph); F(L.dwth); F(L.dwph); F(L.dthT_ptr); F(L.dthT_row); F(L.dthT_w); F(L.dphT_ptr);
         F(L.dphT_row); F(L.dphT_w);
     }
-    F(c->dR); F(c->dperm); F(c->dbox_ptr); F(c->dbox_of_sorted); F(c->dia); F(c->dja); F(c->dZ);
+    F(c->dR); F(c->dperm); F(c->dpos); F(c->dbox_ptr); F(c->dbox_of_sorted); F(c->dia); F(c->dja); F(c->dZ);
     F(c->dp_coord); F(c->dt_baric); F(c->dt_baric_sub); F(c->de_long); F(c->de_centro); F(c->de_t);
     F(c->de_po); F(c->dalu); F(c->djlu); F(c->dju); F(c->dlvl_rows_f); F(c->dlvl_rows_b);
     F(c->dalu64); F(c->doz_tiles); F(c->doz_pat); F(c->doz_exp); F(c->doz_ws); F(c->drcs_edge); F(c->drcs_ws);

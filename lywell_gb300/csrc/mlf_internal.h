@@ -165,7 +165,8 @@ struct Ctx {
     std::vector<int> ia, ja;          // 0-based CSR
     // device: leaf
     double2* dR = nullptr;            // patterns, box order
-    int *dperm = nullptr, *dbox_ptr = nullptr, *dbox_of_sorted = nullptr;
+    int *dperm = nullptr, *dpos = nullptr;   // basis at each box-sorted position, and back
+    int *dbox_ptr = nullptr, *dbox_of_sorted = nullptr;
     int *dia = nullptr, *dja = nullptr;
     float2* dZ = nullptr;
     double2* dZd = nullptr;           // the same near values as complex(8)

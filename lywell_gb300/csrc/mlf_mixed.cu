@@ -25,6 +25,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "mlf_cvt.cuh"
 #include "mlf_internal.h"
 #include "mlf_sep.cuh"
 
@@ -55,7 +56,7 @@ __device__ __forceinline__ void bstore(__half2* p, float2 v, float s) { *p = __f
 
 __global__ void k32_from64(size_t n, const double2* __restrict__ a, float2* __restrict__ b) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        b[i] = make_float2((float)a[i].x, (float)a[i].y);
+        b[i] = make_float2(d2f(a[i].x), d2f(a[i].y));
 }
 
 // x (FP64, ld) -> packed FP32 columns
@@ -64,7 +65,7 @@ __global__ void k32_pack_x(int N, int nrhs, int ld, const double2* __restrict__ 
     const int r = blockIdx.y;
     if (i < N) {
         const double2 v = x[(size_t)r * ld + i];
-        xf[(size_t)r * N + i] = make_float2((float)v.x, (float)v.y);
+        xf[(size_t)r * N + i] = make_float2(d2f(v.x), d2f(v.y));
     }
 }
 
@@ -324,7 +325,7 @@ __global__ void k32_receive_near(int K, int N, int nrhs, int ld, const int* __re
         tr += __shfl_xor_sync(0xffffffff, tr, o);
         ti += __shfl_xor_sync(0xffffffff, ti, o);
     }
-    if (lane == 0) y[(size_t)r * ld + n] = make_double2((double)tr, (double)ti);
+    if (lane == 0) y[(size_t)r * ld + n] = make_double2(f2d(tr), f2d(ti));
 }
 
 // ---------------------------------------------------------------------------
@@ -882,11 +883,11 @@ __global__ void k_combine32(int N, int nrhs, int nvec, const BT* __restrict__ V,
 
 __global__ void k_d2f_m(size_t n, const double2* __restrict__ a, float2* __restrict__ b) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        b[i] = make_float2((float)a[i].x, (float)a[i].y);
+        b[i] = make_float2(d2f(a[i].x), d2f(a[i].y));
 }
 __global__ void k_f2d_m(size_t n, const float2* __restrict__ a, double2* __restrict__ b) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        b[i] = make_double2((double)a[i].x, (double)a[i].y);
+        b[i] = make_double2(f2d(a[i].x), f2d(a[i].y));
 }
 
 namespace {

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "mlf_cvt.cuh"
 #include "mlf_internal.h"
 
 namespace mlf {
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256) k32_near_warp(int N, int nrhs, int ld, in
         ti = fmaf(facy, sr, ti);
     }
     if (g == 0 && live) {
-        if (OUT == 0) y[(size_t)(c0 + r) * ld + n] = make_double2((double)tr, (double)ti);
+        if (OUT == 0) y[(size_t)(c0 + r) * ld + n] = make_double2(f2d(tr), f2d(ti));
         else out32[(size_t)(c0 + r) * ld + n] = make_float2(tr, ti);
     }
 }
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(128) k32_nearrecv_box(int nrhs, int ld, int K2
         recv_row<NR>(R + (size_t)pos * K2, As, K2, lane, r, nrhs - c0, sr, si);
         tr = fmaf(-facy, si, tr);
         ti = fmaf(facy, sr, ti);
-        if (g == 0 && live) y[(size_t)(c0 + r) * ld + n] = make_double2((double)tr, (double)ti);
+        if (g == 0 && live) y[(size_t)(c0 + r) * ld + n] = make_double2(f2d(tr), f2d(ti));
     }
 }
 

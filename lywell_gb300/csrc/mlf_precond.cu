@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "mlf_cvt.cuh"
 #include "mlf_internal.h"
 
 namespace mlf {
@@ -273,7 +274,7 @@ __global__ void k32_spmv_z(int N, int nrhs, const int* __restrict__ ia, const in
 
 __global__ void k_d2f(size_t n, const double2* __restrict__ a, float2* __restrict__ b) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        b[i] = make_float2((float)a[i].x, (float)a[i].y);
+        b[i] = make_float2(d2f(a[i].x), d2f(a[i].y));
 }
 
 int device_nearinv_apply32(Ctx* c, const float2* y, float2* x, int nrhs, cudaStream_t s) {

@@ -58,6 +58,7 @@
 #include <mutex>
 #include <vector>
 
+#include "mlf_cvt.cuh"
 #include "mlf_internal.h"
 #include "mlf_tcgen05.h"
 
@@ -117,7 +118,6 @@ struct TcState {
     float2* dws = nullptr;          // parts' sums [part][box-sorted basis][column], the near field's, then the receive's
     size_t ws_cap = 0;
     int* dzrow = nullptr;           // per block entry e: first Z-operand row (chunk 0)
-    int* dpos = nullptr;            // box-sorted position of each basis
     int* dcbase = nullptr;          // per box: its first chunk
     int2* dchunk = nullptr;         // per chunk: (first box-sorted position, bases in it)
     int* derr = nullptr;            // set by a CTA whose wait gave up
@@ -692,19 +692,11 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
     if (warp == 0) tc::tmem_dealloc(tmem, 2 * TC_TMEM_COLS);
 }
 
-// (double)f; a normal number by moving its fields, as a conversion instruction
-// takes a slot of the FP64 pipe (one warp instruction in 19 cycles an SM)
-__device__ __forceinline__ double f2d(float f) {
-    const unsigned u = __float_as_uint(f), ex = u >> 23 & 255u;
-    if (ex == 0 || ex == 255) return (double)f;
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
-}
-
 // Row n of y = the receive's parts + the near field's, or of out32 = the near
 // parts alone: the parts ws[part][pos[n]][col] of each added in order in FP32, as
 // they were accumulated, the two sums in FP64.  Tiles of 32 rows x 32 columns
 // turned in shared memory, so that both sides move whole sectors.  30720 x 64:
-// 70 us with the parts converted and added in FP64 -> 38 us
+// 70 us with the parts converted and added in FP64 -> 29 us
 template <class T2>
 __global__ void __launch_bounds__(256) k_tc_sum(int N, int nrhs, int ld, const int* __restrict__ pos,
                                                 const unsigned char* __restrict__ npn, const float2* __restrict__ wsn,
@@ -880,7 +872,7 @@ void tc_free(Ctx* c) {
     TcState* t = c->tc;
     if (!t) return;
     auto F = [](void* p) { if (p) cudaFree(p); };
-    F(t->dlist); F(t->dpos); F(t->dzrow); F(t->dcbase); F(t->dchunk); F(t->derr);
+    F(t->dlist); F(t->dzrow); F(t->dcbase); F(t->dchunk); F(t->derr);
     F(t->Z.hi); F(t->Z.lo); F(t->Z.rinv); F(t->M.hi); F(t->M.lo); F(t->M.rinv); F(t->xhi); F(t->xlo);
     F(t->dcmax); F(t->dcinv); F(t->drowmax); F(t->RA.rinv);
     F(t->dabase); F(t->drbase); F(t->RA.hi); F(t->RA.lo); F(t->RR.hi); F(t->RR.lo);
@@ -1008,10 +1000,6 @@ static int tc_setup_build(Ctx* c) {
     t->tiles = tiles;
     for (const int4& q : tiles) t->maxrows = std::max(t->maxrows, q.z);
     if ((st = tc_slots(c, &t->near, tiles, tch, true))) return st;
-    std::vector<int> pos(std::max(c->N, 1), 0);
-    for (int p = 0; p < c->N; ++p) pos[c->box_bases[p]] = p;
-    CK(cudaMalloc(&t->dpos, pos.size() * sizeof(int)));
-    CK(cudaMemcpy(t->dpos, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&t->dlist, std::max<size_t>(list.size(), 1) * sizeof(int2)));
     CK(cudaMemcpy(t->dlist, list.data(), list.size() * sizeof(int2), cudaMemcpyHostToDevice));
     t->nchunk = (int)chunk.size();
@@ -1126,7 +1114,7 @@ int device_near_tc(Ctx* c, int ld, int nrhs, double2* y, cudaStream_t s) {
     TcArgs a = tc_args(c, nrhs);
     a.rinv = t->Z.rinv;
     tc_launch<TCM_NEAR>(t, t->near, t->maxrows, t->Z.mhi, t->Z.mlo, t->mxhi, t->mxlo, a, s);
-    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, ld, t->dpos, t->near.np, t->dws, t->recv.np,
+    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, ld, c->dpos, t->near.np, t->dws, t->recv.np,
                                                   tc_recv_ws(c, nrhs), y);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near field") ? MLF_OK : MLF_E_CUDA;
 }
@@ -1144,7 +1132,7 @@ int device_near_pattern_tc(Ctx* c, const float2* Mblk, const float2* xs, int nrh
     TcArgs a = tc_args(c, nrhs);
     a.rinv = t->M.rinv;
     tc_launch<TCM_NEAR>(t, t->near, t->maxrows, t->M.mhi, t->M.mlo, t->mxhi, t->mxlo, a, s);
-    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, c->N, t->dpos, t->near.np, t->dws,
+    k_tc_sum<<<tc_sum_grid(c, nrhs), 256, 0, s>>>(c->N, nrhs, c->N, c->dpos, t->near.np, t->dws,
                                                   static_cast<const unsigned char*>(nullptr),
                                                   static_cast<const float2*>(nullptr), out);
     return cuda_ok(c, cudaGetLastError(), "tensor-core near-pattern preconditioner") ? MLF_OK : MLF_E_CUDA;

@@ -45,3 +45,22 @@ def test_parts_and_rings(gpu_lib, level, axis):
         assert out["status"][k] == "converged"
         assert np.linalg.norm(m.matvec(out["x"][:, k]) - B[:, k]) / np.linalg.norm(B[:, k]) < 1e-3
     m.close()
+
+
+@pytest.mark.parametrize("cut,nrhs", [(1, 2), (7, 31), (30, 33), (5, 17)])
+def test_ragged_blocks(gpu_lib, cut, nrhs):
+    """An open body whose unknowns fill no tile of 32 rows: the block's copy to box
+    order and the sums back, all engines.  A misplaced row is an error of order one;
+    the FP32 operator is 2e-5 from FP64, the bound five times that."""
+    tris = meshes.icosphere(3, 1.0)[:-cut]
+    m = MLFMA(RWG(tris), lam=1.0, ladomax=0.25)
+    assert m.N % 32
+    rng = np.random.default_rng(cut)
+    X = rng.standard_normal((m.N, nrhs)) + 1j * rng.standard_normal((m.N, nrhs))
+    X[3, 0] = 0.0
+    Y = np.stack([m.matvec(X[:, k].copy()) for k in range(nrhs)], 1)
+    for engine in (0, 1, 3, 4, -1):
+        m.set_block_engine(engine)
+        Y32 = m.matvec32(X)
+        assert max(_rel(Y32[:, k], Y[:, k]) for k in range(nrhs)) < 1e-4
+    m.close()
