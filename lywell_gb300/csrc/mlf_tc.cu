@@ -3,47 +3,51 @@
 // (and the near-pattern preconditioner), as tcgen05.mma with TMEM
 // accumulators, operands staged into shared memory by TMA
 // (cp.async.bulk.tensor) through tensor maps over this GPU's own memory,
-// 3xTF32 for FP32 accuracy.
+// hi and lo parts of each factor for FP32 accuracy.
 //
 // The near matrix (llenarZesparcida, modMLFMA.f90:1594-1634) is a union of
 // dense box-pair blocks Z_ij (bases of leaf box i x bases of near box j).  For
 // a block of right-hand sides, leaf box i needs Y_i = sum_j Z_ij X_j.  Here it
-// is computed transposed, as a real GEMM whose M side is the right-hand sides:
-//   D (2 nrhs x n_i) = A (2 nrhs x 2 n_j) * B^T,   B = [Zr Zi] interleaved
-// with the complex product written as a real one on the contraction side:
+// is computed transposed, as a real GEMM whose M side is the right-hand sides
+// (A the right-hand sides, B the box's rows, both with the contraction along rows).
+// Near field and aggregation (FP16 operands) take two real products per tile,
+//   A row 2c = Xr(:, c), row 2c+1 = Xi(:, c);   B row p = [ Zr(p, :) | Zi(p, :) ]
+//   D1 = A Zr^T, D2 = A Zi^T;   Re Y = D1(2c) - D2(2c+1), Im Y = D1(2c+1) + D2(2c)
+// combined in the epilogue; the receive (TF32 operands) one on twice the length,
 //   A row 2c   = [ Xr(t,c), -Xi(t,c) ]_t   -> D row 2c   = Re Y(:, c)
 //   A row 2c+1 = [ Xi(t,c),  Xr(t,c) ]_t   -> D row 2c+1 = Im Y(:, c)
-//   B row p    = [ Zr(p,t),  Zi(p,t) ]_t   (the complex(4) row of Z, as stored)
-// so that M = 128 covers 64 right-hand sides exactly and N = the box's bases
+//   B row p    = [ Zr(p,t),  Zi(p,t) ]_t
+// The first form reads half the A bytes and accumulates over half the length
+// (7680 RWG: 3.7e-6 from FP64 instead of 6.2e-6); its pair of accumulators fits
+// TMEM twice only up to 128 rows.  Either way M = 128 covers 64 right-hand sides
+// exactly and N = the box's bases
 // (padded to 16), with no padding of the rows to 128.  The leaf aggregation
 // (llenar_campoCyB, modMLFMA.f90:1805-1811: C_b = R_b^T x_b) and receive
 // (MatxVec_MLFMA, modMLFMA.f90:1915-1924: y_b = j facy conj(R_b) A_b) are the
 // same GEMM with the patterns R in place of Z.
 //
 // Layouts in HBM (built once per context; the X operand once per call):
-//   Z operand: per block e = (i, j) and chunk kc of 16 columns t, the n_i
-//     rows p of 32 floats [re, im] x 16 (zero past n_j), rows of all blocks
-//     and chunks stacked: one 2-D tensor map [rows][32 floats], boxes of 32
-//     rows; split into TF32 hi and lo copies.
-//   X operand: per column tile of 64 right-hand sides, per box j and chunk kc,
-//     128 rows of 32 floats as above, hi and lo; one tensor map, boxes of 128
-//     rows.
-//   Aggregation / receive operands: R^T and conj R in the same row format
-//     (tc_leaf_setup); the receive's right-hand side operand is the leaf A
-//     field itself, read raw.
-// Each TMA box of an operand is written with 128-byte swizzling, which is the
-// canonical K-major SWIZZLE_128B layout tcgen05.mma reads (8-row atoms of
-// 1024 bytes).
+//   Z operand: per block e = (i, j) and chunk kc of 32 columns t, the n_i rows p
+//     of [32 re | 32 im] (zero past n_j) in scaled FP16, rows of all blocks and
+//     chunks stacked: one 2-D tensor map of 128-byte rows, boxes of 32 rows; hi
+//     and lo copies.
+//   X operand: per column tile of 64 right-hand sides, per box j and chunk kc, 128
+//     rows of 32 FP16, hi and lo; a tensor map of 64-byte rows, boxes of 128 rows.
+//   Aggregation / receive operands: R^T as the Z operand, conj R as rows of 16
+//     (re, im) pairs in TF32 (tc_leaf_setup); the receive's right-hand side
+//     operand is the leaf A field itself, read raw.
+// Each TMA box of an operand is written with 128-byte (X: 64-byte) swizzling, the
+// canonical K-major SWIZZLE_128B / 64B layouts tcgen05.mma reads (8-row atoms of
+// 1024 / 512 bytes).
 //
 // A persistent CTA (8 warps, the receive's 10) per SM walks its share of the work
 // (tiles of at most 160 rows, 64 columns, cut into parts where shares meet, the
-// parts' sums added by k_tc_sum).  Thread 0 issues the TMA loads of a 3- or 4-stage ring; thread
-// 32 issues the MMAs: per chunk of 32 real K, 4 K-steps x 3 products (A_lo
-// B_hi, A_hi B_lo, A_hi B_hi) into a 128 x N FP32 accumulator in TMEM, and
+// parts' sums added by k_tc_sum).  Thread 0 issues the TMA loads of a ring of
+// three to five stages; thread 32 issues the MMAs: per chunk 4 K-steps x 3 products
+// (A_lo B_hi, A_hi B_lo, A_hi B_hi) into 128 x N FP32 accumulators in TMEM, and
 // tcgen05.commit frees a stage once its MMAs are done.  Warps 4-7 read their
-// 32 TMEM lanes each (tcgen05.ld), pair the real and imaginary rows with one
-// shuffle and write the output, while the next item accumulates into the
-// other of two TMEM accumulators.
+// 32 TMEM lanes each (tcgen05.ld), pair the real and imaginary rows by shuffles and
+// write the output, while the next item accumulates into the other TMEM buffer.
 //
 // Every wait on an mbarrier is bounded; on a timeout the CTA records an error
 // flag, lets its loads in flight land, frees its TMEM and skips the output.
@@ -74,22 +78,26 @@ constexpr int TC_KCH = 16;                   // complex contraction values per 1
 constexpr int TC_KCH_H = 32;                 // complex contraction values per 128-byte FP16 row (near, aggregation)
 constexpr int TC_COLS = 64;                  // right-hand sides per column tile (MMA M = 128)
 constexpr int TC_ZBOX = 32;                  // rows per TMA box of the B operands
-constexpr int TC_ABYTES = 128 * 128;         // one A tile: 128 rows x 128 bytes
-// The ring: three stages of 72 KB for tiles of up to 160 rows, or four of 56 KB
-// where no tile has more than 96 (bytes in flight bound the kernel).
-template <int ST> struct TcRing {
-    static constexpr int ROWS = ST == 4 ? 96 : TC_ROWS;
-    static constexpr int BBYTES = ROWS * 128;               // one B tile at most
-    static constexpr int STAGE = 2 * TC_ABYTES + 2 * BBYTES;
-    static constexpr size_t SMEM = (size_t)ST * STAGE + 1024;   // + alignment of the ring
+constexpr int TC_ABYTES = 128 * 128;         // an A tile of 128-byte rows
+// The ring of a mode (TCM_*): for tiles of up to 160 rows four stages of 56 KB
+// (the receive, whose A tiles are expanded, three of 72), where no tile has more
+// than 96 five of 40 KB (four of 56)
+template <int MODE, bool LOW> struct TcRing {
+    static constexpr bool RAW = MODE == 2;
+    static constexpr int ST = (RAW ? 3 : 4) + LOW;
+    static constexpr int ROWS = LOW ? 96 : TC_ROWS;
+    static constexpr int ABYTES = RAW ? TC_ABYTES : TC_ABYTES / 2;   // one A tile
+    static constexpr int BBYTES = ROWS * 128;                       // one B tile at most
+    static constexpr int STAGE = 2 * ABYTES + 2 * BBYTES;
+    static constexpr size_t SMEM = (size_t)ST * STAGE + 1024;       // + alignment of the ring
 };
 constexpr int TC_PARTS = 15;                 // parts of a tile at most (about)
 constexpr uint32_t TC_TMEM_COLS = 256;
 constexpr uint32_t TC_SPIN = 1u << 20;       // mbarrier polls before a wait gives up
 
-// An operand in rows of 128 bytes: 16 complex values as TF32 (re, im) pairs,
-// or 32 as FP16 pairs scaled by a power of two per output row (rinv holds the
-// inverse scales), split into hi and lo parts.
+// An operand in rows of 128 bytes: 16 complex values as TF32 (re, im) pairs, or 32
+// as FP16, real parts before imaginary ones, scaled by a power of two per output
+// row (rinv holds the inverse scales); hi and lo parts.
 struct TcOperand {
     void* hi = nullptr;
     void* lo = nullptr;
@@ -186,6 +194,18 @@ __global__ void k_rinv(int n, const unsigned* __restrict__ rowmax, float* __rest
     if (k < n) rinv[k] = ldexpf(1.f, -h_scale_exp(__uint_as_float(rowmax[k])));
 }
 
+// Values v, w of places 2u, 2u + 1, scaled by 2^ex, to a row's [32 re][32 im], hi
+// and lo; o = the row's first pair + u
+__device__ __forceinline__ void put_planar(__half2* __restrict__ hi, __half2* __restrict__ lo, size_t o, float2 v,
+                                           float2 w, int ex) {
+    const float a = ldexpf(v.x, ex), b = ldexpf(w.x, ex), c = ldexpf(v.y, ex), d = ldexpf(w.y, ex);
+    const __half2 r = h_hi(a, b), i = h_hi(c, d);
+    hi[o] = r;
+    hi[o + TC_KCH_H / 2] = i;
+    lo[o] = h_lo(a, b, r);
+    lo[o + TC_KCH_H / 2] = h_lo(c, d, i);
+}
+
 // Z operand of block entry e (one CTA each) from the box-pair blocks (column-
 // major n_i x n_j at blk_off[e]): row zrow[e] + kc n_i + p holds
 // s_p Z(p, 32 kc + u), u = 0..31, as FP16 (re, im) pairs, hi and lo, with
@@ -201,16 +221,13 @@ __global__ void k_tc_fill_zh(const int* __restrict__ entry_box, const int* __res
     const int nkc = (nj + TC_KCH_H - 1) / TC_KCH_H;
     const float2* src = blk + blk_off[e];
     const size_t base = (size_t)zrow[e] * TC_KCH_H;
-    for (int q = threadIdx.x; q < nkc * ni * TC_KCH_H; q += blockDim.x) {
-        const int u = q % TC_KCH_H, rp = q / TC_KCH_H;     // rp = kc n_i + p
+    for (int q = threadIdx.x; q < nkc * ni * (TC_KCH_H / 2); q += blockDim.x) {
+        const int u = q % (TC_KCH_H / 2), rp = q / (TC_KCH_H / 2);     // rp = kc n_i + p
         const int kc = rp / ni, p = rp - kc * ni;
-        const int t = kc * TC_KCH_H + u;
+        const int t = kc * TC_KCH_H + 2 * u;
         const float2 v = t < nj ? src[(size_t)t * ni + p] : make_float2(0.f, 0.f);
-        const int ex = h_scale_exp(__uint_as_float(rowmax[i0 + p]));
-        const float a = ldexpf(v.x, ex), b = ldexpf(v.y, ex);
-        const __half2 h = h_hi(a, b);
-        zhi[base + (size_t)rp * TC_KCH_H + u] = h;
-        zlo[base + (size_t)rp * TC_KCH_H + u] = h_lo(a, b, h);
+        const float2 w = t + 1 < nj ? src[(size_t)(t + 1) * ni + p] : make_float2(0.f, 0.f);
+        put_planar(zhi, zlo, base + (size_t)rp * TC_KCH_H + u, v, w, h_scale_exp(__uint_as_float(rowmax[i0 + p])));
     }
 }
 
@@ -259,15 +276,15 @@ __global__ void __launch_bounds__(256) k_tc_pack_xh(int nchunk, int nrhs, const 
         xsm[u][cl] = (u < cd.y && col < nrhs) ? xs[(size_t)(cd.x + u) * nrhs + col] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    const size_t base = ((size_t)ct * nchunk + ch) * 128 * TC_KCH_H;
-    for (int q = threadIdx.x; q < 128 * TC_KCH_H; q += blockDim.x) {
-        const int row = q / TC_KCH_H, u = q - row * TC_KCH_H;
-        const float2 v = xsm[u][row >> 1];
+    const size_t base = ((size_t)ct * nchunk + ch) * 128 * (TC_KCH_H / 2);
+    for (int q = threadIdx.x; q < 128 * (TC_KCH_H / 2); q += blockDim.x) {
+        const int row = q / (TC_KCH_H / 2), u = 2 * (q - row * (TC_KCH_H / 2));
+        const float2 v = xsm[u][row >> 1], w = xsm[u + 1][row >> 1];
         const int ex = sexp[row >> 1];
-        const float a = ldexpf((row & 1) ? v.y : v.x, ex), b = ldexpf((row & 1) ? v.x : -v.y, ex);
+        const float a = ldexpf((row & 1) ? v.y : v.x, ex), b = ldexpf((row & 1) ? w.y : w.x, ex);
         const __half2 h = h_hi(a, b);
-        xhi[base + (size_t)row * TC_KCH_H + u] = h;
-        xlo[base + (size_t)row * TC_KCH_H + u] = h_lo(a, b, h);
+        xhi[base + q] = h;
+        xlo[base + q] = h_lo(a, b, h);
     }
 }
 
@@ -291,14 +308,11 @@ __global__ void k_tc_fill_rah(int K2, const int* __restrict__ box_ptr, const int
         const int ex = h_scale_exp(m);
         rinv[(size_t)b * K2 + q] = ldexpf(1.f, -ex);
         for (int kc = 0; kc < nkc; ++kc)
-            for (int u = 0; u < TC_KCH_H; ++u) {
-                const int t = kc * TC_KCH_H + u;
+            for (int u = 0; u < TC_KCH_H / 2; ++u) {
+                const int t = kc * TC_KCH_H + 2 * u;
                 const float2 v = t < n ? R[(size_t)(j0 + t) * K2 + q] : make_float2(0.f, 0.f);
-                const float x = ldexpf(v.x, ex), y = ldexpf(v.y, ex);
-                const __half2 h = h_hi(x, y);
-                const size_t o = base + ((size_t)kc * K2 + q) * TC_KCH_H + u;
-                hi[o] = h;
-                lo[o] = h_lo(x, y, h);
+                const float2 w = t + 1 < n ? R[(size_t)(j0 + t + 1) * K2 + q] : make_float2(0.f, 0.f);
+                put_planar(hi, lo, base + ((size_t)kc * K2 + q) * TC_KCH_H + u, v, w, ex);
             }
     }
 }
@@ -352,6 +366,7 @@ enum : int { TCM_NEAR = 0, TCM_AGG = 1, TCM_RECV = 2 };
 
 struct TcArgs {
     int nslots, nct;         // shares of the work, column tiles of 64
+    int nbuf;                // accumulators (pairs of them) in TMEM
     const int* slot;         // TcSlots ptr, item, ch
     const int4* item;
     const int2* ch;
@@ -381,13 +396,14 @@ struct TcFmt {
 template <int MODE>
 constexpr int TC_THREADS = MODE == TCM_RECV ? 320 : 256;
 
-template <int MODE, int ST>
+template <int MODE, bool LOW>
 __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mbhi, const __grid_constant__ CUtensorMap mblo,
               const __grid_constant__ CUtensorMap mxhi, const __grid_constant__ CUtensorMap mxlo, const TcArgs a) {
     constexpr bool NEAR = MODE == TCM_NEAR;
     constexpr bool RAW = MODE == TCM_RECV;
-    constexpr int STAGE = TcRing<ST>::STAGE, BBYTES = TcRing<ST>::BBYTES;
+    using Ring = TcRing<MODE, LOW>;
+    constexpr int ST = Ring::ST, STAGE = Ring::STAGE, ABYTES = Ring::ABYTES, BBYTES = Ring::BBYTES;
     constexpr uint32_t RAW_BYTES = TC_COLS * 128;   // 64 field rows of 16 complex values
     extern __shared__ unsigned char tc_raw[];
     __shared__ __align__(8) uint64_t full[ST], empty[ST], conv[ST], accf[2], acce[2], done;
@@ -397,6 +413,7 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
     const uint32_t raw = tc::smem_u32(tc_raw);
     unsigned char* ring = tc_raw + (((raw + 1023u) & ~1023u) - raw);   // 1024-aligned swizzle atoms
     const int nwork = a.nslots * a.nct;
+    const uint32_t nbuf = (uint32_t)a.nbuf, dim = nbuf == 2 ? TC_TMEM_COLS / 2 : TC_TMEM_COLS;   // second accumulator of a pair
     volatile int* vfail = &fail_s;
     if (tid == 0) {
         for (int s = 0; s < ST; ++s) {
@@ -445,7 +462,7 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                 const int i = tl.x, r0 = tl.y, nrow = tl.z, nch = ch.y;
                 const int ni = a.box_ptr[i + 1] - a.box_ptr[i];
                 const int nB = (nrow + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX;          // B rows staged
-                const uint32_t bytes = (RAW ? RAW_BYTES : 2u * TC_ABYTES) + 2u * (uint32_t)nB * 128u;
+                const uint32_t bytes = (RAW ? RAW_BYTES : 2u * ABYTES) + 2u * (uint32_t)nB * 128u;
                 int2 next = NEAR && nch ? a.list[ch.x] : make_int2(0, 0);   // a chunk ahead of its use
                 for (int cI = 0; cI < nch; ++cI, ++g) {
                     const int s = g % ST;
@@ -460,24 +477,24 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                         const int xr = (ct * a.nchunk + next.x) * 128;
                         zr = next.y + r0;
                         tc::tma_load_2d(st, &mxhi, 0, xr, &full[s]);
-                        tc::tma_load_2d(st + TC_ABYTES, &mxlo, 0, xr, &full[s]);
+                        tc::tma_load_2d(st + ABYTES, &mxlo, 0, xr, &full[s]);
                         if (cI + 1 < nch) next = a.list[ch.x + cI + 1];
                     } else if (MODE == TCM_AGG) {
                         const int xr = (ct * a.nchunk + a.cbase[i] + cI) * 128;
                         tc::tma_load_2d(st, &mxhi, 0, xr, &full[s]);
-                        tc::tma_load_2d(st + TC_ABYTES, &mxlo, 0, xr, &full[s]);
+                        tc::tma_load_2d(st + ABYTES, &mxlo, 0, xr, &full[s]);
                         zr = a.zrow[i] + cI * a.K2 + r0;
                     } else {
                         // raw field rows (box i, columns of this tile) into the lo tile's first 8 KB
-                        tc::tma_load_2d_hint(st + TC_ABYTES, &mxhi, 2 * TC_KCH * (ch.x + cI), i * a.nrhs + ct * TC_COLS,
+                        tc::tma_load_2d_hint(st + ABYTES, &mxhi, 2 * TC_KCH * (ch.x + cI), i * a.nrhs + ct * TC_COLS,
                                              &full[s], pol_b);
                         zr = a.zrow[i] + (ch.x + cI) * ni + r0;
                     }
                     // the aggregation's and receive's pattern operands are read by the
                     // tiles of one box (and the column tiles) only: streamed too
                     for (int qq = 0; qq < nB; qq += TC_ZBOX) {
-                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + qq * 128, &mbhi, 0, zr + qq, &full[s], pol_b);
-                        tc::tma_load_2d_hint(st + 2 * TC_ABYTES + BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s], pol_b);
+                        tc::tma_load_2d_hint(st + 2 * ABYTES + qq * 128, &mbhi, 0, zr + qq, &full[s], pol_b);
+                        tc::tma_load_2d_hint(st + 2 * ABYTES + BBYTES + qq * 128, &mblo, 0, zr + qq, &full[s], pol_b);
                     }
                 }
             }
@@ -495,8 +512,8 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
             for (int it = a.slot[sl]; it < t1; ++it) {
                 const int nch = a.ch[it].y;
                 if (nch == 0) continue;
-                const uint32_t buf = na & 1;
-                if (na >= 2 && !tc::mbar_wait(&acce[buf], ((na >> 1) - 1) & 1, TC_SPIN)) {
+                const uint32_t buf = na % nbuf;
+                if (na >= nbuf && !tc::mbar_wait(&acce[buf], (na / nbuf - 1) & 1, TC_SPIN)) {
                     ok = false;
                     break;
                 }
@@ -512,20 +529,27 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                     }
                     tc::tc_fence_after_sync();
                     const uint32_t st = tc::smem_u32(ring + (size_t)s * STAGE);
-                    const uint32_t ahi = st, alo = st + TC_ABYTES, bhi = st + 2 * TC_ABYTES, blo = bhi + BBYTES;
+                    const uint32_t ahi = st, alo = st + ABYTES, bhi = st + 2 * ABYTES, blo = bhi + BBYTES;
+                    if constexpr (RAW) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {   // K steps of 32 bytes of the 128-byte rows
-                        const uint32_t ko = 32u * k;
-                        const uint64_t dal = tc::kmajor_sw128_desc(alo + ko), dah = tc::kmajor_sw128_desc(ahi + ko);
-                        const uint64_t dbl = tc::kmajor_sw128_desc(blo + ko), dbh = tc::kmajor_sw128_desc(bhi + ko);
-                        if (TcFmt<MODE>::H) {
-                            tc::mma_f16(d, dal, dbh, idesc, (cI | k) != 0);
-                            tc::mma_f16(d, dah, dbl, idesc, 1);
-                            tc::mma_f16(d, dah, dbh, idesc, 1);
-                        } else {
+                        for (int k = 0; k < 4; ++k) {   // K steps of 32 bytes of the 128-byte rows
+                            const uint32_t ko = 32u * k;
+                            const uint64_t dal = tc::kmajor_sw128_desc(alo + ko), dah = tc::kmajor_sw128_desc(ahi + ko);
+                            const uint64_t dbl = tc::kmajor_sw128_desc(blo + ko), dbh = tc::kmajor_sw128_desc(bhi + ko);
                             tc::mma_tf32(d, dal, dbh, idesc, (cI | k) != 0);
                             tc::mma_tf32(d, dah, dbl, idesc, 1);
                             tc::mma_tf32(d, dah, dbh, idesc, 1);
+                        }
+                    } else {
+                        // K steps of 32 bytes of A's 64-byte rows, against Zr and Zi
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t ka = 32u * (k >> 1), kb = ka + 64u * (k & 1), dd = d + (k & 1 ? dim : 0u);
+                            const uint64_t dal = tc::kmajor_sw64_desc(alo + ka), dah = tc::kmajor_sw64_desc(ahi + ka);
+                            const uint64_t dbl = tc::kmajor_sw128_desc(blo + kb), dbh = tc::kmajor_sw128_desc(bhi + kb);
+                            tc::mma_f16(dd, dal, dbh, idesc, (cI | (k >> 1)) != 0);
+                            tc::mma_f16(dd, dah, dbl, idesc, 1);
+                            tc::mma_f16(dd, dah, dbh, idesc, 1);
                         }
                     }
                     tc::mma_commit(&empty[s]);
@@ -571,7 +595,7 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                     float4 v[4];
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        v[k] = *reinterpret_cast<const float4*>(st + TC_ABYTES + tc::sw128_offset(cl, kh + k));
+                        v[k] = *reinterpret_cast<const float4*>(st + ABYTES + tc::sw128_offset(cl, kh + k));
                     tc::named_bar_sync(1, 128);   // every raw row is read before the lo tile overwrites them
                     // rows 2cl and 2cl+1 place chunk k at k ^ (2cl & 7) (resp. +1): lanes
                     // with cl & 4 take the chunks in the order k ^ 1 so that the 8 lanes
@@ -592,8 +616,8 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                         const uint32_t oe = tc::sw128_offset(2 * cl, k), oo = tc::sw128_offset(2 * cl + 1, k);
                         *reinterpret_cast<float4*>(st + oe) = eh;
                         *reinterpret_cast<float4*>(st + oo) = oh;
-                        *reinterpret_cast<float4*>(st + TC_ABYTES + oe) = el;
-                        *reinterpret_cast<float4*>(st + TC_ABYTES + oo) = ol;
+                        *reinterpret_cast<float4*>(st + ABYTES + oe) = el;
+                        *reinterpret_cast<float4*>(st + ABYTES + oo) = ol;
                     }
                     tc::fence_proxy_async_smem();
                     tc::mbar_arrive(&conv[s]);
@@ -622,9 +646,9 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
                 continue;
             }
             const int i0 = a.box_ptr[i];
-            const uint32_t buf = na & 1;
+            const uint32_t buf = na % nbuf;
             // a warp-uniform decision: tcgen05.ld below is a whole-warp instruction
-            const bool got = __all_sync(0xffffffffu, tc::mbar_wait(&accf[buf], (na >> 1) & 1, TC_SPIN) ? 1 : 0);
+            const bool got = __all_sync(0xffffffffu, tc::mbar_wait(&accf[buf], (na / nbuf) & 1, TC_SPIN) ? 1 : 0);
             if (!got) {
                 *vfail = 1;
                 go = false;
@@ -633,41 +657,47 @@ __global__ void __launch_bounds__(TC_THREADS<MODE>, 1)
             tc::tc_fence_after_sync();
             const uint32_t d = tmem + buf * TC_TMEM_COLS + ((uint32_t)(32 * ew) << 16);
             for (int n0 = 0; n0 < nrow; n0 += 32) {
+                // the rows' inverse scales, one a lane (read row by row between the stores
+                // they were 10 000 cycles an item)
+                float rl = 1.f;
+                if (!RAW && n0 + lane < nrow)
+                    rl = __ldg(a.rinv + (MODE == TCM_AGG ? (size_t)i * a.K2 + r0 : (size_t)(i0 + r0)) + n0 + lane);
                 float v[32];
                 tc::tmem_ld_32x32b_x32(d + (uint32_t)n0, v);
-                // lane 2c holds Re and lane 2c + 1 Im of column c
+                // lane 2c holds Re and lane 2c + 1 Im of column c; with FP16 operands lane
+                // 2c Xr Zr (v) and Xr Zi (w), lane 2c + 1 Xi Zr and Xi Zi.  Half the rows
+                // are completed by each of the two.
+                float w[32];
+                if constexpr (!RAW) tc::tmem_ld_32x32b_x32(d + dim + (uint32_t)n0, w);
+                auto value = [&](int e, int o) {   // row e in the even lane, o in the odd lane
+                    const float m = odd ? v[o] : v[e], x = __shfl_xor_sync(0xffffffffu, odd ? v[e] : v[o], 1);
+                    if constexpr (RAW) return odd ? make_float2(x, m) : make_float2(m, x);
+                    const float n = odd ? w[o] : w[e], z = __shfl_xor_sync(0xffffffffu, odd ? w[e] : w[o], 1);
+                    return odd ? make_float2(x - n, m + z) : make_float2(m - z, x + n);
+                };
                 if (MODE == TCM_AGG) {
-                    // of four rows the even lane writes two, the odd lane two: 32 bytes of
-                    // the column's field a pair (8-byte stores by even lanes were a
-                    // sector each: 27 000 cycles an item, most of the kernel)
+                    // two rows of four each, 32 bytes of the column's field a pair (8-byte
+                    // stores by even lanes were a sector each: 27 000 cycles an item, most
+                    // of the kernel)
 #pragma unroll
                     for (int u = 0; u < 32; u += 4) {
-                        const float e0 = __shfl_xor_sync(0xffffffffu, odd ? v[u] : v[u + 2], 1);
-                        const float e1 = __shfl_xor_sync(0xffffffffu, odd ? v[u + 1] : v[u + 3], 1);
+                        const float2 v0 = value(u, u + 2), v1 = value(u + 1, u + 3);
                         const int p = n0 + u + 2 * odd;
-                        if (writer && p < nrow) {   // rows and 2K are even
-                            const float2 rs = *reinterpret_cast<const float2*>(a.rinv + (size_t)i * a.K2 + r0 + p);
-                            const float4 w = odd ? make_float4(e0, v[u + 2], e1, v[u + 3])
-                                                 : make_float4(v[u], e0, v[u + 1], e1);
-                            // powers of two: exact
+                        const float r0s = __shfl_sync(0xffffffffu, rl, u + 2 * odd) * cs;   // powers of two: exact
+                        const float r1s = __shfl_sync(0xffffffffu, rl, u + 2 * odd + 1) * cs;
+                        if (writer && p < nrow)   // rows and 2K are even
                             *reinterpret_cast<float4*>(a.C + ((size_t)i * a.nrhs + col) * a.K2 + r0 + p) =
-                                make_float4(w.x * rs.x * cs, w.y * rs.x * cs, w.z * rs.y * cs, w.w * rs.y * cs);
-                        }
+                                make_float4(v0.x * r0s, v0.y * r0s, v1.x * r1s, v1.y * r1s);
                     }
                 } else {
-                    // of two rows the even lane writes one, the odd lane the other
 #pragma unroll
                     for (int u = 0; u < 32; u += 2) {
-                        const float e = __shfl_xor_sync(0xffffffffu, odd ? v[u] : v[u + 1], 1);
-                        const float re = odd ? e : v[u], im = odd ? v[u + 1] : e;
+                        const float2 t = value(u, u + 1);
                         const int p = n0 + u + odd;
-                        if (writer && p < nrow) {
-                            const int pos = i0 + r0 + p;
-                            const float rs = NEAR ? a.rinv[pos] : 1.f;
-                            a.ws[((size_t)tl.w * a.N + pos) * a.nrhs + col] =
-                                NEAR ? make_float2(re * rs * cs, im * rs * cs)
-                                     : make_float2(-(a.facy * im), a.facy * re);
-                        }
+                        const float rs = NEAR ? __shfl_sync(0xffffffffu, rl, u + odd) * cs : 1.f;
+                        if (writer && p < nrow)
+                            a.ws[((size_t)tl.w * a.N + i0 + r0 + p) * a.nrhs + col] =
+                                NEAR ? make_float2(t.x * rs, t.y * rs) : make_float2(-(a.facy * t.y), a.facy * t.x);
                     }
                 }
             }
@@ -800,19 +830,22 @@ static void tc_slots_free(TcSlots* w) {
 // Whole tiles per CTA left SMs idle: 184 tiles of the 30720-RWG spheroid's boxes
 // need two rounds on 152 SMs, 46 tiles of the 7680-RWG one under a third.  A share
 // holds eight chunks or more, a tile about TC_PARTS parts at most.  The FP32
-// accumulations are shorter in parts: 7680 RWG are 6.2e-6
-// from FP64 instead of 1.5e-5.
-// 30720 RWG x 64 columns: near field 167 -> 136 us, receive 80 -> 54, the whole
-// product 708 -> 592 (with k_tc_sum and the aggregation's stores); a mixed solve of
-// 17280 unknowns x 32 columns 104 -> 84 ms.
-static int tc_slots(Ctx* c, TcSlots* w, const std::vector<int4>& tiles, const std::vector<int2>& ch, bool split) {
+// accumulations are shorter in parts: 7680 RWG are 6.2e-6 from FP64 instead of
+// 1.5e-5.  30720 RWG x 64 columns: near field 167 -> 136 us, receive 80 -> 54.
+// chunk_cost and item_cost, in rows staged: a line through the CTAs' measured
+// times, near field 780 + 4.2 rows cycles a chunk and 10 600 an item, aggregation
+// 1500 a chunk and 5100 an item, receive 1420 + 5.1 rows and 670.  By bytes alone
+// the last CTA took 25 % (near) to 80 % (aggregation) longer than the mean, now 10 to
+// 27 %: near field 136 -> 124 us, aggregation 59 -> 35.
+static int tc_slots(Ctx* c, TcSlots* w, const std::vector<int4>& tiles, const std::vector<int2>& ch, bool split,
+                    double chunk_cost, double item_cost) {
     tc_slots_free(w);
-    auto cost = [&](size_t k) { return 128.0 + (tiles[k].z + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX; };   // rows staged a chunk
+    auto cost = [&](size_t k) { return chunk_cost + (tiles[k].z + TC_ZBOX - 1) / TC_ZBOX * TC_ZBOX; };   // rows staged a chunk
     double all = 0, most = 0;
     long long chunks = 0;
     for (size_t k = 0; k < tiles.size(); ++k) {
-        all += cost(k) * ch[k].y;
-        most = std::max(most, cost(k) * ch[k].y);
+        all += item_cost + cost(k) * ch[k].y;
+        most = std::max(most, item_cost + cost(k) * ch[k].y);
         chunks += ch[k].y;
     }
     int n = c->tc->nsm;
@@ -837,11 +870,11 @@ static int tc_slots(Ctx* c, TcSlots* w, const std::vector<int4>& tiles, const st
         const int nch = ch[k].y;
         int part = 0;
         if (!split) {
-            s = all > 0 ? std::max(s, std::min(n - 1, (int)((before + 0.5 * ck * nch) * n / all))) : 0;
+            s = all > 0 ? std::max(s, std::min(n - 1, (int)((before + 0.5 * (item_cost + ck * nch)) * n / all))) : 0;
             put(k, part++, 0, nch);
         }
         for (int a = 0; split && a < nch;) {
-            int e = s == n - 1 ? nch : std::min(nch, (int)std::lround((all * (s + 1) / n - before) / ck));
+            int e = s == n - 1 ? nch : std::min(nch, (int)std::lround((all * (s + 1) / n - before - item_cost) / ck));
             if (nch - e <= 2) e = nch;
             if (e <= a || (e < nch && e - a <= 2)) {
                 ++s;
@@ -851,7 +884,7 @@ static int tc_slots(Ctx* c, TcSlots* w, const std::vector<int4>& tiles, const st
             a = e;
             if (e < nch) ++s;
         }
-        before += ck * nch;
+        before += item_cost + ck * nch;
         w->parts = std::max(w->parts, part);
         if (split)
             for (int r = 0; r < tiles[k].z; ++r) np[c->box_ptr[tiles[k].x] + tiles[k].y + r] = (unsigned char)part;
@@ -936,6 +969,14 @@ static int tc_setup(Ctx* c) {
     return st;
 }
 
+template <int MODE>
+static bool tc_smem(Ctx* c) {
+    return cuda_ok(c, cudaFuncSetAttribute(k_tc_gemm<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)TcRing<MODE, false>::SMEM), "shared memory") &&
+           cuda_ok(c, cudaFuncSetAttribute(k_tc_gemm<MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)TcRing<MODE, true>::SMEM), "shared memory");
+}
+
 static int tc_setup_build(Ctx* c) {
     int st;
     if ((st = device_blocks_ready(c))) return st;
@@ -999,7 +1040,7 @@ static int tc_setup_build(Ctx* c) {
     c->tc = t;
     t->tiles = tiles;
     for (const int4& q : tiles) t->maxrows = std::max(t->maxrows, q.z);
-    if ((st = tc_slots(c, &t->near, tiles, tch, true))) return st;
+    if ((st = tc_slots(c, &t->near, tiles, tch, true, 184, 2500))) return st;
     CK(cudaMalloc(&t->dlist, std::max<size_t>(list.size(), 1) * sizeof(int2)));
     CK(cudaMemcpy(t->dlist, list.data(), list.size() * sizeof(int2), cudaMemcpyHostToDevice));
     t->nchunk = (int)chunk.size();
@@ -1014,12 +1055,7 @@ static int tc_setup_build(Ctx* c) {
     CK(cudaMemcpy(t->dchunk, chunk.data(), chunk.size() * sizeof(int2), cudaMemcpyHostToDevice));
     CK(cudaMemset(t->derr, 0, sizeof(int)));
     if ((st = tc_near_operand(c, c->dZblk, &t->Z, c->stream))) return st;
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<3>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_NEAR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_AGG, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
-    CK(cudaFuncSetAttribute(k_tc_gemm<TCM_RECV, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcRing<4>::SMEM));
+    if (!tc_smem<TCM_NEAR>(c) || !tc_smem<TCM_AGG>(c) || !tc_smem<TCM_RECV>(c)) return MLF_E_CUDA;
     CK(cudaStreamSynchronize(c->stream));
     return MLF_OK;
 }
@@ -1046,13 +1082,13 @@ static int tc_x_buffers(Ctx* c, int nrhs) {
     t->dcinv = nullptr;
     t->xrows_cap = 0;
     t->cols_cap = 0;
-    CK(cudaMalloc(&t->xhi, (size_t)rows * 128));
-    CK(cudaMalloc(&t->xlo, (size_t)rows * 128));
+    CK(cudaMalloc(&t->xhi, (size_t)rows * 64));
+    CK(cudaMalloc(&t->xlo, (size_t)rows * 64));
     CK(cudaMalloc(&t->dcmax, (size_t)nct * TC_COLS * sizeof(unsigned)));
     CK(cudaMalloc(&t->dcinv, (size_t)nct * TC_COLS * sizeof(float)));
     int st;
-    if ((st = make_rows_map(c, &t->mxhi, t->xhi, rows, 128))) return st;
-    if ((st = make_rows_map(c, &t->mxlo, t->xlo, rows, 128))) return st;
+    if ((st = make_map_2d(c, &t->mxhi, t->xhi, 16, rows, 64, 16, 128, CU_TENSOR_MAP_SWIZZLE_64B))) return st;
+    if ((st = make_map_2d(c, &t->mxlo, t->xlo, 16, rows, 64, 16, 128, CU_TENSOR_MAP_SWIZZLE_64B))) return st;
     t->xrows_cap = rows;
     t->cols_cap = nct * TC_COLS;
     return MLF_OK;
@@ -1096,10 +1132,12 @@ static void tc_launch(const TcState* t, const TcSlots& w, int rows, const CUtens
     a.item = w.item;
     a.ch = w.ch;
     const unsigned grid = (unsigned)std::max(1, std::min(t->nsm, w.n * a.nct));
-    if (rows <= TcRing<4>::ROWS)
-        k_tc_gemm<MODE, 4><<<grid, TC_THREADS<MODE>, TcRing<4>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
+    // the pair of a tile's accumulators twice in TMEM up to 128 rows, the receive's one always
+    a.nbuf = MODE == TCM_RECV || rows <= (int)TC_TMEM_COLS / 2 ? 2 : 1;
+    if (rows <= TcRing<MODE, true>::ROWS)
+        k_tc_gemm<MODE, true><<<grid, TC_THREADS<MODE>, TcRing<MODE, true>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
     else
-        k_tc_gemm<MODE, 3><<<grid, TC_THREADS<MODE>, TcRing<3>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
+        k_tc_gemm<MODE, false><<<grid, TC_THREADS<MODE>, TcRing<MODE, false>::SMEM, s>>>(bhi, blo, xhi, xlo, a);
 }
 
 static dim3 tc_sum_grid(const Ctx* c, int nrhs) { return dim3((c->N + 31) / 32, (nrhs + 31) / 32); }
@@ -1189,8 +1227,9 @@ static int tc_leaf_setup(Ctx* c, const float2* R, int K2) {
     abase[nb] = (int)arows;
     rbase[nb] = (int)rrows;
     t->arows = std::min(per, K2);
-    if ((st = tc_slots(c, &t->agg, tiles, tch, false))) return st;
-    if ((st = tc_slots(c, &t->recv, t->tiles, std::vector<int2>(t->tiles.size(), make_int2(0, nqc)), true))) return st;
+    if ((st = tc_slots(c, &t->agg, tiles, tch, false, 248, 1200))) return st;
+    if ((st = tc_slots(c, &t->recv, t->tiles, std::vector<int2>(t->tiles.size(), make_int2(0, nqc)), true, 279,
+                       131))) return st;
     CK(cudaMalloc(&t->dabase, abase.size() * sizeof(int)));
     CK(cudaMalloc(&t->drbase, rbase.size() * sizeof(int)));
     CK(cudaMemcpy(t->dabase, abase.data(), abase.size() * sizeof(int), cudaMemcpyHostToDevice));

@@ -43,6 +43,9 @@ MLF_HD constexpr uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t 
 // 8 TF32 values inside the 128-byte row moves the start address by 32 bytes.
 MLF_HD constexpr uint64_t kmajor_sw128_desc(uint32_t addr) { return smem_desc(addr, 16, 1024, SWIZZLE_128B); }
 
+// The same with rows of 64 bytes and 64-byte swizzling: 8-row atoms of 512 bytes.
+MLF_HD constexpr uint64_t kmajor_sw64_desc(uint32_t addr) { return smem_desc(addr, 16, 512, SWIZZLE_64B); }
+
 // Byte offset of 16-byte chunk c (0..7) of row r in such a tile, for operands
 // written by threads rather than TMA: the 128-byte swizzle places the chunk at
 // c XOR (r mod 8) within its row (the tile 1024-byte aligned).
