@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "mlf_cvt.cuh"
+#include "mlf_f32x2.cuh"
 #include "mlf_internal.h"
 #include "mlf_sep.cuh"
 
@@ -79,25 +80,6 @@ __global__ void k32_aggregate(int K, int nrhs, int N, const int* __restrict__ bo
         for (int j = j0; j < j1; ++j) fmac(acc, R[(size_t)j * 2 * K + q], xr[perm[j]]);
         C[((size_t)b * nrhs + r) * 2 * K + q] = acc;
     }
-}
-
-// Two FP32 values in one 64-bit register pair: Blackwell's packed FMA does two
-// per instruction slot.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 up2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 
 // 16 bytes if on, else r as it was (not read then): the load is predicated, so

@@ -44,6 +44,7 @@
 #include <cmath>
 #include <vector>
 
+#include "mlf_f32x2.cuh"
 #include "mlf_internal.h"
 
 namespace mlf {
@@ -102,7 +103,11 @@ __device__ __forceinline__ int bsearch_cols(const int* S, int n, int v) {
 // and the current tile's D values are already in flight (registers), so the
 // loads overlap the FMAs.  Warp w owns columns 8w .. 8w+7 of a tile and each
 // lane rows lane and lane + 32: the U values are warp-wide broadcasts and the
-// D accesses coalesced.  The caller synchronises before; this ends synchronised.
+// D accesses coalesced.  The FMAs are packed over pairs of columns, in half the
+// issue slots, each sum as before (inverses, scalar -> packed: 2216 boxes of 776
+// unknowns 164 -> 151 ms, 504 of 790 55.8 -> 53, 824 of 2157 1155 -> 1127, 32 of
+// 2014 unchanged; 128 rows a tile were slower).  The caller synchronises before;
+// this ends synchronised.
 // The 2-ring variant (training targets of the learned preconditioner): the
 // system comes from a dense Z (complex(4), row-major N x N) over each box's
 // sorted 2-ring list, and the rows go to M2 on the near pattern.  Zd null:
@@ -118,8 +123,12 @@ struct LuRing {
 
 struct LuTiles {
     float2 L[LU_T][LU_P + 1];
-    float2 U[2][LU_P][LU_T + 1];
+    union {
+        float2 U[2][LU_P][LU_T + 1];
+        float P[2][2][LU_P][LU_T + 4];   // trailing update: real and imaginary parts apart, pairs of columns
+    };
 };
+static_assert(sizeof(LuTiles) <= LU_SMEM2, "the one-CTA kernel's shared memory holds the tiles");
 
 // The panel's row swaps as one move: row k0 + t gets row top[t]; row pos[t] (below
 // the panel's diagonal block, -1: none) gets row from[t].
@@ -165,7 +174,8 @@ __device__ __forceinline__ void lu_strip_update(LuTiles& sm, float2* __restrict_
         for (int k = 0; k < PER; ++k) {
             const int e = tid + k * LU_THREADS;
             const int j = e / LU_P, t = e - j * LU_P;
-            sm.U[buf][t][j] = un[k];
+            sm.P[buf][0][t][j] = un[k].x;
+            sm.P[buf][1][t][j] = un[k].y;
         }
     };
     load_u(cbeg);
@@ -188,24 +198,30 @@ __device__ __forceinline__ void lu_strip_update(LuTiles& sm, float2* __restrict_
         }
         // the K-sum accumulates on its own and is subtracted once (the
         // in-place form rounds each product against the larger D value)
-        float2 acc[2][8];
+        f32x2 ax[2][4], ay[2][4];   // rows lane, lane + 32; pairs of columns
 #pragma unroll
         for (int u = 0; u < 2; ++u)
 #pragma unroll
-            for (int v = 0; v < 8; ++v) acc[u][v] = make_float2(0.f, 0.f);
+            for (int v = 0; v < 4; ++v) ax[u][v] = ay[u][v] = 0;
         for (int t = 0; t < kb; ++t) {
-            const float2 a0 = sm.L[lane][t], a1 = sm.L[lane + 32][t];
+            const ulonglong2* px = reinterpret_cast<const ulonglong2*>(&sm.P[buf][0][t][8 * w]);
+            const ulonglong2* py = reinterpret_cast<const ulonglong2*>(&sm.P[buf][1][t][8 * w]);
+            const ulonglong2 x0 = px[0], x1 = px[1], y0 = py[0], y1 = py[1];
+            const f32x2 bx[4] = {x0.x, x0.y, x1.x, x1.y}, by[4] = {y0.x, y0.y, y1.x, y1.y};
 #pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                const float2 b = sm.U[buf][t][8 * w + v];
-                acc[0][v].x = fmaf(a0.x, b.x, acc[0][v].x);
-                acc[0][v].x = fmaf(-a0.y, b.y, acc[0][v].x);
-                acc[0][v].y = fmaf(a0.x, b.y, acc[0][v].y);
-                acc[0][v].y = fmaf(a0.y, b.x, acc[0][v].y);
-                acc[1][v].x = fmaf(a1.x, b.x, acc[1][v].x);
-                acc[1][v].x = fmaf(-a1.y, b.y, acc[1][v].x);
-                acc[1][v].y = fmaf(a1.x, b.y, acc[1][v].y);
-                acc[1][v].y = fmaf(a1.y, b.x, acc[1][v].y);
+            for (int u = 0; u < 2; ++u) {
+                const float2 l = sm.L[lane + 32 * u][t];
+                const f32x2 lx = pk2(l.x, l.x), ly = pk2(l.y, l.y), ln = pk2(-l.y, -l.y);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    ax[u][v] = fma2(lx, bx[v], ax[u][v]);
+                    ay[u][v] = fma2(lx, by[v], ay[u][v]);
+                }
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    ax[u][v] = fma2(ln, by[v], ax[u][v]);
+                    ay[u][v] = fma2(ly, bx[v], ay[u][v]);
+                }
             }
         }
 #pragma unroll
@@ -216,7 +232,9 @@ __device__ __forceinline__ void lu_strip_update(LuTiles& sm, float2* __restrict_
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int i = lane + 32 * u;
-                if (r0 + i < nrows) col[dr + r0 + i] = make_float2(d[u][v].x - acc[u][v].x, d[u][v].y - acc[u][v].y);
+                const float2 x = up2(ax[u][v / 2]), y = up2(ay[u][v / 2]);
+                if (r0 + i < nrows)
+                    col[dr + r0 + i] = make_float2(d[u][v].x - (v & 1 ? x.y : x.x), d[u][v].y - (v & 1 ? y.y : y.x));
             }
         }
         if (c0 + LU_T < cend) stage_u(buf ^ 1);
