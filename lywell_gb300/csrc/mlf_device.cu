@@ -17,7 +17,7 @@
 //   k_aggregate       leaf C = sum_n R_n x_n                  (:1805-1811)
 //   k_interp_sep      parent C += shift * Interpolar(child C), as a theta
 //                     pass then a phi pass (mlf_sep.cuh)       (:1818-1831)
-//   k_translate       B = w * sum_far C_src T                  (:1838-1853)
+//   k_translate       B = w * sum_far C_src T, all levels      (:1838-1853)
 //   k_anterp_sep      A = B + Anterpolar(shift* parent A|B), transposed
 //                     phi pass then theta pass (mlf_sep.cuh)   (:1857-1897)
 //   k_receive_near_d  y = fac sum conj(R) A + Znear x, near values in
@@ -188,25 +188,49 @@ __global__ void k_aggregate(int K, int nrhs, int ld, const int* __restrict__ box
     }
 }
 
-// blockIdx.x = (box*nrhs + r)*nchunk + chunk
-__global__ void k_translate(int K, int nrhs, int nchunk, const int* __restrict__ far_ptr,
-                            const int* __restrict__ far_src, const int* __restrict__ far_tid,
-                            const double2* __restrict__ T, const double* __restrict__ wq,
-                            const double2* __restrict__ C, double2* __restrict__ B) {
-    const int chunk = blockIdx.x % nchunk;
-    const int br = blockIdx.x / nchunk;
+// One level of the translation; its CTAs follow block0, (box*nrhs + r)*nchunk + chunk
+struct TrLevel {
+    int K, nchunk;
+    unsigned block0;
+    const int *far_ptr, *far_src, *far_tid;
+    const double2* T;
+    const double* wq;
+    const double2* C;
+    double2* B;
+};
+constexpr int TR_LEVELS = 16;   // levels of one launch
+struct TrLevels {
+    TrLevel l[TR_LEVELS];
+    int n;
+};
+
+// The levels' translations do not depend on each other: one launch, so that small
+// levels, which leave the FP64 pipes of most SMs idle one by one, run together
+// (a warp's FP64 instruction holds its pipe for 64 cycles, four an entry of the far
+// list).  One column of 1920 unknowns: the product 117.2 -> 109.1 us, of 122 880 6378 ->
+// 6285.
+__global__ void __launch_bounds__(128) k_translate(int nrhs, const __grid_constant__ TrLevels ls) {
+    int lv = 0;
+    while (lv + 1 < ls.n && blockIdx.x >= ls.l[lv + 1].block0) ++lv;
+    const TrLevel& l = ls.l[lv];
+    const int K = l.K, chunk = (blockIdx.x - l.block0) % l.nchunk;
+    const int br = (blockIdx.x - l.block0) / l.nchunk;
     const int b = br / nrhs, r = br % nrhs;
     const int q = chunk * blockDim.x + threadIdx.x;
     if (q >= 2 * K) return;
     const int k = q >= K ? q - K : q;
+    const int* __restrict__ far_src = l.far_src;
+    const int* __restrict__ far_tid = l.far_tid;
+    const double2* __restrict__ T = l.T;
+    const double2* __restrict__ C = l.C;
     double2 acc = make_double2(0, 0);
-    const int f1 = far_ptr[b + 1];
-    for (int f = far_ptr[b]; f < f1; ++f) {
+    const int f1 = l.far_ptr[b + 1];
+    for (int f = l.far_ptr[b]; f < f1; ++f) {
         const double2 cs = C[((size_t)far_src[f] * nrhs + r) * 2 * K + q];
         cmac(acc, cs, T[(size_t)far_tid[f] * K + k]);
     }
-    const double wk = wq[k];
-    B[((size_t)b * nrhs + r) * 2 * K + q] = make_double2(acc.x * wk, acc.y * wk);
+    const double wk = l.wq[k];
+    l.B[((size_t)b * nrhs + r) * 2 * K + q] = make_double2(acc.x * wk, acc.y * wk);
 }
 
 // One warp per (sorted basis j, rhs): y[perm[j]] = fac * sum conj(R_j) A_box
@@ -504,11 +528,16 @@ int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, c
             Cf[n], Cf[n - 1]);
     }
     if (ev) cudaEventRecord(ev[2], s);
-    for (int n = 3; n <= nl; ++n) {
-        Level& L = c->lv[n];
-        const int bd = 128, nch = chunks(2 * L.K, bd);
-        k_translate<<<L.nb * nrhs * nch, bd, 0, s>>>(L.K, nrhs, nch, L.dfar_ptr, L.dfar_src, L.dfar_tid,
-                                                     L.dT, L.dwq, Cf[n], Bf[n]);
+    for (int n = nl; n >= 3;) {   // from the leaves, as many levels as a launch takes
+        TrLevels ls{};
+        unsigned blocks = 0;
+        for (; n >= 3 && ls.n < TR_LEVELS; --n) {
+            Level& L = c->lv[n];
+            const int nch = chunks(2 * L.K, 128);
+            ls.l[ls.n++] = {L.K, nch, blocks, L.dfar_ptr, L.dfar_src, L.dfar_tid, L.dT, L.dwq, Cf[n], Bf[n]};
+            blocks += (unsigned)(L.nb * nrhs * nch);
+        }
+        k_translate<<<blocks, 128, 0, s>>>(nrhs, ls);
     }
     if (ev) cudaEventRecord(ev[3], s);
     for (int n = 4; n <= nl; ++n) {
