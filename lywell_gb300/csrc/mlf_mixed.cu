@@ -105,14 +105,37 @@ __device__ __forceinline__ void ldg128_if(bool on, float4& r, const float4* p) {
 // in flight (3.0, 3.5 ms).  69120-RWG sphere, 16 columns: 2.97 -> 2.58 ms;
 // 122880-RWG sphere, one column: 0.449 -> 0.389 ms; 30720-RWG spheroid, 64
 // columns: 0.180 -> 0.141 ms (before: one sample a thread, unpacked, 4 boxes).
+// The levels share a launch: a small one alone leaves SMs idle (the product
+// of one column of 122880 unknowns 961 -> 846 us, of 30720 x 64 530 -> 521, of 69120 x
+// 16 5614 -> 5530).
+struct Tr32Level {
+    int KP, nb, nchunk;
+    unsigned block0;                  // first of its (group, chunk) blocks
+    const int *gptr, *gsrc, *gtid;
+    const float4* T;
+    const float2* wq;
+    const float4* C;
+    float4* B;
+};
+constexpr int TR32_LEVELS = 16;       // levels of one launch
+struct Tr32Levels {
+    Tr32Level l[TR32_LEVELS];
+    int n;
+};
+
 template <int NR, int G>
-__global__ void __launch_bounds__(32)
-k32_translate_grp(int KP, int nb, int nrhs, int nchunk, const int* __restrict__ gptr,
-                  const int* __restrict__ gsrc, const int* __restrict__ gtid, const float4* __restrict__ T,
-                  const float2* __restrict__ wq, const float4* __restrict__ C, float4* __restrict__ B) {
-    const int gr = blockIdx.x / nchunk;
+__global__ void __launch_bounds__(32) k32_translate_grp(int nrhs, const __grid_constant__ Tr32Levels ls) {
+    int lv = 0;
+    while (lv + 1 < ls.n && blockIdx.x >= ls.l[lv + 1].block0) ++lv;
+    const Tr32Level& l = ls.l[lv];
+    const int KP = l.KP, nb = l.nb, nchunk = l.nchunk, bx = (int)(blockIdx.x - l.block0);
+    const int *__restrict__ gptr = l.gptr, *__restrict__ gsrc = l.gsrc, *__restrict__ gtid = l.gtid;
+    const float4 *__restrict__ T = l.T, *__restrict__ C = l.C;
+    const float2* __restrict__ wq = l.wq;
+    float4* __restrict__ B = l.B;
+    const int gr = bx / nchunk;
     const int c0 = blockIdx.y * NR;
-    const int k = blockIdx.x % nchunk * 32 + threadIdx.x;   // pair of samples
+    const int k = bx % nchunk * 32 + threadIdx.x;   // pair of samples
     if (k >= KP) return;
     f32x2 a[G][2 * NR][2], b[G][2 * NR][2];   // sums of C Re T and C Im T, per box, slot and sample
 #pragma unroll
@@ -519,23 +542,23 @@ static int matvec32_core(Ctx* c, const double2* x, const float2* x32, double2* y
             mp.C);
     }
     if (prof) cudaEventRecord(c->ev[2], s);
-    for (int n = 3; n <= nl; ++n) {
-        Level& L = c->lv[n];
-        const Mixed32::Lv& m = c->m32.lv[n];
+    for (int n = nl; n >= 3;) {   // from the leaves, as many levels as a launch takes
         const int G = c->tr_group ? c->tr_group : 2;
         const int nr = std::min(nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : 4, c->tr_cols ? c->tr_cols : 2);
-        const int KP = L.K / 2, ng = (L.nb + G - 1) / G, ncol = (nrhs + nr - 1) / nr;
-        const int nch = (KP + 31) / 32;
-        const dim3 grid(ng * nch, ncol);
-        const int* gp = G == 1 ? L.dfar_ptr : m.grp[G / 4].ptr;
-        const int* gs = G == 1 ? L.dfar_src : m.grp[G / 4].src;
-        const int* gt = G == 1 ? L.dfar_tid : m.grp[G / 4].tid;
-#define TGRP(NR_, G_)                                                                                              \
-    k32_translate_grp<NR_, G_><<<grid, 32, 0, s>>>(KP, L.nb, nrhs, nch, gp, gs, gt,                          \
-                                                    reinterpret_cast<const float4*>(m.T),                          \
-                                                    reinterpret_cast<const float2*>(m.wq),                         \
-                                                    reinterpret_cast<const float4*>(m.C),                          \
-                                                    reinterpret_cast<float4*>(m.B))
+        Tr32Levels ls{};
+        unsigned blocks = 0;
+        for (; n >= 3 && ls.n < TR32_LEVELS; --n) {
+            Level& L = c->lv[n];
+            const Mixed32::Lv& m = c->m32.lv[n];
+            const int KP = L.K / 2, nch = (KP + 31) / 32;
+            ls.l[ls.n++] = {KP, L.nb, nch, blocks, G == 1 ? L.dfar_ptr : m.grp[G / 4].ptr,
+                            G == 1 ? L.dfar_src : m.grp[G / 4].src, G == 1 ? L.dfar_tid : m.grp[G / 4].tid,
+                            reinterpret_cast<const float4*>(m.T), reinterpret_cast<const float2*>(m.wq),
+                            reinterpret_cast<const float4*>(m.C), reinterpret_cast<float4*>(m.B)};
+            blocks += (unsigned)((L.nb + G - 1) / G * nch);
+        }
+        const dim3 grid(blocks, (nrhs + nr - 1) / nr);
+#define TGRP(NR_, G_) k32_translate_grp<NR_, G_><<<grid, 32, 0, s>>>(nrhs, ls)
 #define TNR(G_)                                                       \
     do {                                                              \
         if (nr == 1) TGRP(1, G_);                                     \
