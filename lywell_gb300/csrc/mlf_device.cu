@@ -22,6 +22,8 @@
 //                     phi pass then theta pass (mlf_sep.cuh)   (:1857-1897)
 //   k_receive_near_d  y = fac sum conj(R) A + Znear x, near values in
 //                     complex(8)                               (:1915-1942)
+// Blocks of columns on full leaf boxes take aggregation, receive and near field
+// to the tensor cores by exact digit splits (mlf_split64.cu).
 // fp64_matvec_launch issues these on given field buffers: the context's own
 // (device_matvec) or the allocation-free entry point's fixed scratch
 // (mlf_noalloc.cu).
