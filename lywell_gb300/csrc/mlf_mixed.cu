@@ -684,47 +684,68 @@ __global__ void k_mdot(int N, int nrhs, const double2* __restrict__ V, size_t vs
     if (threadIdx.x == 0) partial[((size_t)i * nrhs + col) * gridDim.x + blockIdx.x] = make_double2(rs[0], is[0]);
 }
 
-// out[k] = sum_b partial[k*GM_BLOCKS + b], fixed order; a thread's loads are the
-// time (19 us one after the other), so 16 are in flight
-__global__ void k_reduce_partials(int nk, const double2* __restrict__ partial, double2* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
+// out[k] = sum_b partial[k*GM_BLOCKS + b], a warp each: four in order a lane, then
+// halves (one thread's chain of FP64 additions, 64 cycles each, took 15.6 us)
+__global__ void __launch_bounds__(32) k_reduce_partials(const double2* __restrict__ partial, double2* __restrict__ out) {
+    const double2* p = partial + (size_t)blockIdx.x * GM_BLOCKS;
     double2 s = make_double2(0, 0);
-#pragma unroll 16
-    for (int b = 0; b < GM_BLOCKS; ++b) {
-        s.x += partial[(size_t)k * GM_BLOCKS + b].x;
-        s.y += partial[(size_t)k * GM_BLOCKS + b].y;
+#pragma unroll
+    for (int b = 0; b < GM_BLOCKS / 32; ++b) {
+        const double2 v = p[32 * b + threadIdx.x];
+        s.x += v.x;
+        s.y += v.y;
     }
-    out[k] = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 // FP32 Arnoldi kernels: basis V32 and work vector w32 in float, per-thread
 // sums in float, block and final reductions in double.
-__global__ void k_mdot32(int N, int nrhs, const float2* __restrict__ V, size_t vstride, const float2* __restrict__ w,
-                         double2* __restrict__ partial) {
-    const int col = blockIdx.y, i = blockIdx.z;
-    const float2* wc = w + (size_t)col * N;
-    const float2* vc = V ? V + i * vstride + (size_t)col * N : nullptr;
-    float sr = 0.f, si = 0.f;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
-        const float2 b = wc[e];
-        if (vc) {
-            const float2 a = vc[e];
-            sr = fmaf(a.x, b.x, sr); sr = fmaf(a.y, b.y, sr);
-            si = fmaf(a.x, b.y, si); si = fmaf(-a.y, b.x, si);
-        } else {
-            sr = fmaf(b.x, b.x, sr); sr = fmaf(b.y, b.y, sr);
+
+// partial[col * gridDim.x + block] = sum |w|^2 of NRM_E values a thread, squares in
+// float, sums in double (float -> double by moves); with a value a thread on 128 CTAs
+// a column, and the sums of 128 partials by one thread each, the norms of 17280 x 32
+// took 27 us, 9.7 now with the scales
+constexpr int NRM_E = 8;
+__global__ void __launch_bounds__(256) k_norm32(int N, const float2* __restrict__ w, double* __restrict__ partial) {
+    const float2* wc = w + (size_t)blockIdx.y * N;
+    double s = 0;
+#pragma unroll
+    for (int u = 0; u < NRM_E; ++u) {
+        const int e = (blockIdx.x * NRM_E + u) * 256 + threadIdx.x;
+        if (e < N) {
+            const float2 v = wc[e];
+            s += f2d(fmaf(v.y, v.y, v.x * v.x));
         }
     }
-    __shared__ double rs[256], is[256];
-    rs[threadIdx.x] = sr;
-    is[threadIdx.x] = si;
+    __shared__ double ws[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) { rs[threadIdx.x] += rs[threadIdx.x + s]; is[threadIdx.x] += is[threadIdx.x + s]; }
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; ++q) s += ws[q];
+        partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
     }
-    if (threadIdx.x == 0) partial[((size_t)i * nrhs + col) * gridDim.x + blockIdx.x] = make_double2(rs[0], is[0]);
+}
+
+// norm[col].x = ||w(:, col)||^2, and scale[col], 1 or 0 for a column that runs or
+// not, becomes 1 / ||w(:, col)|| (0 where that vanishes); a warp each
+__global__ void __launch_bounds__(32) k_norm_scale(int nblk, const double* __restrict__ partial,
+                                                   double2* __restrict__ norm, double* __restrict__ scale) {
+    const int col = blockIdx.x;
+    double s = 0;
+    for (int b = threadIdx.x; b < nblk; b += 32) s += partial[(size_t)col * nblk + b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x) return;
+    norm[col] = make_double2(s, 0.0);
+    const double h = sqrt(s);
+    scale[col] = scale[col] != 0.0 && h > 1e-300 ? 1.0 / h : 0.0;
 }
 
 // Block dot products for the FP32 Arnoldi step: each CTA keeps its slice of
@@ -914,21 +935,18 @@ inline Cx divx(Cx a, Cx b) {
 static int col_norms(Ctx* c, int nrhs, const double2* w, double2* partial, double2* dred, std::vector<double2>& h,
                      std::vector<double>& out, cudaStream_t s) {
     k_mdot<<<dim3(GM_BLOCKS, nrhs, 1), 256, 0, s>>>(c->N, nrhs, nullptr, 0, w, partial);
-    k_reduce_partials<<<(nrhs + 127) / 128, 128, 0, s>>>(nrhs, partial, dred);
+    k_reduce_partials<<<nrhs, 32, 0, s>>>(partial, dred);
     CK(cudaMemcpyAsync(h.data(), dred, nrhs * sizeof(double2), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     for (int col = 0; col < nrhs; ++col) out[col] = std::sqrt(h[col].x);
     return MLF_OK;
 }
 
-static int col_norms32(Ctx* c, int nrhs, const float2* w, double2* partial, double2* dred, std::vector<double2>& h,
-                       std::vector<double>& out, cudaStream_t s) {
-    k_mdot32<<<dim3(GM_BLOCKS, nrhs, 1), 256, 0, s>>>(c->N, nrhs, nullptr, 0, w, partial);
-    k_reduce_partials<<<(nrhs + 127) / 128, 128, 0, s>>>(nrhs, partial, dred);
-    CK(cudaMemcpyAsync(h.data(), dred, nrhs * sizeof(double2), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    for (int col = 0; col < nrhs; ++col) out[col] = std::sqrt(h[col].x);
-    return MLF_OK;
+static void col_norms32(int N, int nrhs, const float2* w, double2* partial, double2* norm, double* scale, cudaStream_t s) {
+    const int nblk = (N + 256 * NRM_E - 1) / (256 * NRM_E);
+    double* p = reinterpret_cast<double*>(partial);
+    k_norm32<<<dim3(nblk, nrhs), 256, 0, s>>>(N, w, p);
+    k_norm_scale<<<nrhs, 32, 0, s>>>(nblk, p, norm, scale);
 }
 
 // FP64 M^-1 applied to the correction once per cycle
@@ -1108,6 +1126,8 @@ static int solve_mixed_t(Ctx* c, const double2* b, const double2* x0, double tol
             for (int col = 0; col < nrhs; ++col) any = any || live[col];
             if (!any) break;
             if (prof) cudaEventRecord(c->sev[0], s);
+            for (int col = 0; col < nrhs; ++col) scl[col] = live[col] ? 1.0 : 0.0;   // for k_norm_scale
+            CK(cudaMemcpyAsync(dscale, scl.data(), nrhs * sizeof(double), cudaMemcpyHostToDevice, s));
             const float2* vj;
             if (f32) {
                 vj = reinterpret_cast<const float2*>(V + (size_t)j * V1);
@@ -1159,15 +1179,20 @@ static int solve_mixed_t(Ctx* c, const double2* b, const double2* x0, double tol
                 k_reduce_partials_n<<<((j + 1) * nrhs + 127) / 128, 128, 0, s>>>((j + 1) * nrhs, md_chunks, partial,
                                                                                   dred);
                 k_gs_update32<BT><<<gc, 256, 0, s>>>(N, nrhs, j + 1, V, V1, ls, dred, w32);
-                CK(cudaMemcpyAsync(hbuf.data(), dred, (size_t)(j + 1) * nrhs * sizeof(double2), cudaMemcpyDeviceToHost, s));
+                // the last pass's sums and the norms come back together, after the next
+                // basis vector is on its way: one synchronisation a step
+                const bool last = pass + 1 == c->gs_passes;
+                if (last) {
+                    col_norms32(N, nrhs, w32, partial, dred + (size_t)(j + 1) * nrhs, dscale, s);
+                    k_colscale32<BT><<<gc, 256, 0, s>>>(N, w32, dscale, V + (size_t)(j + 1) * V1, ss);
+                }
+                CK(cudaMemcpyAsync(hbuf.data(), dred, (size_t)(j + 1 + last) * nrhs * sizeof(double2),
+                                   cudaMemcpyDeviceToHost, s));
                 CK(cudaStreamSynchronize(s));
                 for (size_t q = 0; q < (size_t)(j + 1) * nrhs; ++q) { hsum[q].x += hbuf[q].x; hsum[q].y += hbuf[q].y; }
             }
             std::vector<double> hn(nrhs);
-            if ((st = col_norms32(c, nrhs, w32, partial, dred, hbuf, hn, s))) break;
-            for (int col = 0; col < nrhs; ++col) scl[col] = (live[col] && hn[col] > 1e-300) ? 1.0 / hn[col] : 0.0;
-            CK(cudaMemcpyAsync(dscale, scl.data(), nrhs * sizeof(double), cudaMemcpyHostToDevice, s));
-            k_colscale32<BT><<<gc, 256, 0, s>>>(N, w32, dscale, V + (size_t)(j + 1) * V1, ss);
+            for (int col = 0; col < nrhs; ++col) hn[col] = std::sqrt(hbuf[(size_t)(j + 1) * nrhs + col].x);
             if (prof) {
                 cudaEventRecord(c->sev[3], s);
                 cudaEventSynchronize(c->sev[3]);
