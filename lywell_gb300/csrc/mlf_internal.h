@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/lywell_mlfma.h"
+#include "mlf_split64.h"
 
 namespace mlf {
 
@@ -177,7 +178,7 @@ struct Ctx {
     int *doz_pat = nullptr, *doz_exp = nullptr;
     int noz_tiles = 0, nsm = 0;
     double2* doz_ws = nullptr;
-    size_t oz_cap = 0;
+    OzSizes oz_cap;                   // of doz_ws and doz_exp
     // device geometry for set-up kernels and RCS
     double *dp_coord = nullptr, *dt_baric = nullptr, *dt_baric_sub = nullptr, *de_long = nullptr,
            *de_centro = nullptr;

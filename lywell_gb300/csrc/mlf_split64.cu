@@ -49,7 +49,6 @@ namespace mlf {
 
 constexpr int OZ_D = 8;            // digits
 constexpr int OZ_R = 64;           // rows (bases of one box) per CTA
-constexpr int OZ_C = 12;           // complex columns per CTA
 constexpr int OZ_K = 32;           // bases of S per step: 64 real terms
 constexpr int OZ_PITCH = 4 * OZ_K + 16;                    // bytes of a row of 64 FP16, padded: ldmatrix without conflicts
 constexpr int OZ_ABYTES = OZ_D * OZ_R * OZ_PITCH;          // Z digits  [digit][row][term]
@@ -60,7 +59,6 @@ constexpr int OZ_WARPS = 12;       // 4 tiles of 16 rows x 3 of 8 real columns
 constexpr int OZ_THREADS = 32 * OZ_WARPS;
 constexpr int OZ_WR = (OZ_R + OZ_WARPS - 1) / OZ_WARPS;   // rows that a warp converts
 static_assert(OZ_C == OZ_WARPS && 2 * OZ_C == 8 * (OZ_WARPS / 4), "a warp converts one column and multiplies one tile");
-constexpr int OZ_MAX_SPLIT = 4, OZ_MAX_DENSE_SPLIT = 8;
 
 // |v| < 2^e to an integer below 2^62, truncated: v = m 2^(e - 62)
 __device__ __forceinline__ long long oz_fix(unsigned long long m62, int t, uint32_t sign) {
@@ -437,25 +435,22 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
     }
 }
 
-// Parts of the terms: enough CTAs for about four waves of one per SM
-static int near64_split(const Ctx* c, int nrhs) {
-    const int ctas = c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C);
-    return std::max(1, std::min(c->dense ? OZ_MAX_DENSE_SPLIT : OZ_MAX_SPLIT, (4 * c->nsm + ctas - 1) / ctas));
-}
+static int near64_split(const Ctx* c, int nrhs) { return oz_split(c->noz_tiles, c->nsm, nrhs, c->dense); }
 
-// workspace for blocks of up to nrhs columns, with `ints` exponents beside it
-static int oz_workspace(Ctx* c, int nrhs, size_t ints) {
-    size_t need = 0;
-    for (int n = 2; n <= nrhs; ++n) need = std::max(need, (size_t)near64_split(c, n) * n * c->N);
-    if (c->oz_cap >= need) return MLF_OK;
+// workspace for blocks of up to nrhs columns, with `fixed` exponents beside it and
+// `per_col` more a column
+static int oz_workspace(Ctx* c, int nrhs, size_t fixed, size_t per_col) {
+    const OzSizes need = oz_sizes(c->noz_tiles, c->nsm, c->N, c->dense, fixed, per_col, nrhs);
+    if (!oz_short(c->oz_cap, need)) return MLF_OK;
     if (c->doz_ws) cudaFree(c->doz_ws);
     if (c->doz_exp) cudaFree(c->doz_exp);
     c->doz_ws = nullptr;
     c->doz_exp = nullptr;
-    c->oz_cap = 0;
-    CK(cudaMalloc(&c->doz_ws, need * sizeof(double2)));
-    CK(cudaMalloc(&c->doz_exp, ints * sizeof(int)));
-    c->oz_cap = need;
+    const OzSizes grown{std::max(c->oz_cap.sums, need.sums), std::max(c->oz_cap.exps, need.exps)};
+    c->oz_cap = OzSizes();
+    CK(cudaMalloc(&c->doz_ws, grown.sums * sizeof(double2)));
+    CK(cudaMalloc(&c->doz_exp, grown.exps * sizeof(int)));
+    c->oz_cap = grown;
     return MLF_OK;
 }
 
@@ -498,7 +493,7 @@ int split64_ready(Ctx* c, int nrhs) {
         c->doz_tiles = d;
         c->noz_tiles = (int)t.size();
     }
-    return oz_workspace(c, nrhs, 2 * (size_t)c->N + nb * nrhs);
+    return oz_workspace(c, nrhs, 2 * (size_t)c->N, nb);
 }
 
 static OzArgs oz_args(const Ctx* c, int nrhs, int ld) {
@@ -560,7 +555,7 @@ static int dense64_ready(Ctx* c, int nrhs) {
         }
         c->doz_pat = p;
     }
-    return oz_workspace(c, nrhs, 2 * (size_t)N + nblk + nrhs);
+    return oz_workspace(c, nrhs, 2 * (size_t)N + nblk, 1);
 }
 
 int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
