@@ -92,13 +92,17 @@ __device__ __forceinline__ int oz_exp(double2 v) {
     return ef == 0x7ff ? OZ_BAD : max(ef, 1) - 1022;   // zeros count as the smallest number
 }
 
-// sexp[n] = exponent of x's row n over the columns
+// sexp[n] = exponent of x's row n over the columns where it is finite (a column
+// that is not is marked by its own exponent; its entries tell the others nothing)
 __global__ void k_row_exp(int N, int nrhs, int ld, const double2* __restrict__ x, int* __restrict__ sexp) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
     int e = OZ_ZERO;
-    for (int c = 0; c < nrhs; ++c) e = max(e, oz_exp(x[(size_t)c * ld + n]));
-    sexp[n] = e == OZ_BAD ? 0 : e;
+    for (int c = 0; c < nrhs; ++c) {
+        const int v = oz_exp(x[(size_t)c * ld + n]);
+        if (v != OZ_BAD) e = max(e, v);
+    }
+    sexp[n] = e == OZ_ZERO ? 0 : e;   // in no column
 }
 
 // rexp[pos] = exponent of row perm[pos] of Z 2^sexp; a warp per row

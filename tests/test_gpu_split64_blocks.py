@@ -33,3 +33,18 @@ def test_smaller_block_first(kind, gpu_lib):
     for n, y in zip(sizes, after):
         with _body(kind) as m:
             assert np.array_equal(m.matvec(X[:, :n]), y)
+
+
+@pytest.mark.parametrize("kind", ["spheroid4", "dense"])
+@pytest.mark.parametrize("size", [1e-12, 1e15])
+def test_finite_columns_beside_a_nan(kind, size, gpu_lib):
+    """Columns of another magnitude than one beside a column with a NaN.  Against the
+    columns alone: both sides round, sums of up to 3000 terms, 1e-13 of the norm."""
+    with _body(kind) as m:
+        X = size * _columns(m.N, 14, 11)
+        X[m.N // 3, 2] = np.nan
+        Y = m.matvec(X)
+        assert np.isnan(Y[:, 2]).any()
+        for c in (0, 3, 13):
+            ref = m.matvec(X[:, c])
+            assert np.linalg.norm(Y[:, c] - ref) < 1e-13 * np.linalg.norm(ref)
