@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "mlf_internal.h"
+#include "mlf_fma64.cuh"
 #include "mlf_sep.cuh"
 #include "mlf_zmn.cuh"
 
@@ -64,13 +65,6 @@ static int upload(Ctx* c, T** dst, const std::vector<T>& v) {
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ void cmac(double2& acc, double2 a, double2 b) {
-    acc.x = fma(a.x, b.x, acc.x);
-    acc.x = fma(-a.y, b.y, acc.x);
-    acc.y = fma(a.x, b.y, acc.y);
-    acc.y = fma(a.y, b.x, acc.y);
-}
-
 // ---------------------------------------------------------------------------
 // set-up kernels
 // ---------------------------------------------------------------------------
@@ -183,11 +177,8 @@ __global__ void k_aggregate(int K, int nrhs, int ld, const int* __restrict__ box
     const int b = blockIdx.x / nrhs, r = blockIdx.x % nrhs;
     const int j0 = box_ptr[b], j1 = box_ptr[b + 1];
     const double2* xr = x + (size_t)r * ld;
-    for (int q = threadIdx.x; q < 2 * K; q += blockDim.x) {
-        double2 acc = make_double2(0, 0);
-        for (int j = j0; j < j1; ++j) cmac(acc, R[(size_t)j * 2 * K + q], xr[perm[j]]);
-        C[((size_t)b * nrhs + r) * 2 * K + q] = acc;
-    }
+    for (int q = threadIdx.x; q < 2 * K; q += blockDim.x)
+        C[((size_t)b * nrhs + r) * 2 * K + q] = aggregate_direction(2 * K, j0, j1, q, perm, R, xr);
 }
 
 // One level of the translation; its CTAs follow block0, (box*nrhs + r)*nchunk + chunk
@@ -249,30 +240,9 @@ __global__ void k_receive_near_d(int K, int N, int nrhs, int ld, const int* __re
     if (gw >= N * nrhs) return;
     const int j = gw / nrhs, r = gw % nrhs;
     const int n = perm[j], b = box_of_sorted[j];
-    const double2* Rj = R + (size_t)j * 2 * K;
-    const double2* Ab = A + ((size_t)b * nrhs + r) * 2 * K;
-    double sr = 0, si = 0;
-    for (int q = lane; q < 2 * K; q += 32) {
-        const double2 a = Rj[q], v = Ab[q];
-        sr = fma(a.x, v.x, sr); sr = fma(a.y, v.y, sr);
-        si = fma(a.x, v.y, si); si = fma(-a.y, v.x, si);
-    }
-    const double2* xr = x + (size_t)r * ld;
-    double nr = 0, ni = 0;
-    for (int q = ia[n] + lane; q < ia[n + 1]; q += 32) {
-        const double2 z = Zd[q];
-        const double2 xv = xr[ja[q]];
-        nr = fma(xv.x, z.x, nr); nr = fma(-xv.y, z.y, nr);
-        ni = fma(xv.x, z.y, ni); ni = fma(xv.y, z.x, ni);
-    }
-    // combine before the reduction: t = j*facy*s + near
-    double tr = fma(-facy, si, nr), ti = fma(facy, sr, ni);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        tr += __shfl_xor_sync(0xffffffff, tr, o);
-        ti += __shfl_xor_sync(0xffffffff, ti, o);
-    }
-    if (lane == 0) y[(size_t)r * ld + n] = make_double2(tr, ti);
+    const double2 t = receive_near_row(2 * K, n, R + (size_t)j * 2 * K, A + ((size_t)b * nrhs + r) * 2 * K, ia, ja, Zd,
+                                       x + (size_t)r * ld, facy);
+    if (lane == 0) y[(size_t)r * ld + n] = t;
 }
 
 __global__ void k_f2d(size_t n, const float2* __restrict__ a, double2* __restrict__ b) {

@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "mlf_internal.h"
+#include "mlf_fma64.cuh"
 #include "mlf_zmn.cuh"
 
 namespace mlf {
@@ -42,20 +43,8 @@ __global__ void k_mom_gemv(int N, int ld, const double2* __restrict__ Z, const d
     const int lane = threadIdx.x & 31;
     if (gw >= N) return;
     const int m = (int)gw;
-    const double2* zr = Z + (size_t)m * N;
-    double ar = 0, ai = 0;
-#pragma unroll 4
-    for (int n = lane; n < N; n += 32) {
-        const double2 z = zr[n], v = x[n];
-        ar = fma(z.x, v.x, ar); ar = fma(-z.y, v.y, ar);
-        ai = fma(z.x, v.y, ai); ai = fma(z.y, v.x, ai);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ar += __shfl_xor_sync(0xffffffff, ar, o);
-        ai += __shfl_xor_sync(0xffffffff, ai, o);
-    }
-    if (lane == 0) y[m] = make_double2(ar, ai);
+    const double2 t = dense_row(N, Z + (size_t)m * N, x);
+    if (lane == 0) y[m] = t;
 }
 
 int dense_setup(Ctx* c) {

@@ -17,20 +17,30 @@
 // [-128, 127] of weight 2^(8 (7 - i)).  The 36 digit products with i + j <= 7
 // are summed per s = i + j in FP32 over 64 real terms: at most 8 * 64 * 2^14 =
 // 2^23, exact; then the eight sums are joined in 64-bit integers over all terms,
-// and rounded to double once at the end.  In the near field each source k is
-// scaled by a power of two before that: x_k to magnitude one (over the block's
-// columns), Z's column k by the inverse, so that a row's integers are relative
-// to its largest term |Z_mk x_k|: what is lost lies below 2^-62 of that, whatever
-// the range of x or Z, where a sum in double precision loses 2^-53 of its
-// partial sums.  Measured on a 7680-unknown list against extended precision:
-// relative error 1.8e-16 (rms over rows), 1.7e-15 with FP64 FMAs; the same with
-// x over six decades.
+// and rounded to double once at the end.  What is left out, the products with
+// i + j >= 8 foremost, is under 2^-59 a real term (typically 2^-62, of either sign)
+// of the bound 2^(er + ec) on the row's and column's largest product.  In the near
+// field (and the dense operator) each source k is scaled by a power of two before
+// that: x_k to magnitude one (over the block's columns), Z's column k by the
+// inverse, so that the bound is near the row's largest term |Z_mk x_k| also where
+// x varies over decades.
+//
+// A column that varies otherwise than its neighbours, or a row whose large entries
+// meet small ones of x, can have terms far below that bound.  So each value is
+// checked: the top digits' magnitudes are multiplied too (a 37th product), and
+// their sum says how large the value's terms are.  A value whose terms' sum is not
+// surely 2^-6 of the bound (OZ_COVER) or more, or whose row or column has an Inf
+// or a NaN, is computed again in FP64 FMAs (mlf_fma64.cuh): what stands beside a
+// column costs time, not digits.
+// Error against extended precision over the terms' sum, rms (dense operator of 1920
+// unknowns, FMAs -> here): Gaussian columns 7.7e-17 -> 2.4e-17; a column over two
+// decades beside them 9.4e-17 -> 5.8e-17 with 21 % of the values computed again, over
+// six decades 1.0e-16 -> 9.0e-17 with 68 %.  Of the spheroid's product below, one
+// value in 288000 is.
 //
 // mma.sync keeps each digit sum in the registers of the warp that joins it.
-// 12000-RWG spheroid (49 M near entries), 24 columns, before -> now: near +
-// receive 8.66 -> 1.66 ms, aggregation 1.00 -> 0.18 ms.
-//
-// A row or column with an Inf or a NaN gives NaN in its results.
+// 12000-RWG spheroid (49 M near entries), 24 columns: the whole product 9.77 ms with
+// FMAs, 1.95 ms without the check, 2.02 ms with it.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -39,6 +49,7 @@
 #include <vector>
 
 #include "mlf_internal.h"
+#include "mlf_fma64.cuh"
 
 namespace mlf {
 
@@ -81,6 +92,9 @@ __device__ __forceinline__ long long oz_fix(double v, int e) {
 // exponent e with |v| < 2^e of the larger of two magnitudes, OZ_ZERO for zeros,
 // OZ_BAD for an Inf or a NaN
 constexpr int OZ_ZERO = -100000, OZ_BAD = 100000;
+// With others added or taken off: of a sum, and its mark for the check below
+__device__ __forceinline__ bool oz_zero(int e) { return e < OZ_ZERO / 2; }
+__device__ __forceinline__ bool oz_bad(int e) { return e > OZ_BAD / 2; }
 __device__ __forceinline__ int oz_exp(float2 v) {
     const uint32_t m = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
     const int ef = (int)(m >> 23);
@@ -89,20 +103,24 @@ __device__ __forceinline__ int oz_exp(float2 v) {
 __device__ __forceinline__ int oz_exp(double2 v) {
     const uint32_t m = max((uint32_t)__double2hiint(v.x) & 0x7fffffffu, (uint32_t)__double2hiint(v.y) & 0x7fffffffu);
     const int ef = (int)(m >> 20);
-    return ef == 0x7ff ? OZ_BAD : max(ef, 1) - 1022;   // zeros count as the smallest number
+    if (m == 0 && (__double2loint(v.x) | __double2loint(v.y)) == 0) return OZ_ZERO;
+    return ef == 0x7ff ? OZ_BAD : max(ef, 1) - 1022;
 }
 
 // sexp[n] = exponent of x's row n over the columns where it is finite (a column
-// that is not is marked by its own exponent; its entries tell the others nothing)
-__global__ void k_row_exp(int N, int nrhs, int ld, const double2* __restrict__ x, int* __restrict__ sexp) {
+// that is not is marked by its own exponent; its entries tell the others nothing),
+// the smallest number's where it is zero; *nredo = 0
+__global__ void k_row_exp(int N, int nrhs, int ld, const double2* __restrict__ x, int* __restrict__ sexp,
+                          int* __restrict__ nredo) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
+    if (n == 0) *nredo = 0;
     int e = OZ_ZERO;
     for (int c = 0; c < nrhs; ++c) {
         const int v = oz_exp(x[(size_t)c * ld + n]);
         if (v != OZ_BAD) e = max(e, v);
     }
-    sexp[n] = e == OZ_ZERO ? 0 : e;   // in no column
+    sexp[n] = max(e, -1021);
 }
 
 // rexp[pos] = exponent of row perm[pos] of Z 2^sexp; a warp per row
@@ -126,10 +144,13 @@ enum { OZ_NEAR = 0, OZ_RECEIVE = 1, OZ_AGGREGATE = 2, OZ_DENSE = 3 };
 template <int MODE>
 __global__ void k_col_exp(int nrhs, int ld, int K2, const int* __restrict__ box_ptr, const int* __restrict__ perm,
                           const int* __restrict__ ia, const int* __restrict__ ja, const double2* __restrict__ x,
-                          const int* __restrict__ sexp, int* __restrict__ cexp) {
+                          const int* __restrict__ sexp, int* __restrict__ cexp, int* __restrict__ redo) {
     const int b = blockIdx.x / nrhs, c = blockIdx.x % nrhs;
     __shared__ int top;
-    if (threadIdx.x == 0) top = OZ_ZERO;
+    if (threadIdx.x == 0) {
+        top = OZ_ZERO;
+        if (MODE == OZ_AGGREGATE) redo[blockIdx.x] = 0;
+    }
     __syncthreads();
     int e = OZ_ZERO;
     if (MODE == OZ_NEAR) {
@@ -244,18 +265,84 @@ __global__ void k_set_int(int n, int v, int* __restrict__ a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = v;
 }
+// The check of a value: cover = sum over the real terms of its two parts of the
+// product of the top digits' magnitudes, parts of the terms added up.  A top digit
+// d stands for a magnitude of (|d| - 0.51) 2^-6 or more of its operand's bound, so a
+// cover of 512 surely means complex terms of 512 / 2 / 4 * 2^-12 = 2^-6 of the value's
+// bound in sum (a part that is small beside the other is off by what that one allows).
+constexpr float OZ_COVER = 512.f, OZ_SURE = 1e30f;
+__device__ __forceinline__ float oz_cover(float c, int er, int ec) {
+    if (oz_bad(er) || oz_bad(ec)) return -OZ_SURE;
+    return oz_zero(er) || oz_zero(ec) ? OZ_SURE : c;   // exactly zero
+}
+
+// list[(*n)++] = v of each active lane
+__device__ __forceinline__ void oz_append(int* n, unsigned* list, unsigned v) {
+    const unsigned on = __activemask(), lane = threadIdx.x & 31;
+    const int first = __ffs(on) - 1;
+    int base = 0;
+    if ((int)lane == first) base = atomicAdd(n, __popc(on));
+    base = __shfl_sync(on, base, first);
+    list[base + __popc(on & ((1u << lane) - 1))] = v;
+}
+
 // y = sum of the parts, in order
 __global__ void k_sum_parts(int N, int nrhs, int ld, int nsplit, const double2* __restrict__ ws,
-                            double2* __restrict__ y) {
+                            const float* __restrict__ cov, double2* __restrict__ y, int* __restrict__ nredo,
+                            unsigned* __restrict__ redo) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (i >= N) return;
     double2 t = make_double2(0, 0);
+    float g = 0.f;
     for (int p = 0; p < nsplit; ++p) {
-        const double2 v = ws[((size_t)p * nrhs + c) * N + i];
+        const size_t at = ((size_t)p * nrhs + c) * N + i;
+        const double2 v = ws[at];
         t.x += v.x;
         t.y += v.y;
+        g += cov[at];
     }
     y[(size_t)c * ld + i] = t;
+    if (g < OZ_COVER) oz_append(nredo, redo, (unsigned)c * N + i);
+}
+
+// Values computed again in FMAs.  Leaf fields: CTA (box, column), where one of its
+// directions asks for it
+__global__ void k_redo_aggregate(int K2, int nrhs, int ld, const int* __restrict__ redo,
+                                 const int* __restrict__ box_ptr, const int* __restrict__ perm,
+                                 const double2* __restrict__ R, const double2* __restrict__ x, double2* __restrict__ C) {
+    if (!redo[blockIdx.x]) return;
+    const int b = blockIdx.x / nrhs, r = blockIdx.x % nrhs;
+    for (int q = threadIdx.x; q < K2; q += blockDim.x)
+        C[(size_t)blockIdx.x * K2 + q] =
+            aggregate_direction(K2, box_ptr[b], box_ptr[b + 1], q, perm, R, x + (size_t)r * ld);
+}
+// y of the listed (column, box-sorted basis), a warp each
+__global__ void __launch_bounds__(256) k_redo_receive_near(int K2, int N, int nrhs, int ld, const int* __restrict__ nredo,
+                                                           const unsigned* __restrict__ redo,
+                                                           const int* __restrict__ perm,
+                                                           const int* __restrict__ box_of_sorted,
+                                                           const double2* __restrict__ R, const double2* __restrict__ A,
+                                                           const int* __restrict__ ia, const int* __restrict__ ja,
+                                                           const double2* __restrict__ Zd, const double2* __restrict__ x,
+                                                           double facy, double2* __restrict__ y) {
+    const int n = *nredo;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += gridDim.x * (blockDim.x >> 5)) {
+        const int r = redo[k] / N, j = redo[k] % N, i = perm[j];
+        const double2 t = receive_near_row(K2, i, R + (size_t)j * K2, A + ((size_t)box_of_sorted[j] * nrhs + r) * K2, ia,
+                                           ja, Zd, x + (size_t)r * ld, facy);
+        if ((threadIdx.x & 31) == 0) y[(size_t)r * ld + i] = t;
+    }
+}
+// y of the listed (column, row) of the dense operator, a warp each
+__global__ void __launch_bounds__(256) k_redo_dense(int N, int ld, const int* __restrict__ nredo,
+                                                    const unsigned* __restrict__ redo, const double2* __restrict__ Z,
+                                                    const double2* __restrict__ x, double2* __restrict__ y) {
+    const int n = *nredo;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += gridDim.x * (blockDim.x >> 5)) {
+        const int r = redo[k] / N, i = redo[k] % N;
+        const double2 t = dense_row(N, Z + (size_t)i * N, x + (size_t)r * ld);
+        if ((threadIdx.x & 31) == 0) y[(size_t)r * ld + i] = t;
+    }
 }
 
 struct OzArgs {
@@ -267,6 +354,10 @@ struct OzArgs {
     const int *sexp, *rexp, *cexp;      // exponents of sources (near), rows and columns
     double2* out;                       // near: [split][col][box-sorted place]; receive: y; aggregate: the field C
     const double2* near;                // receive: the near field's parts
+    float* cov;                        // near: the parts' covers, as out (receive: read)
+    int* nredo;                         // receive: values to compute again, and their list
+    unsigned* redo;
+    int* redo_box;                      // aggregate: (box, column) to compute again
     int nsplit;
     double facy;
 };
@@ -360,6 +451,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
     const uint32_t b_addr = base + OZ_ABYTES + (lane >> 4) * (2 * OZ_C * OZ_PITCH) +
                             (nt * 8 + (lane & 7)) * OZ_PITCH + ((lane >> 3) & 1) * 16;
     long long hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0};
+    float cover[4] = {0.f, 0.f, 0.f, 0.f};
     auto products = [&](uint32_t off) {
         float acc[OZ_D][4];
 #pragma unroll
@@ -375,6 +467,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
             for (int i = 0; i < OZ_D; ++i) {
                 uint32_t a[4];
                 ldsm4(a, a_addr + off + i * (OZ_R * OZ_PITCH) + ks * 32);
+                if (i == 0) {   // the top digits' magnitudes
+                    constexpr uint32_t M = 0x7fff7fffu;
+                    const uint32_t m[4] = {a[0] & M, a[1] & M, a[2] & M, a[3] & M};
+                    mma_f16(cover, m, b[0][0] & M, b[0][1] & M);
+                }
 #pragma unroll
                 for (int j = 0; i + j < OZ_D; ++j)
                     mma_f16(acc[i + j], a, b[j / 2][2 * (j & 1)], b[j / 2][2 * (j & 1) + 1]);
@@ -413,7 +510,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
         if (!((warp >> 2) & 1)) next();
     }
     if (!mine) return;
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
     const int cc = nt * 4 + (lane & 3);
     if (cc >= nc) return;
 #pragma unroll
@@ -422,22 +518,34 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
         if (row >= nr) continue;
         const int e = er[row], f = ec[cc];
         double2 v = make_double2(oz_value(hi[2 * h], lo[2 * h], e, f), oz_value(hi[2 * h + 1], lo[2 * h + 1], e, f));
-        if (e > OZ_BAD / 2 || f > OZ_BAD / 2) v = make_double2(nan, nan);
+        const float cv = oz_cover(cover[2 * h] + cover[2 * h + 1], e, f);
         if (MODE == OZ_NEAR || MODE == OZ_DENSE) {
-            g.out[((size_t)blockIdx.y * g.nrhs + c0 + cc) * g.N + p0 + row] = v;
+            const size_t at = ((size_t)blockIdx.y * g.nrhs + c0 + cc) * g.N + p0 + row;
+            g.out[at] = v;
+            g.cov[at] = cv;
         } else if (MODE == OZ_AGGREGATE) {
             g.out[((size_t)tl.x * g.nrhs + c0 + cc) * g.K2 + tl.y + row] = v;
+            if (cv < OZ_COVER) g.redo_box[(size_t)tl.x * g.nrhs + c0 + cc] = 1;
         } else {   // y = j facy v + near
             double2 w = make_double2(0, 0);
+            float cn = 0.f;
             for (int p = 0; p < g.nsplit; ++p) {
-                const double2 t = g.near[((size_t)p * g.nrhs + c0 + cc) * g.N + p0 + row];
+                const size_t at = ((size_t)p * g.nrhs + c0 + cc) * g.N + p0 + row;
+                const double2 t = g.near[at];
                 w.x += t.x;
                 w.y += t.y;
+                cn += g.cov[at];
             }
             g.out[(size_t)(c0 + cc) * g.ld + g.perm[p0 + row]] = make_double2(fma(-g.facy, v.y, w.x), fma(g.facy, v.x, w.y));
+            if (cv < OZ_COVER || cn < OZ_COVER) oz_append(g.nredo, g.redo, (unsigned)(c0 + cc) * g.N + p0 + row);
         }
     }
 }
+
+static float* oz_covers(const Ctx* c) { return reinterpret_cast<float*>(c->doz_ws + c->oz_cap.sums); }
+
+// CTAs of 256 threads that go through a list of values to compute again
+constexpr int OZ_REDO_CTAS = 8;   // per SM
 
 static int near64_split(const Ctx* c, int nrhs) { return oz_split(c->noz_tiles, c->nsm, nrhs, c->dense); }
 
@@ -452,7 +560,7 @@ static int oz_workspace(Ctx* c, int nrhs, size_t fixed, size_t per_col) {
     c->doz_exp = nullptr;
     const OzSizes grown{std::max(c->oz_cap.sums, need.sums), std::max(c->oz_cap.exps, need.exps)};
     c->oz_cap = OzSizes();
-    CK(cudaMalloc(&c->doz_ws, grown.sums * sizeof(double2)));
+    CK(cudaMalloc(&c->doz_ws, grown.sums * (sizeof(double2) + sizeof(float))));   // sums, then covers
     CK(cudaMalloc(&c->doz_exp, grown.exps * sizeof(int)));
     c->oz_cap = grown;
     return MLF_OK;
@@ -497,7 +605,7 @@ int split64_ready(Ctx* c, int nrhs) {
         c->doz_tiles = d;
         c->noz_tiles = (int)t.size();
     }
-    return oz_workspace(c, nrhs, 2 * (size_t)c->N, nb);
+    return oz_workspace(c, nrhs, 2 * (size_t)c->N + 1, 2 * nb + c->N);
 }
 
 static OzArgs oz_args(const Ctx* c, int nrhs, int ld) {
@@ -509,15 +617,34 @@ static OzArgs oz_args(const Ctx* c, int nrhs, int ld) {
     return g;
 }
 
+// The parts of doz_exp: exponents of sources, rows and columns, values to compute
+// again (a flag a box and column, and a list with its length)
+struct OzExps {
+    int *sexp, *rexp, *nredo, *cexp, *redo_box;
+    unsigned* redo;
+};
+static OzExps oz_exps(const Ctx* c, size_t nb, int nrhs) {
+    OzExps e;
+    e.sexp = c->doz_exp;
+    e.rexp = e.sexp + c->N;
+    e.nredo = e.rexp + c->N;
+    e.cexp = e.nredo + 1;
+    e.redo_box = e.cexp + nb * nrhs;
+    e.redo = reinterpret_cast<unsigned*>(e.redo_box + nb * nrhs);
+    return e;
+}
+
 // C (leaf fields) = R^T x
 int split64_aggregate(Ctx* c, const double2* x, int nrhs, int ld, double2* C, cudaStream_t s) {
     const int nb = (int)c->box_ptr.size() - 1;
     OzArgs g = oz_args(c, nrhs, ld);
-    int* cexp = c->doz_exp + 2 * (size_t)c->N;
-    k_col_exp<OZ_AGGREGATE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, nullptr, cexp);
-    g.x = x; g.rexp = c->doz_pat + c->N; g.cexp = cexp; g.out = C;
+    const OzExps e = oz_exps(c, nb, nrhs);
+    k_col_exp<OZ_AGGREGATE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, nullptr, e.cexp,
+                                                      e.redo_box);
+    g.x = x; g.rexp = c->doz_pat + c->N; g.cexp = e.cexp; g.out = C; g.redo_box = e.redo_box;
     k_split64<OZ_AGGREGATE><<<(unsigned)((size_t)nb * ((g.K2 + OZ_R - 1) / OZ_R) * ((nrhs + OZ_C - 1) / OZ_C)), OZ_THREADS,
                               OZ_SMEM, s>>>(g);
+    k_redo_aggregate<<<nb * nrhs, 256, 0, s>>>(g.K2, nrhs, ld, e.redo_box, g.box_ptr, g.perm, g.R, x, C);
     return cuda_ok(c, cudaGetLastError(), "aggregation (split)") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -526,16 +653,21 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
                          cudaStream_t s) {
     const int nb = (int)c->box_ptr.size() - 1, ncb = (nrhs + OZ_C - 1) / OZ_C;
     OzArgs g = oz_args(c, nrhs, ld);
-    int *sexp = c->doz_exp, *rexp = sexp + c->N, *cexp = rexp + c->N;
-    k_row_exp<<<(c->N + 255) / 256, 256, 0, s>>>(c->N, nrhs, ld, x, sexp);
-    k_near_exp<<<(c->N + 7) / 8, 256, 0, s>>>(c->N, c->dperm, c->dia, c->dja, c->dZ, sexp, rexp);
-    k_col_exp<OZ_NEAR><<<nb * nrhs, 256, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, sexp, cexp);
+    const OzExps e = oz_exps(c, nb, nrhs);
+    k_row_exp<<<(c->N + 255) / 256, 256, 0, s>>>(c->N, nrhs, ld, x, e.sexp, e.nredo);
+    k_near_exp<<<(c->N + 7) / 8, 256, 0, s>>>(c->N, c->dperm, c->dia, c->dja, c->dZ, e.sexp, e.rexp);
+    k_col_exp<OZ_NEAR><<<nb * nrhs, 256, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, e.sexp, e.cexp,
+                                                 nullptr);
     const int nsplit = near64_split(c, nrhs);
-    g.x = x; g.sexp = sexp; g.rexp = rexp; g.cexp = cexp; g.out = c->doz_ws;
+    g.x = x; g.sexp = e.sexp; g.rexp = e.rexp; g.cexp = e.cexp; g.out = c->doz_ws; g.cov = oz_covers(c);
     k_split64<OZ_NEAR><<<dim3(ncb * c->noz_tiles, nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
-    k_col_exp<OZ_RECEIVE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, A, nullptr, cexp);
+    k_col_exp<OZ_RECEIVE><<<nb * nrhs, 128, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, A, nullptr, e.cexp,
+                                                    nullptr);
     g.x = A; g.rexp = c->doz_pat; g.out = y; g.near = c->doz_ws; g.nsplit = nsplit; g.facy = facy;
+    g.nredo = e.nredo; g.redo = e.redo;
     k_split64<OZ_RECEIVE><<<ncb * c->noz_tiles, OZ_THREADS, OZ_SMEM, s>>>(g);
+    k_redo_receive_near<<<OZ_REDO_CTAS * c->nsm, 256, 0, s>>>(g.K2, c->N, nrhs, ld, e.nredo, e.redo, g.perm,
+                                                              c->dbox_of_sorted, g.R, A, g.ia, g.ja, c->dZd, x, facy, y);
     return cuda_ok(c, cudaGetLastError(), "near + receive (split)") ? MLF_OK : MLF_E_CUDA;
 }
 
@@ -559,15 +691,16 @@ static int dense64_ready(Ctx* c, int nrhs) {
         }
         c->doz_pat = p;
     }
-    return oz_workspace(c, nrhs, 2 * (size_t)N + nblk, 1);
+    return oz_workspace(c, nrhs, 2 * (size_t)N + 1 + nblk, 1 + (size_t)N);
 }
 
 int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
     int st;
     if ((st = dense64_ready(c, nrhs))) return st;
     const int N = c->N, nblk = (N + 31) / 32, nsplit = near64_split(c, nrhs);
-    int *sexp = c->doz_exp, *rexp = sexp + N, *bmax = rexp + N, *cexp = bmax + nblk;
-    k_row_exp<<<(N + 255) / 256, 256, 0, s>>>(N, nrhs, ld, x, sexp);
+    int *sexp = c->doz_exp, *rexp = sexp + N, *nredo = rexp + N, *bmax = nredo + 1, *cexp = bmax + nblk;
+    unsigned* redo = reinterpret_cast<unsigned*>(cexp + nrhs);
+    k_row_exp<<<(N + 255) / 256, 256, 0, s>>>(N, nrhs, ld, x, sexp, nredo);
     k_set_int<<<(nrhs + 255) / 256, 256, 0, s>>>(nrhs, OZ_ZERO, cexp);
     k_dense_col_exp<<<std::min((nblk + 7) / 8, 256), 256, 0, s>>>(N, nrhs, ld, nblk, x, sexp, bmax, cexp);
     k_dense_row_exp<<<(N + 7) / 8, 256, 0, s>>>(N, nblk, reinterpret_cast<const short*>(c->doz_pat), bmax, rexp);
@@ -575,9 +708,11 @@ int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaS
     g.N = N; g.nrhs = nrhs; g.ld = ld; g.K2 = 1;
     g.R = c->dZdense; g.x = x;
     g.sexp = sexp; g.rexp = rexp; g.cexp = cexp;
-    g.out = c->doz_ws;
+    g.out = c->doz_ws; g.cov = oz_covers(c);
     k_split64<OZ_DENSE><<<dim3((unsigned)c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C), nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
-    k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, y);
+    k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, g.cov, y, nredo,
+                                                               redo);
+    k_redo_dense<<<OZ_REDO_CTAS * c->nsm, 256, 0, s>>>(N, ld, nredo, redo, c->dZdense, x, y);
     return cuda_ok(c, cudaGetLastError(), "dense matvec (split)") ? MLF_OK : MLF_E_CUDA;
 }
 

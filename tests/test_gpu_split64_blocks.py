@@ -48,3 +48,43 @@ def test_finite_columns_beside_a_nan(kind, size, gpu_lib):
         for c in (0, 3, 13):
             ref = m.matvec(X[:, c])
             assert np.linalg.norm(Y[:, c] - ref) < 1e-13 * np.linalg.norm(ref)
+
+
+def _neighbours(m, kind):
+    """Columns whose ranges differ: flat, over twelve decades along the body (up and
+    down), unit vectors, spikes."""
+    X = _columns(m.N, 14, 12)
+    along = np.linspace(0.0, 12.0, m.N)
+    X[:, 1] *= 10.0 ** along
+    X[:, 2] *= 10.0 ** -along
+    X[:, 3] = 0
+    X[m.N // 2, 3] = 1.0
+    X[:, 4] = 0
+    X[m.N // 2 + 1, 4] = 1e-9j
+    X[::97, 5] *= 1e12
+    X[::89, 6] *= 1e-12
+    X[:, 7] = X[:, 7].real
+    X[:, 8] *= 1e-120
+    return X
+
+
+@pytest.mark.parametrize("kind", ["spheroid4", "superellipsoid", "dense"])
+def test_columns_of_different_ranges(kind, gpu_lib):
+    """A column's accuracy does not depend on its neighbours: each against itself
+    alone, over the norm and, for the dense operator, row by row (relative to the
+    row's terms).  A warp's sums of n <= 3000 terms have n / 32 + 5 = 100 roundings in
+    a row: under 100 2^-53 = 1.1e-14 of the terms' sum, which is up to n^0.5 times the
+    result, and of either sign, so 100^0.5 2^-53 n^0.5 = 6e-14 of the norm."""
+    with _body(kind) as m:
+        X = _neighbours(m, kind)
+        Y = m.matvec(X)
+        for c in range(X.shape[1]):
+            ref = m.matvec(X[:, c])
+            assert np.linalg.norm(Y[:, c] - ref) < 1e-13 * np.linalg.norm(ref), c
+        if kind == "dense":
+            Z = m.matvec(np.eye(m.N, 64))   # |Z| of 64 sources at a time
+            A = np.concatenate([np.abs(m.matvec(np.roll(np.eye(m.N, 64), k, 0))) for k in range(0, m.N, 64)], 1)
+            assert np.array_equal(np.abs(Z), A[:, :64])
+            for c in range(X.shape[1]):
+                terms = A @ np.abs(X[:, c])
+                assert (np.abs(Y[:, c] - m.matvec(X[:, c])) <= 1e-14 * terms).all(), c

@@ -2,9 +2,8 @@
 products of 2 to 64 columns on one context, both buffers hold what the second
 writes.  No GPU: the header is compiled with the host C++ compiler.
 
-What a product of n columns writes is worked out here from the kernels' indices:
-parts [split][column][unknown] and, of exponents, two per unknown (dense: and one
-a block of 32) and one per box and column (dense: per column)."""
+What a product of n columns writes: parts [split][column][unknown], the split
+worked out here, and exponents, some per unknown and some per column (of a box)."""
 import os
 import shutil
 import subprocess
