@@ -207,8 +207,10 @@ k_ilu_cta(int N, const int* __restrict__ jlu, const int* __restrict__ ju, const 
 // one lane a batch took four, and the half that waits goes last.  The first
 // reduction step adds the halves, the last operations do Re and Im together.
 // A row that is not there yet holds a signalling NaN, which no operation returns,
-// in place of a flag, a fence and a second read.  12 warps: the polls of more
-// of them slow the chain.  Same sums, bit for bit.
+// in place of a flag, a fence and a second read; its two parts are accesses of 64
+// bits on both sides (b64 loads: 1.153 ms an apply of 1080 unknowns from the host,
+// f64 ones 1.160, one part a load 1.194).  12 warps: the polls of more of them slow
+// the chain.  Same sums, bit for bit.
 // Measured against k_ilu_cta: ILUT of 1080 unknowns 1.45 -> 1.04 ms, of 1470 2.33
 // -> 1.82 ms; ILU0 of 1920 (10.7 rows a level) 0.66 -> 0.78 ms, of 13230 5.2 ->
 // 6.6 ms.  8 warps 1.14, 16 1.17 ms; three batches ahead 1.21 ms.
@@ -240,15 +242,14 @@ __device__ void ilu_narrow_sweep(int N, const int* __restrict__ jlu, const int* 
                     a[h][u] = k < k1 ? alu[k] : make_double2(0, 0);
                     if (!im) a[h][u].y = -a[h][u].y;
                 }
-            // the entry's x, own part and other part; false: not there yet
+            // the entry's x, own part and other part; false: not there yet.  Two accesses
+            // of 64 bits, as the stores are: a part is there as a whole or not at all
             auto load = [&](unsigned at, double& own, double& oth) {
-                unsigned rl, rh, il, ih;
-                asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(rl), "=r"(rh), "=r"(il), "=r"(ih) : "r"(at));
-                const double r = __hiloint2double((int)rh, (int)rl), i = __hiloint2double((int)ih, (int)il);
-                own = im ? i : r;
-                oth = im ? r : i;
-                return rh != ILU_ABSENT_HI && ih != ILU_ABSENT_HI;
+                long long r, i;
+                asm volatile("ld.volatile.shared.v2.b64 {%0, %1}, [%2];" : "=l"(r), "=l"(i) : "r"(at));
+                own = __longlong_as_double(im ? i : r);
+                oth = __longlong_as_double(im ? r : i);
+                return (unsigned)(r >> 32) != ILU_ABSENT_HI && (unsigned)(i >> 32) != ILU_ABSENT_HI;
             };
             // batch u's half h, if its values are there or once they are
             auto step = [&](int h, int u, bool wait) {
