@@ -34,8 +34,8 @@ def _nvcc():
 def _compile(src: str) -> str:
     obj = os.path.join(OBJ_DIR, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
-    deps = [path, os.path.join(CSRC, "mlf_internal.h"), os.path.join(CSRC, "mlf_tcgen05.h"),
-            os.path.join(os.path.dirname(HERE), "include", "lywell_mlfma.h")]
+    deps = [path, os.path.join(os.path.dirname(HERE), "include", "lywell_mlfma.h"),
+            *(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh")))]
     if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in deps):
         return obj
     cmd = [_nvcc(), "-std=c++17", "-O3", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC,-ffp-contract=off",
