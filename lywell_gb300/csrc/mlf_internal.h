@@ -259,6 +259,7 @@ int fp64_matvec_launch(Ctx* c, const double2* x, double2* y, int nrhs, int ld, c
                        double2* const* Cf, double2* const* Bf, double2* const* Af, cudaEvent_t* ev);
 // FP64 near field, leaf aggregation and receive on blocks of columns (mlf_split64.cu)
 bool split64_on(const Ctx* c, int nrhs);
+int dense64_setup(Ctx* c);
 int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s);
 int split64_ready(Ctx* c, int nrhs);
 int split64_aggregate(Ctx* c, const double2* x, int nrhs, int ld, double2* C, cudaStream_t s);

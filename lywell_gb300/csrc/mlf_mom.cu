@@ -64,6 +64,7 @@ int dense_setup(Ctx* c) {
     k_mom_fill<<<c->N, 256, 0, c->stream>>>(c->N, c->dt_baric, c->dt_baric_sub, c->dp_coord, c->de_t, c->de_po,
                                             c->de_long, c->ph.w, c->ph.w * c->ph.smue, c72, c->dZdense);
     CK(cudaGetLastError());
+    if ((st = dense64_setup(c))) return st;
     CK(cudaStreamSynchronize(c->stream));
     return MLF_OK;
 }

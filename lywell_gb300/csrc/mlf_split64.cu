@@ -228,9 +228,10 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int er, i
 __global__ void k_dense_block_exp(int N, int nblk, const double2* __restrict__ Z, short* __restrict__ bexp) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (row >= N) return;
+#pragma unroll 4
     for (int b = 0; b < nblk; ++b) {
         const int k = 32 * b + lane;
-        const int e = __reduce_max_sync(0xffffffffu, k < N ? oz_exp(Z[(size_t)row * N + k]) : -1022);
+        const int e = __reduce_max_sync(0xffffffffu, k < N ? oz_exp(Z[(size_t)row * N + k]) : OZ_ZERO);
         if (lane == 0) bexp[(size_t)row * nblk + b] = (short)min(max(e, -2000), 2000);   // 2000: not finite
     }
 }
@@ -673,30 +674,25 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
 
 // Dense operator: y = Z x for blocks of columns.  The row exponents are bounds by
 // blocks of 32 unknowns, so that a product reads the matrix once.  FP64 FMAs, four
-// columns a pass, against here: 6750 unknowns x 3: 1399, 467 us; x 24: 7678, 1297;
-// 3000 x 2: 339, 120; 1920 x 4: 131, 59; 1080 x 6: 86, 39.
-static int dense64_ready(Ctx* c, int nrhs) {
+// columns a pass, against here: 6750 unknowns x 3: 1399, 474 us; x 24: 7678, 1297;
+// 3000 x 2: 339, 120; 1920 x 4: 131, 59; 1080 x 6: 86, 39.  At most OZ_DENSE_COLS
+// columns at a time, so that the workspace is made with the context and products
+// of any number of columns allocate nothing (the first one may be captured).
+constexpr int OZ_DENSE_COLS = 48;
+
+int dense64_setup(Ctx* c) {
     const int N = c->N, nblk = (N + 31) / 32;
-    if (!c->doz_pat) {
-        CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->dev));
-        CK(cudaFuncSetAttribute(k_split64<OZ_DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-        c->noz_tiles = (N + OZ_R - 1) / OZ_R;
-        int* p = nullptr;
-        CK(cudaMalloc(&p, (size_t)N * nblk * sizeof(short)));
-        k_dense_block_exp<<<(N + 7) / 8, 256, 0, c->stream>>>(N, nblk, c->dZdense, reinterpret_cast<short*>(p));
-        if (!cuda_ok(c, cudaGetLastError(), "k_dense_block_exp") ||
-            !cuda_ok(c, cudaStreamSynchronize(c->stream), "k_dense_block_exp")) {   // products may run on another stream
-            cudaFree(p);
-            return MLF_E_CUDA;
-        }
-        c->doz_pat = p;
-    }
-    return oz_workspace(c, nrhs, 2 * (size_t)N + 1 + nblk, 1 + (size_t)N);
+    CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->dev));
+    // a limit of the kernel, the same for every context
+    CK(cudaFuncSetAttribute(k_split64<OZ_DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+    c->noz_tiles = (N + OZ_R - 1) / OZ_R;
+    CK(cudaMalloc(&c->doz_pat, (size_t)N * nblk * sizeof(short)));
+    k_dense_block_exp<<<(N + 7) / 8, 256, 0, c->stream>>>(N, nblk, c->dZdense, reinterpret_cast<short*>(c->doz_pat));
+    CK(cudaGetLastError());
+    return oz_workspace(c, OZ_DENSE_COLS, 2 * (size_t)N + 1 + nblk, 1 + (size_t)N);
 }
 
-int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
-    int st;
-    if ((st = dense64_ready(c, nrhs))) return st;
+static void dense64_columns(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
     const int N = c->N, nblk = (N + 31) / 32, nsplit = near64_split(c, nrhs);
     int *sexp = c->doz_exp, *rexp = sexp + N, *nredo = rexp + N, *bmax = nredo + 1, *cexp = bmax + nblk;
     unsigned* redo = reinterpret_cast<unsigned*>(cexp + nrhs);
@@ -710,9 +706,15 @@ int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaS
     g.sexp = sexp; g.rexp = rexp; g.cexp = cexp;
     g.out = c->doz_ws; g.cov = oz_covers(c);
     k_split64<OZ_DENSE><<<dim3((unsigned)c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C), nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
-    k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, g.cov, y, nredo,
-                                                               redo);
+    k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, g.cov, y, nredo, redo);
     k_redo_dense<<<OZ_REDO_CTAS * c->nsm, 256, 0, s>>>(N, ld, nredo, redo, c->dZdense, x, y);
+}
+
+int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
+    const int groups = (nrhs + OZ_DENSE_COLS - 1) / OZ_DENSE_COLS;
+    const int per = ((nrhs + groups - 1) / groups + OZ_C - 1) / OZ_C * OZ_C;   // whole blocks of 12
+    for (int c0 = 0; c0 < nrhs; c0 += per)
+        dense64_columns(c, x + (size_t)c0 * ld, y + (size_t)c0 * ld, std::min(per, nrhs - c0), ld, s);
     return cuda_ok(c, cudaGetLastError(), "dense matvec (split)") ? MLF_OK : MLF_E_CUDA;
 }
 

@@ -88,3 +88,22 @@ def test_columns_of_different_ranges(kind, gpu_lib):
             for c in range(X.shape[1]):
                 terms = A @ np.abs(X[:, c])
                 assert (np.abs(Y[:, c] - m.matvec(X[:, c])) <= 1e-14 * terms).all(), c
+
+
+@pytest.mark.parametrize("nrhs", [1, 3, 60])
+def test_first_dense_block_under_capture(nrhs, gpu_lib):
+    """A dense operator's products allocate nothing and wait for nothing: the first
+    one of a context, of any number of columns, can be captured in a CUDA graph."""
+    import torch
+    with _body("dense") as m:
+        x = torch.from_numpy(np.ascontiguousarray(_columns(m.N, nrhs, 3).T)).cuda()
+        y = torch.zeros_like(x)
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            m.matvec_device(x.data_ptr(), y.data_ptr(), nrhs, s.cuda_stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        ref = m.matvec(x.cpu().numpy().T)
+        assert np.array_equal(y.cpu().numpy().T, ref.reshape(m.N, nrhs))
