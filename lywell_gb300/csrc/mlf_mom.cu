@@ -1,11 +1,11 @@
 // Dense method-of-moments operator on the GPU (modMoM.f90:85-128 fill,
 // MatxVec_MoM modMoM.f90:273-277): the full N x N impedance matrix in FP64,
 // filled on the device by the same Z_mn element as the near field, and a
-// matvec that streams it once per group of twelve right-hand sides.  A
-// context made with MLF_FLAG_DENSE_MOM holds this operator instead of the
-// octree; CGS, excitation and RCS run on it unchanged.  At N = 30720 the
-// matrix is 15 GB, within HBM, so it also serves as the exact reference for
-// the MLFMA matvec error.
+// matvec that streams it once per column where a block's columns are few or the
+// matrix small, else once per group of twelve (mlf_split64.cu).  A context made
+// with MLF_FLAG_DENSE_MOM holds this operator instead of the octree; CGS,
+// excitation and RCS run on it unchanged.  At N = 30720 the matrix is 15 GB, within
+// HBM, so it also serves as the exact reference for the MLFMA matvec error.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -71,10 +71,14 @@ int dense_setup(Ctx* c) {
 
 int dense_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
     // blocks of columns go to the digit splits, but for small matrices, where their
-    // six launches (about 30 us) cost more: 1080 unknowns x 2 is 36 us either way
-    if (nrhs > 1 && (double)c->N * c->N * nrhs > 2.5e6) return dense64_matvec(c, x, y, nrhs, ld, s);
-    const long long threads = (long long)c->N * 32;
-    k_mom_gemv<<<dim3((unsigned)((threads + 255) / 256), nrhs), 256, 0, s>>>(c->N, ld, c->dZdense, x, y);
+    // seven launches a group of columns (about 30 us) cost more: 1080 unknowns x 2 is
+    // 36 us either way
+    if (nrhs > 1 && (double)c->N * c->N * std::min(nrhs, OZ_DENSE_COLS) > 2.5e6)
+        return dense64_matvec(c, x, y, nrhs, ld, s);
+    const unsigned ctas = (unsigned)(((long long)c->N * 32 + 255) / 256);
+    for (int c0 = 0; c0 < nrhs; c0 += 65535)   // a grid has so many rows
+        k_mom_gemv<<<dim3(ctas, std::min(nrhs - c0, 65535)), 256, 0, s>>>(c->N, ld, c->dZdense, x + (size_t)c0 * ld,
+                                                                          y + (size_t)c0 * ld);
     return cuda_ok(c, cudaGetLastError(), "dense matvec") ? MLF_OK : MLF_E_CUDA;
 }
 

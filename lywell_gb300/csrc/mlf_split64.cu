@@ -678,8 +678,6 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
 // 3000 x 2: 339, 120; 1920 x 4: 131, 59; 1080 x 6: 86, 39.  At most OZ_DENSE_COLS
 // columns at a time, so that the workspace is made with the context and products
 // of any number of columns allocate nothing (the first one may be captured).
-constexpr int OZ_DENSE_COLS = 48;
-
 int dense64_setup(Ctx* c) {
     const int N = c->N, nblk = (N + 31) / 32;
     CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->dev));

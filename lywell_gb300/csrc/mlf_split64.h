@@ -6,6 +6,7 @@
 namespace mlf {
 
 constexpr int OZ_C = 12;           // complex columns per CTA
+constexpr int OZ_DENSE_COLS = 48;  // columns at a time of the dense operator
 constexpr int OZ_MAX_SPLIT = 4, OZ_MAX_DENSE_SPLIT = 8;
 
 // Parts of the terms: enough CTAs for about four waves of one per SM

@@ -107,3 +107,17 @@ def test_first_dense_block_under_capture(nrhs, gpu_lib):
         torch.cuda.synchronize()
         ref = m.matvec(x.cpu().numpy().T)
         assert np.array_equal(y.cpu().numpy().T, ref.reshape(m.N, nrhs))
+
+
+@pytest.mark.parametrize("nrhs", [65536, 66000, 70001])
+def test_more_dense_columns_than_a_grid_has_rows(nrhs, gpu_lib):
+    """A tetrahedron's six unknowns.  Against the matrix itself; sums of six terms,
+    1e-14 of the norm."""
+    from lywell_gb300 import RWG, MoM
+    v = 0.3 * np.array([[1.0, 1, 1], [1, -1, -1], [-1, 1, -1], [-1, -1, 1]])
+    tris = v[np.array([[0, 1, 2], [0, 3, 1], [0, 2, 3], [1, 3, 2]])]
+    with MoM(RWG(tris)) as m:
+        assert m.N == 6
+        Z = m.matvec(np.eye(6) + 0j)
+        X = _columns(6, nrhs, 1)
+        assert np.linalg.norm(m.matvec(X) - Z @ X) < 1e-14 * np.linalg.norm(Z @ X)
