@@ -336,9 +336,11 @@ k_ilu_narrow(int N, const int* __restrict__ jlu, const int* __restrict__ ju, con
 }
 
 // Whether k_ilu_cta takes the factors: x must fit in one CTA's shared memory
-// (13 900 unknowns), and levels must be narrow: one SM takes up to 0.2 us a row
+// (13 600 unknowns), and levels must be narrow: one SM takes up to 0.2 us a row
 // (measured 0.15 to 0.20 with ILU0's 180 to 600 levels), a launch per level
-// 6 us (measured 4.7 to 7).
+// 6 us (measured 4.7 to 7).  Long rows take longer in either: 4108 entries a row and
+// 2.6 rows a level (ILU0 of a 12000-RWG spheroid) 432 ms by levels, 164 in a CTA;
+// 621 and 11.7: 24.6, 12.1; 158 and 21.8: 8.0, 4.6.
 static bool ilu_in_cta(const Ctx* c, int optin) {
     constexpr double ROW_US = 0.2, LEVEL_US = 6.0;
     if ((size_t)c->N * (sizeof(double2) + 1) + 1024 > (size_t)optin) return false;
@@ -346,10 +348,16 @@ static bool ilu_in_cta(const Ctx* c, int optin) {
     return 2 * ROW_US * c->N < LEVEL_US * levels;
 }
 
-// Whether those rows go to k_ilu_narrow: fewer than four a level (both sides in
-// its comment, at 1.8 and 10.7).
+// Whether those rows go to k_ilu_narrow: fewer than four a level, with fewer than
+// 600 entries in the rows of one; where there are more, the entries that are there
+// count, not the wait for the last, and k_ilu_cta has more warps for them.  Applies
+// in ms, k_ilu_cta against k_ilu_narrow, by rows a level x entries a row: 1.8 x 149:
+// 1.57, 1.15; 1.7 x 205: 2.53, 1.95; 2.5 x 95: 0.99, 0.84; 3.6 x 118: 1.35, 1.30; 2.65 x
+// 182: 2.31, 2.24; 3.3 x 219: 5.71, 6.32; 3.5 x 457: 7.62, 9.77; 1.5 x 1010: 21.2, 25.3;
+// 8.5 x 97: 1.69, 2.12.
 static bool ilu_narrow(const Ctx* c) {
-    return 2 * (size_t)c->N < 4 * (c->lvl_ptr_f.size() + c->lvl_ptr_b.size() - 2);
+    const size_t levels = c->lvl_ptr_f.size() + c->lvl_ptr_b.size() - 2;
+    return 2 * (size_t)c->N < 4 * levels && 2 * c->alu.size() < 600 * levels;
 }
 
 int device_ilu_upload(Ctx* c) {
