@@ -172,13 +172,14 @@ struct Ctx {
     float2* dZ = nullptr;
     double2* dZd = nullptr;           // the same near values as complex(8)
     // FP64 products on blocks of columns (mlf_split64.cu): row tiles (box, first
-    // row), exponents of the patterns (or of the dense matrix), the call's exponents (x's rows, Z's rows,
-    // columns) and the near sums [split][column][box-sorted place]
+    // row) and, behind them, exponents of the patterns (doz_pat; of the dense matrix
+    // on its own); sums [split][column][box-sorted place], their covers and, behind
+    // them, exponents and lists of the call (doz_exp)
     int2* doz_tiles = nullptr;
     int *doz_pat = nullptr, *doz_exp = nullptr;
     int noz_tiles = 0, nsm = 0;
     double2* doz_ws = nullptr;
-    OzSizes oz_cap;                   // of doz_ws and doz_exp
+    OzSizes oz_cap;                   // of the sums and of doz_exp
     // device geometry for set-up kernels and RCS
     double *dp_coord = nullptr, *dt_baric = nullptr, *dt_baric_sub = nullptr, *de_long = nullptr,
            *de_centro = nullptr;

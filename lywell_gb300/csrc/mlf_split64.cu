@@ -40,7 +40,7 @@
 //
 // mma.sync keeps each digit sum in the registers of the warp that joins it.
 // 12000-RWG spheroid (49 M near entries), 24 columns: the whole product 9.77 ms with
-// FMAs, 1.95 ms without the check, 2.02 ms with it.
+// FMAs, 1.95 ms without the check, 1.96 to 2.02 ms with it.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -556,23 +556,24 @@ static int oz_workspace(Ctx* c, int nrhs, size_t fixed, size_t per_col) {
     const OzSizes need = oz_sizes(c->noz_tiles, c->nsm, c->N, c->dense, fixed, per_col, nrhs);
     if (!oz_short(c->oz_cap, need)) return MLF_OK;
     if (c->doz_ws) cudaFree(c->doz_ws);
-    if (c->doz_exp) cudaFree(c->doz_exp);
     c->doz_ws = nullptr;
     c->doz_exp = nullptr;
     const OzSizes grown{std::max(c->oz_cap.sums, need.sums), std::max(c->oz_cap.exps, need.exps)};
     c->oz_cap = OzSizes();
-    CK(cudaMalloc(&c->doz_ws, grown.sums * (sizeof(double2) + sizeof(float))));   // sums, then covers
-    CK(cudaMalloc(&c->doz_exp, grown.exps * sizeof(int)));
+    // one allocation: sums, their covers, exponents
+    CK(cudaMalloc(&c->doz_ws, grown.sums * (sizeof(double2) + sizeof(float)) + grown.exps * sizeof(int)));
     c->oz_cap = grown;
+    c->doz_exp = reinterpret_cast<int*>(oz_covers(c) + grown.sums);
     return MLF_OK;
 }
 
 // Where the products run here: a CTA's tile is 64 rows of one box by 12 columns,
-// so boxes and blocks must fill it to some part.  Aggregation, receive and near
-// field in ms, FP64 FMAs against here, by bases per box x columns: 4 x 24: 1.95,
-// 4.48; 14 x 2: 0.39, 0.97; 14 x 8: 1.42, 1.19; 35 x 2: 0.43, 0.53; 35 x 8: 1.36,
-// 0.62; 61 x 24: 8.59, 2.29; 240 x 2: 0.62, 0.38.  One column stays with the
-// FMAs, whose order of sums single solves keep.
+// so boxes and blocks must fill it to some part.  Whole products in us, FP64 FMAs
+// against here, by bases per box x columns, of bodies of 7680 to 48000 unknowns:
+// 4.3 x 24: 21801, 24565; 11.0 x 12: 14051, 13987; 15.5 x 6: 2830, 2915; x 8: 3736,
+// 3548; 21.9 x 4: 4118, 4106; x 6: 6061, 5549; 37.3 x 2: 1194, 1351; x 4: 2119, 1703; 41.7 x
+// 3: 509, 443; 240 x 2: 639, 421.  One column stays with the FMAs, whose order of
+// sums single solves keep.
 bool split64_on(const Ctx* c, int nrhs) {
     const long long nb = (long long)c->box_ptr.size() - 1;
     return nrhs >= 2 && c->N >= 12 * nb && (long long)c->N * nrhs >= 112 * nb;
@@ -592,18 +593,19 @@ int split64_ready(Ctx* c, int nrhs) {
         CK(cudaFuncSetAttribute(k_split64<OZ_NEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
         CK(cudaFuncSetAttribute(k_split64<OZ_RECEIVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
         CK(cudaFuncSetAttribute(k_split64<OZ_AGGREGATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-        if (!c->doz_pat) CK(cudaMalloc(&c->doz_pat, (c->N + nb * K2) * sizeof(int)));
-        k_pattern_exp<<<(c->N + 7) / 8, 256, 0, c->stream>>>(c->N, (int)K2, c->dR, c->doz_pat);
-        k_direction_exp<<<(unsigned)nb, 256, 0, c->stream>>>((int)K2, c->dbox_ptr, c->dR, c->doz_pat + c->N);
-        CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(c->stream));   // products may run on another stream
-        int2* d = nullptr;
-        CK(cudaMalloc(&d, t.size() * sizeof(int2)));
-        if (!cuda_ok(c, cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice), "tiles")) {
+        int2* d = nullptr;   // the tiles, then the exponents
+        CK(cudaMalloc(&d, t.size() * sizeof(int2) + (c->N + nb * K2) * sizeof(int)));
+        int* pat = reinterpret_cast<int*>(d + t.size());
+        k_pattern_exp<<<(c->N + 7) / 8, 256, 0, c->stream>>>(c->N, (int)K2, c->dR, pat);
+        k_direction_exp<<<(unsigned)nb, 256, 0, c->stream>>>((int)K2, c->dbox_ptr, c->dR, pat + c->N);
+        if (!cuda_ok(c, cudaGetLastError(), "pattern exponents") ||
+            !cuda_ok(c, cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice), "tiles") ||
+            !cuda_ok(c, cudaStreamSynchronize(c->stream), "pattern exponents")) {   // products may run on another stream
             cudaFree(d);
             return MLF_E_CUDA;
         }
         c->doz_tiles = d;
+        c->doz_pat = pat;
         c->noz_tiles = (int)t.size();
     }
     return oz_workspace(c, nrhs, 2 * (size_t)c->N + 1, 2 * nb + c->N);
