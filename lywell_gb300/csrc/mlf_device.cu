@@ -240,8 +240,8 @@ __global__ void k_receive_near_d(int K, int N, int nrhs, int ld, const int* __re
     if (gw >= N * nrhs) return;
     const int j = gw / nrhs, r = gw % nrhs;
     const int n = perm[j], b = box_of_sorted[j];
-    const double2 t = receive_near_row(2 * K, n, R + (size_t)j * 2 * K, A + ((size_t)b * nrhs + r) * 2 * K, ia, ja, Zd,
-                                       x + (size_t)r * ld, facy);
+    const double2 t = warp_sum(receive_near_terms(lane, 32, 2 * K, n, R + (size_t)j * 2 * K,
+                                                  A + ((size_t)b * nrhs + r) * 2 * K, ia, ja, Zd, x + (size_t)r * ld, facy));
     if (lane == 0) y[(size_t)r * ld + n] = t;
 }
 

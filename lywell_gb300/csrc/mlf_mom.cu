@@ -43,7 +43,7 @@ __global__ void k_mom_gemv(int N, int ld, const double2* __restrict__ Z, const d
     const int lane = threadIdx.x & 31;
     if (gw >= N) return;
     const int m = (int)gw;
-    const double2 t = dense_row(N, Z + (size_t)m * N, x);
+    const double2 t = warp_sum(dense_terms(lane, 32, N, Z + (size_t)m * N, x));
     if (lane == 0) y[m] = t;
 }
 

@@ -317,33 +317,61 @@ __global__ void k_redo_aggregate(int K2, int nrhs, int ld, const int* __restrict
         C[(size_t)blockIdx.x * K2 + q] =
             aggregate_direction(K2, box_ptr[b], box_ptr[b + 1], q, perm, R, x + (size_t)r * ld);
 }
-// y of the listed (column, box-sorted basis), a warp each
-__global__ void __launch_bounds__(256) k_redo_receive_near(int K2, int N, int nrhs, int ld, const int* __restrict__ nredo,
-                                                           const unsigned* __restrict__ redo,
-                                                           const int* __restrict__ perm,
-                                                           const int* __restrict__ box_of_sorted,
-                                                           const double2* __restrict__ R, const double2* __restrict__ A,
-                                                           const int* __restrict__ ia, const int* __restrict__ ja,
-                                                           const double2* __restrict__ Zd, const double2* __restrict__ x,
-                                                           double facy, double2* __restrict__ y) {
-    const int n = *nredo;
-    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += gridDim.x * (blockDim.x >> 5)) {
-        const int r = redo[k] / N, j = redo[k] % N, i = perm[j];
-        const double2 t = receive_near_row(K2, i, R + (size_t)j * K2, A + ((size_t)box_of_sorted[j] * nrhs + r) * K2, ia,
-                                           ja, Zd, x + (size_t)r * ld, facy);
-        if ((threadIdx.x & 31) == 0) y[(size_t)r * ld + i] = t;
+// The listed values v: store(v, sum of terms(v, first, step) over first = 0 .. step - 1).
+// A warp each, or, while there are no more of them than CTAs, a CTA each: one row's
+// chain of FP64 FMAs is the time then (one row of 4100 terms 18 us, with a warp 71).
+constexpr int OZ_REDO_T = 256;
+template <class Terms, class Store>
+__device__ __forceinline__ void redo_listed(int n, const unsigned* __restrict__ redo, Terms terms, Store store) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (n <= (int)gridDim.x) {
+        __shared__ double2 part[OZ_REDO_T / 32];
+        if ((int)blockIdx.x >= n) return;
+        const unsigned v = redo[blockIdx.x];
+        const double2 t = warp_sum(terms(v, threadIdx.x, OZ_REDO_T));
+        if (lane == 0) part[warp] = t;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double2 s = part[0];
+            for (int w = 1; w < OZ_REDO_T / 32; ++w) {
+                s.x += part[w].x;
+                s.y += part[w].y;
+            }
+            store(v, s);
+        }
+        return;
+    }
+    for (int k = blockIdx.x * (OZ_REDO_T / 32) + warp; k < n; k += gridDim.x * (OZ_REDO_T / 32)) {
+        const unsigned v = redo[k];
+        const double2 t = warp_sum(terms(v, lane, 32));
+        if (lane == 0) store(v, t);
     }
 }
-// y of the listed (column, row) of the dense operator, a warp each
-__global__ void __launch_bounds__(256) k_redo_dense(int N, int ld, const int* __restrict__ nredo,
-                                                    const unsigned* __restrict__ redo, const double2* __restrict__ Z,
-                                                    const double2* __restrict__ x, double2* __restrict__ y) {
-    const int n = *nredo;
-    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += gridDim.x * (blockDim.x >> 5)) {
-        const int r = redo[k] / N, i = redo[k] % N;
-        const double2 t = dense_row(N, Z + (size_t)i * N, x + (size_t)r * ld);
-        if ((threadIdx.x & 31) == 0) y[(size_t)r * ld + i] = t;
-    }
+// y of the listed (column, box-sorted basis)
+__global__ void __launch_bounds__(OZ_REDO_T)
+k_redo_receive_near(int K2, int N, int nrhs, int ld, const int* __restrict__ nredo, const unsigned* __restrict__ redo,
+                    const int* __restrict__ perm, const int* __restrict__ box_of_sorted, const double2* __restrict__ R,
+                    const double2* __restrict__ A, const int* __restrict__ ia, const int* __restrict__ ja,
+                    const double2* __restrict__ Zd, const double2* __restrict__ x, double facy, double2* __restrict__ y) {
+    redo_listed(*nredo, redo,
+                [&](unsigned v, int first, int step) {
+                    const int r = v / N, j = v % N;
+                    return receive_near_terms(first, step, K2, perm[j], R + (size_t)j * K2,
+                                              A + ((size_t)box_of_sorted[j] * nrhs + r) * K2, ia, ja, Zd,
+                                              x + (size_t)r * ld, facy);
+                },
+                [&](unsigned v, double2 t) { y[(size_t)(v / N) * ld + perm[v % N]] = t; });
+}
+// y of the listed (column, row) of the dense operator
+__global__ void __launch_bounds__(OZ_REDO_T) k_redo_dense(int N, int ld, const int* __restrict__ nredo,
+                                                          const unsigned* __restrict__ redo,
+                                                          const double2* __restrict__ Z, const double2* __restrict__ x,
+                                                          double2* __restrict__ y) {
+    redo_listed(*nredo, redo,
+                [&](unsigned v, int first, int step) {
+                    return dense_terms(first, step, N, Z + (size_t)(v % N) * N, x + (size_t)(v / N) * ld);
+                },
+                [&](unsigned v, double2 t) { y[(size_t)(v / N) * ld + v % N] = t; });
 }
 
 struct OzArgs {
@@ -545,7 +573,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_split64(const OzArgs g) {
 
 static float* oz_covers(const Ctx* c) { return reinterpret_cast<float*>(c->doz_ws + c->oz_cap.sums); }
 
-// CTAs of 256 threads that go through a list of values to compute again
+// CTAs that go through a list of values to compute again
 constexpr int OZ_REDO_CTAS = 8;   // per SM
 
 static int near64_split(const Ctx* c, int nrhs) { return oz_split(c->noz_tiles, c->nsm, nrhs, c->dense); }
@@ -669,7 +697,7 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
     g.x = A; g.rexp = c->doz_pat; g.out = y; g.near = c->doz_ws; g.nsplit = nsplit; g.facy = facy;
     g.nredo = e.nredo; g.redo = e.redo;
     k_split64<OZ_RECEIVE><<<ncb * c->noz_tiles, OZ_THREADS, OZ_SMEM, s>>>(g);
-    k_redo_receive_near<<<OZ_REDO_CTAS * c->nsm, 256, 0, s>>>(g.K2, c->N, nrhs, ld, e.nredo, e.redo, g.perm,
+    k_redo_receive_near<<<OZ_REDO_CTAS * c->nsm, OZ_REDO_T, 0, s>>>(g.K2, c->N, nrhs, ld, e.nredo, e.redo, g.perm,
                                                               c->dbox_of_sorted, g.R, A, g.ia, g.ja, c->dZd, x, facy, y);
     return cuda_ok(c, cudaGetLastError(), "near + receive (split)") ? MLF_OK : MLF_E_CUDA;
 }
@@ -707,7 +735,7 @@ static void dense64_columns(Ctx* c, const double2* x, double2* y, int nrhs, int 
     g.out = c->doz_ws; g.cov = oz_covers(c);
     k_split64<OZ_DENSE><<<dim3((unsigned)c->noz_tiles * ((nrhs + OZ_C - 1) / OZ_C), nsplit), OZ_THREADS, OZ_SMEM, s>>>(g);
     k_sum_parts<<<dim3((N + 255) / 256, nrhs), 256, 0, s>>>(N, nrhs, ld, nsplit, c->doz_ws, g.cov, y, nredo, redo);
-    k_redo_dense<<<OZ_REDO_CTAS * c->nsm, 256, 0, s>>>(N, ld, nredo, redo, c->dZdense, x, y);
+    k_redo_dense<<<OZ_REDO_CTAS * c->nsm, OZ_REDO_T, 0, s>>>(N, ld, nredo, redo, c->dZdense, x, y);
 }
 
 int dense64_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
