@@ -107,6 +107,11 @@ const char* mlf_last_error(const mlf_ctx* ctx);
 
 /* y = Z_MLFMA x for nrhs columns, host arrays (complex(8), n x nrhs, ld >= N).
  * Includes the host<->device copies.
+ * A single column is summed in FP64 FMAs in a fixed order.  Blocks of columns
+ * where leaf boxes are full (and of the dense operator) are summed by exact digit
+ * splits where that is as accurate: each value to FP64 accuracy of its own terms,
+ * whatever its neighbours hold, but a column of a block can differ in the last places
+ * from the same column alone or in a block of another size.
  * Replaces: MatxVec_MLFMA (modMLFMA.f90:1901-1946). */
 int mlf_matvec(mlf_ctx* ctx, const double* x, double* y, int nrhs, int ld);
 
@@ -314,9 +319,10 @@ int mlf_set_nearinv_precision(mlf_ctx* ctx, int bits);
 /* The FP32 LU gives each box one CTA, so the largest neighbourhoods would set
  * the set-up time alone.  Boxes of at least min_unknowns unknowns that hold
  * 1600 unknowns or more, or whose work (n^3) exceeds the remaining boxes' share
- * per CTA, are factorised on many CTAs each instead (panel on one CTA; U12 and
- * the trailing update over the GPU), in groups of boxes in step, on side streams
- * next to the one-CTA-per-box kernel; the results are the same.
+ * per CTA (three times that share where there are four boxes per SM or more),
+ * largest first, are factorised on many CTAs each instead (panel on one CTA; U12
+ * and the trailing update over the GPU), in groups of boxes in step, on side
+ * streams next to the one-CTA-per-box kernel; the results are the same.
  * min_unknowns = 0 turns this off; the default is 1024.  mlf_get_lu_split
  * reads the setting and how many boxes took the many-CTA path in the last
  * build.  No counterpart in the reference. */

@@ -322,11 +322,13 @@ __global__ void __launch_bounds__(TQ, 2) k_mlp_forward_tc(long long ntok, const 
 // Forward + loss + backward over tokens idx[0..ntok) (idx NULL: 0..ntok-1);
 // gradients of the mean loss (scale = 1 / (ntok_total * OUT)) added into G,
 // the loss sum into *loss.  A tile's three 64 x 128 x 128 products are FP32
-// FMAs on values in shared memory (4 x 8 or 8 x 8 sums a thread); 16-byte
-// shared-memory reads without bank conflicts and 16-byte reductions into G
-// keep the FMA pipe the bound (about 13 us a tile).  8192 tokens, one tile on
-// each of 128 SMs, mlf_mlp_grad with its copy to the host: 172 us with scalar
-// reads (conflicts of 4 to 16 ways) and scalar atomics, 65 us now.
+// FMAs on values in shared memory (4 x 8 or 8 x 8 sums a thread), with 16-byte
+// shared-memory reads without bank conflicts and 16-byte reductions into G.  8192
+// tokens, one tile on each of 128 SMs: the kernel takes 38 us, its one CTA of 8
+// warps an SM issuing 2.1 instructions a cycle (FMA pipe 40 % active, shared memory
+// 54 %): too few warps, neither pipe, bound it.  mlf_mlp_grad with its copy to the
+// host: 172 us with scalar reads (conflicts of 4 to 16 ways) and scalar atomics, 65 us
+// now.
 __global__ void __launch_bounds__(256) k_mlp_grad(long long ntok, const long long* __restrict__ idx,
                                                   const float* __restrict__ X, const float* __restrict__ T,
                                                   const float* __restrict__ norm,

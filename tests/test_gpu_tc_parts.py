@@ -1,9 +1,10 @@
 """The tcgen05 engine, its tiles cut into parts by equal shares of the chunks, in
-rings of three and four stages, against the FP64 operator.
+rings of either depth, against the FP64 operator.
 
-Bodies: about 46 tiles of 145 rows (four or five parts each, three stages), 184
-tiles of 42 rows (one or two parts, four stages) and 736 tiles of 42 rows (most
-in one part, four stages).
+Bodies: about 46 tiles of 145 rows (four or five parts each; rings of four stages,
+the receive's three), 184 tiles of 42 rows (one or two parts; at most 96 rows: five
+stages, the receive's four) and 736 tiles of 42 rows (most in one part, as before).
+The aggregation's tiles are rows of directions, with a depth of their own.
 Columns: the fewest, one over half a column tile, one over a whole one, and back
 to few in the workspaces of the larger block.
 
