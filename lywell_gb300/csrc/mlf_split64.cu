@@ -179,14 +179,21 @@ __global__ void k_pattern_exp(int N, int K2, const double2* __restrict__ R, int*
     e = __reduce_max_sync(0xffffffffu, e);
     if (lane == 0) rexp[pos] = e;
 }
-__global__ void k_direction_exp(int K2, const int* __restrict__ box_ptr, const double2* __restrict__ R,
-                                int* __restrict__ qexp) {
-    const int b = blockIdx.x;
-    for (int q = threadIdx.x; q < K2; q += blockDim.x) {
-        int e = OZ_ZERO;
-        for (int t = box_ptr[b]; t < box_ptr[b + 1]; ++t) e = max(e, oz_exp(R[(size_t)t * K2 + q]));
-        qexp[(size_t)b * K2 + q] = e;
-    }
+// ... a CTA per box and 32 directions, its warps over the bases (12000-RWG spheroid, 32
+// boxes: 30 us; a CTA a box, 390)
+__global__ void __launch_bounds__(256) k_direction_exp(int K2, const int* __restrict__ box_ptr,
+                                                       const double2* __restrict__ R, int* __restrict__ qexp) {
+    __shared__ int top[8][32];
+    const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = blockIdx.y * 32 + lane;
+    int e = OZ_ZERO;
+    if (q < K2)
+#pragma unroll 4
+        for (int t = box_ptr[b] + warp; t < box_ptr[b + 1]; t += 8) e = max(e, oz_exp(R[(size_t)t * K2 + q]));
+    top[warp][lane] = e;
+    __syncthreads();
+    if (warp || q >= K2) return;
+    for (int w = 1; w < 8; ++w) e = max(e, top[w][lane]);
+    qexp[(size_t)b * K2 + q] = e;
 }
 
 // The digits of (re, im) as FP16 pairs, most significant first: with 128 added
@@ -625,7 +632,7 @@ int split64_ready(Ctx* c, int nrhs) {
         CK(cudaMalloc(&d, t.size() * sizeof(int2) + (c->N + nb * K2) * sizeof(int)));
         int* pat = reinterpret_cast<int*>(d + t.size());
         k_pattern_exp<<<(c->N + 7) / 8, 256, 0, c->stream>>>(c->N, (int)K2, c->dR, pat);
-        k_direction_exp<<<(unsigned)nb, 256, 0, c->stream>>>((int)K2, c->dbox_ptr, c->dR, pat + c->N);
+        k_direction_exp<<<dim3((unsigned)nb, (unsigned)(K2 + 31) / 32), 256, 0, c->stream>>>((int)K2, c->dbox_ptr, c->dR, pat + c->N);
         if (!cuda_ok(c, cudaGetLastError(), "pattern exponents") ||
             !cuda_ok(c, cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice), "tiles") ||
             !cuda_ok(c, cudaStreamSynchronize(c->stream), "pattern exponents")) {   // products may run on another stream
