@@ -71,7 +71,7 @@ int dense_setup(Ctx* c) {
 
 int dense_matvec(Ctx* c, const double2* x, double2* y, int nrhs, int ld, cudaStream_t s) {
     // blocks of columns go to the digit splits, but for small matrices, where their
-    // seven launches a group of columns (about 30 us) cost more: 1080 unknowns x 2 is
+    // six launches a group of columns (about 30 us) cost more: 1080 unknowns x 2 is
     // 36 us either way
     if (nrhs > 1 && (double)c->N * c->N * std::min(nrhs, OZ_DENSE_COLS) > 2.5e6)
         return dense64_matvec(c, x, y, nrhs, ld, s);

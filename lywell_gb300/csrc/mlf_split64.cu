@@ -109,12 +109,14 @@ __device__ __forceinline__ int oz_exp(double2 v) {
 
 // sexp[n] = exponent of x's row n over the columns where it is finite (a column
 // that is not is marked by its own exponent; its entries tell the others nothing),
-// the smallest number's where it is zero; *nredo = 0
+// the smallest number's where it is zero; *nredo = 0 and, where given, cexp = OZ_ZERO
 __global__ void k_row_exp(int N, int nrhs, int ld, const double2* __restrict__ x, int* __restrict__ sexp,
-                          int* __restrict__ nredo) {
+                          int* __restrict__ nredo, int* __restrict__ cexp) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
     if (n == 0) *nredo = 0;
+    if (cexp)
+        for (int c = n; c < nrhs; c += N) cexp[c] = OZ_ZERO;
     int e = OZ_ZERO;
     for (int c = 0; c < nrhs; ++c) {
         const int v = oz_exp(x[(size_t)c * ld + n]);
@@ -268,10 +270,6 @@ __global__ void k_dense_row_exp(int N, int nblk, const short* __restrict__ bexp,
     }
     e = __reduce_max_sync(0xffffffffu, e);
     if (lane == 0) rexp[row] = e;
-}
-__global__ void k_set_int(int n, int v, int* __restrict__ a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
 }
 // The check of a value: cover = sum over the real terms of its two parts of the
 // product of the top digits' magnitudes, parts of the terms added up.  A top digit
@@ -692,7 +690,7 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
     const int nb = (int)c->box_ptr.size() - 1, ncb = (nrhs + OZ_C - 1) / OZ_C;
     OzArgs g = oz_args(c, nrhs, ld);
     const OzExps e = oz_exps(c, nb, nrhs);
-    k_row_exp<<<(c->N + 255) / 256, 256, 0, s>>>(c->N, nrhs, ld, x, e.sexp, e.nredo);
+    k_row_exp<<<(c->N + 255) / 256, 256, 0, s>>>(c->N, nrhs, ld, x, e.sexp, e.nredo, nullptr);
     k_near_exp<<<(c->N + 7) / 8, 256, 0, s>>>(c->N, c->dperm, c->dia, c->dja, c->dZ, e.sexp, e.rexp);
     k_col_exp<OZ_NEAR><<<nb * nrhs, 256, 0, s>>>(nrhs, ld, g.K2, g.box_ptr, g.perm, g.ia, g.ja, x, e.sexp, e.cexp,
                                                  nullptr);
@@ -711,7 +709,7 @@ int split64_receive_near(Ctx* c, const double2* x, const double2* A, double facy
 
 // Dense operator: y = Z x for blocks of columns.  The row exponents are bounds by
 // blocks of 32 unknowns, so that a product reads the matrix once.  FP64 FMAs, four
-// columns a pass, against here: 6750 unknowns x 3: 1399, 474 us; x 24: 7678, 1297;
+// columns a pass, against here: 6750 unknowns x 3: 1399, 470 us; x 24: 7678, 1297;
 // 3000 x 2: 339, 120; 1920 x 4: 131, 59; 1080 x 6: 86, 39.  At most OZ_DENSE_COLS
 // columns at a time, so that the workspace is made with the context and products
 // of any number of columns allocate nothing (the first one may be captured).
@@ -731,8 +729,7 @@ static void dense64_columns(Ctx* c, const double2* x, double2* y, int nrhs, int 
     const int N = c->N, nblk = (N + 31) / 32, nsplit = near64_split(c, nrhs);
     int *sexp = c->doz_exp, *rexp = sexp + N, *nredo = rexp + N, *bmax = nredo + 1, *cexp = bmax + nblk;
     unsigned* redo = reinterpret_cast<unsigned*>(cexp + nrhs);
-    k_row_exp<<<(N + 255) / 256, 256, 0, s>>>(N, nrhs, ld, x, sexp, nredo);
-    k_set_int<<<(nrhs + 255) / 256, 256, 0, s>>>(nrhs, OZ_ZERO, cexp);
+    k_row_exp<<<(N + 255) / 256, 256, 0, s>>>(N, nrhs, ld, x, sexp, nredo, cexp);
     k_dense_col_exp<<<std::min((nblk + 7) / 8, 256), 256, 0, s>>>(N, nrhs, ld, nblk, x, sexp, bmax, cexp);
     k_dense_row_exp<<<(N + 7) / 8, 256, 0, s>>>(N, nblk, reinterpret_cast<const short*>(c->doz_pat), bmax, rexp);
     OzArgs g{};
